@@ -35,6 +35,7 @@ struct ChainScal {
     double gp[MAXDIST], vare_gp[MAXDIST];
     double mu_store, vare_store, vara_store, included_store;
     int32_t included, counter, keep, err;
+    uint32_t mu_ticket;        // CTAs of k_mu_partial that are done (wraps to 0)
     double p[MAXGM];           // (ngroup, nmix) column-major
     double log_p[MAXGM];
     double varindist[MAXGM];
@@ -189,5 +190,6 @@ constexpr int ROW_THREADS = 128;   // threads of the row kernels
 constexpr int ROWS_PER_THREAD = 1;
 constexpr int ROW_TILE = ROW_THREADS * ROWS_PER_THREAD;   // rows per row tile (= the update's tile)
 constexpr int RECAL_SPLIT = 32;    // column splits of the residual recalibration
+constexpr int RECAL_CTAS = 608;    // CTAs of its kernels at most
 
 }  // namespace soda

@@ -373,8 +373,16 @@ namespace soda {
 // ---------------------------------------------------------------------------
 // iteration start and the mu draw
 // ---------------------------------------------------------------------------
+constexpr int MU_THREADS = 256;
+constexpr int MU_ROWS = 4 * MU_THREADS;   // rows per CTA of the mu kernels and of the sum of r^2
+static_assert(MU_ROWS == (MU_THREADS / 32) * ROW_TILE, "k_mu_apply gives a row tile to each warp");
+
+__host__ __device__ inline int mu_grid(int n) { return (n + MU_ROWS - 1) / MU_ROWS; }
+
 __device__ __forceinline__ void iter_begin_body(const Dev &D, const VB &vb)
 {
+    tc::pdl_trigger();
+    tc::pdl_wait();
     RunCtl *ctl = D.ctl;
     const int rep = ctl->rep + 1;
     ctl->rep = rep;
@@ -387,63 +395,94 @@ __global__ void  k_iter_begin(Dev D)
 }
 
 
+// The mu draw (models.f90:130-132) in two passes over r.  The first sums MU_ROWS rows per CTA, and the last
+// CTA of a chain to finish (a ticket that wraps to zero) adds the chain's partial sums and draws; the second
+// applies the draw.  Both are bound by their launch and one pass over r (16 bytes a row and chain): at n =
+// 50,000 and 16 chains they take 29 us, against 244 us when every CTA of the second pass added all partial
+// sums by itself, one after another.
 __device__ __forceinline__ void mu_partial_body(const Dev &D, const VB &vb)
 {
     __shared__ double sh[33];
+    __shared__ int s_last;
+    tc::pdl_trigger();
+    tc::pdl_wait();
     const int c = vb.y, rep = cur_rep(D);
-    const double mu_old = D.scal[c].mu[(rep - 1) & 1];
+    ChainScal *S = &D.scal[c];
+    const double mu_old = S->mu[(rep - 1) & 1];
+    const double *r = D.r + (size_t)c * D.ldr;
     double v = 0.0;
 #pragma unroll
-    for (int q = 0; q < ROWS_PER_THREAD; ++q) {
-        const int i = vb.x * ROW_TILE + q * ROW_THREADS + threadIdx.x;
-        if (i < D.n) v += D.r[(size_t)c * D.ldr + i] + mu_old;
+    for (int q = 0; q < MU_ROWS / MU_THREADS; ++q) {
+        const int i = vb.x * MU_ROWS + q * MU_THREADS + threadIdx.x;
+        if (i < D.n) v += r[i] + mu_old;
     }
     const double t = block_sum(v, sh);
-    if (threadIdx.x == 0) D.rpart[(size_t)c * D.nr_ctas + vb.x] = t;
+    if (threadIdx.x == 0) {
+        D.rpart[(size_t)c * D.nr_ctas + vb.x] = t;
+        __threadfence();
+        s_last = atomicInc(&S->mu_ticket, (unsigned)(vb.nx - 1)) == (unsigned)(vb.nx - 1);
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double w = 0.0;
+    for (int q = threadIdx.x; q < vb.nx; q += MU_THREADS) w += __ldcg(D.rpart + (size_t)c * D.nr_ctas + q);
+    const double tot = block_sum(w, sh);
+    if (threadIdx.x == 0) {
+        CRng R;
+        crng_site(R, D, c, rep, 0, P_MU);
+        const double nn = (double)D.n;
+        S->mu[rep & 1] = d_rnorm(tot / nn, sqrt(S->vare / nn), R);
+    }
 }
 
-__global__ void __launch_bounds__(ROW_THREADS) k_mu_partial(Dev D)
+__global__ void __launch_bounds__(MU_THREADS) k_mu_partial(Dev D)
 {
     mu_partial_body(D, vb_native());
 }
 
 
+// A warp takes a tile of ROW_TILE rows, four consecutive ones a lane (16-byte loads and stores of r, 8-byte
+// ones of its bf16 split), and leaves the tile's sum for the FP8 centring.  Rows n .. ldr-1 stay zero.
 __device__ __forceinline__ void mu_apply_body(const Dev &D, const VB &vb)
 {
-    __shared__ double sh[33];
-    __shared__ double s_mu;
-    const int c = vb.y, rep = cur_rep(D);
-    ChainScal *S = &D.scal[c];
-    const double mu_old = S->mu[(rep - 1) & 1];
-    if (threadIdx.x == 0) {
-        double tot = 0.0;
-        for (int t = 0; t < D.nr_ctas; ++t) tot += D.rpart[(size_t)c * D.nr_ctas + t];
-        CRng R;
-        crng_site(R, D, c, rep, 0, P_MU);
-        const double nn = (double)D.n;
-        const double mu = d_rnorm(tot / nn, sqrt(S->vare / nn), R);
-        s_mu = mu;
-        if (vb.x == 0) S->mu[rep & 1] = mu;
-    }
-    __syncthreads();
-    const double mu = s_mu;
-    double vs = 0.0;
+    tc::pdl_trigger();
+    tc::pdl_wait();
+    const int c = vb.y, rep = cur_rep(D), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = vb.x * (MU_THREADS / 32) + warp;
+    if (tile >= D.nr_ctas) return;
+    const ChainScal *S = &D.scal[c];
+    const double mu_old = S->mu[(rep - 1) & 1], mu = S->mu[rep & 1];
+    const int i0 = tile * ROW_TILE + 4 * lane;
+    const size_t o = (size_t)c * D.ldr + i0;
+    double2 *r2 = reinterpret_cast<double2 *>(D.r + o);
+    const double2 ra = r2[0], rb = r2[1];
+    double v[4] = {ra.x, ra.y, rb.x, rb.y};
+    float f[4];
 #pragma unroll
-    for (int q = 0; q < ROWS_PER_THREAD; ++q) {
-        const int i = vb.x * ROW_TILE + q * ROW_THREADS + threadIdx.x;
-        if (i < D.n) {
-            const double v = (D.r[(size_t)c * D.ldr + i] + mu_old) - mu;
-            store_r(D, c, i, v);
-            vs += v;
-        }
+    for (int k = 0; k < 4; ++k) {
+        v[k] = i0 + k < D.n ? (v[k] + mu_old) - mu : 0.0;
+        f[k] = (float)v[k];
+    }
+    r2[0] = make_double2(v[0], v[1]);
+    r2[1] = make_double2(v[2], v[3]);
+    if (!D.tc) *reinterpret_cast<float4 *>(D.r32 + o) = make_float4(f[0], f[1], f[2], f[3]);
+    if (D.rsp) {
+        uint32_t h[4], m[4], l[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tc::split3(f[k], h[k], m[k], l[k]);
+        const size_t part = (size_t)D.chains * D.ldr;
+        *reinterpret_cast<uint2 *>(D.rsp + o) = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+        *reinterpret_cast<uint2 *>(D.rsp + o + part) = make_uint2(m[0] | m[1] << 16, m[2] | m[3] << 16);
+        *reinterpret_cast<uint2 *>(D.rsp + o + 2 * part) = make_uint2(l[0] | l[1] << 16, l[2] | l[3] << 16);
     }
     if (D.precision == SODAGPU_FP8) {
-        const double t = block_sum(vs, sh);
-        if (threadIdx.x == 0) D.rsum[(size_t)c * D.nr_ctas + vb.x] = t;
+        const double t = warp_sum((v[0] + v[1]) + (v[2] + v[3]));
+        if (lane == 0) D.rsum[(size_t)c * D.nr_ctas + tile] = t;
     }
 }
 
-__global__ void __launch_bounds__(ROW_THREADS) k_mu_apply(Dev D)
+__global__ void __launch_bounds__(MU_THREADS) k_mu_apply(Dev D)
 {
     mu_apply_body(D, vb_native());
 }
@@ -650,43 +689,96 @@ __global__ void __launch_bounds__(SS_THREADS) k_skipped(Dev D)
 // per-iteration statistics: class counts and sum g^2 per (group, class),
 // sum r^2 (models.f90:194, 321-325, 496-503, 515)
 // ---------------------------------------------------------------------------
+// CTAs 0..NSTAT-1 of a chain take the SNPs, the others MU_ROWS rows of r each.  With up to STAT_FAST (group,
+// class) cells one pass serves all of them: a warp adds the squares of its 32 SNPs cell by cell (sparse chains
+// have a few non-zero effects per warp) into its own row of shared sums, in a fixed order, and the counts go
+// through integer atomics; more cells take one pass over the SNPs each.  At p = 12,000, 12 cells and 16 chains
+// the one pass takes 13 us, twelve passes took 122 us.
+constexpr int STAT_FAST = 64;
+
 __device__ __forceinline__ void stats_body(const Dev &D, const VB &vb)
 {
     __shared__ double sh[33];
+    __shared__ double s_acc[8][STAT_FAST];
+    __shared__ int s_cnt[STAT_FAST];
+    tc::pdl_trigger();
+    tc::pdl_wait();
     const int c = vb.y;
-    if (vb.x < NSTAT) {
-        const int ngm = D.ngroup * D.nmix;
-        const size_t base = (size_t)c * D.p;
-        for (int e = 0; e < ngm; ++e) {
-            const int eg = e % D.ngroup, em = e / D.ngroup;
-            double v = 0.0;
-            int cnt = 0;
-            for (int j = vb.x * 256 + threadIdx.x; j < D.p; j += NSTAT * 256) {
-                const int cl = D.cls[base + j];
-                if (D.grp[j] - 1 == eg && cl - 1 == em) {
-                    const double gj = D.g[base + j];
-                    v += gj * gj;
-                    ++cnt;
-                }
-            }
-            const double tv = block_sum(v, sh);
-            const double tc = block_sum((double)cnt, sh);
-            if (threadIdx.x == 0) {
-                const size_t o = ((size_t)c * NSTAT + vb.x) * ngm + e;
-                D.statpart[o] = tv;
-                D.cntpart[o] = (int32_t)tc;
-            }
-        }
-    } else {
+    if (vb.x >= NSTAT) {
         const int rb = vb.x - NSTAT;
+        const double *r = D.r + (size_t)c * D.ldr;
         double v2 = 0.0;
-        const int i = rb * ROW_TILE + threadIdx.x;
-        if (threadIdx.x < ROW_TILE && i < D.n) {
-            const double v = D.r[(size_t)c * D.ldr + i];
-            v2 = v * v;
+#pragma unroll
+        for (int q = 0; q < MU_ROWS / 256; ++q) {
+            const int i = rb * MU_ROWS + q * 256 + threadIdx.x;
+            if (i < D.n) v2 += r[i] * r[i];
         }
         const double t = block_sum(v2, sh);
         if (threadIdx.x == 0) D.rpart[(size_t)c * D.nr_ctas + rb] = t;
+        return;
+    }
+    const int ngm = D.ngroup * D.nmix;
+    const size_t base = (size_t)c * D.p;
+    if (ngm <= STAT_FAST) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        for (int e = threadIdx.x; e < 8 * ngm; e += 256) s_acc[e / ngm][e % ngm] = 0.0;
+        if (threadIdx.x < ngm) s_cnt[threadIdx.x] = 0;
+        __syncthreads();
+        for (int j0 = vb.x * 256 + 32 * warp; j0 < D.p; j0 += NSTAT * 256) {
+            const int j = j0 + lane;
+            int e = -1;
+            double v = 0.0;
+            if (j < D.p) {
+                e = (D.grp[j] - 1) + (D.cls[base + j] - 1) * D.ngroup;
+                const double gj = D.g[base + j];
+                v = gj * gj;
+            }
+            const unsigned same = __match_any_sync(0xffffffffu, e);
+            if (e >= 0 && lane == __ffs(same) - 1) atomicAdd(&s_cnt[e], __popc(same));
+            unsigned todo = __ballot_sync(0xffffffffu, v != 0.0);
+            while (todo) {   // one cell at a time, in the order of its first lane
+                const int src = __ffs(todo) - 1, e0 = __shfl_sync(0xffffffffu, e, src);
+                const unsigned in = __ballot_sync(0xffffffffu, v != 0.0 && e == e0);
+                if (__popc(in) == 1) {
+                    if (lane == src) s_acc[warp][e0] += v;
+                } else {
+                    const double t = warp_sum(v != 0.0 && e == e0 ? v : 0.0);
+                    if (lane == 0) s_acc[warp][e0] += t;
+                }
+                __syncwarp();
+                todo &= ~in;
+            }
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < ngm; e += 256) {
+            double t = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) t += s_acc[w][e];
+            const size_t o = ((size_t)c * NSTAT + vb.x) * ngm + e;
+            D.statpart[o] = t;
+            D.cntpart[o] = s_cnt[e];
+        }
+        return;
+    }
+    for (int e = 0; e < ngm; ++e) {
+        const int eg = e % D.ngroup, em = e / D.ngroup;
+        double v = 0.0;
+        int cnt = 0;
+        for (int j = vb.x * 256 + threadIdx.x; j < D.p; j += NSTAT * 256) {
+            const int cl = D.cls[base + j];
+            if (D.grp[j] - 1 == eg && cl - 1 == em) {
+                const double gj = D.g[base + j];
+                v += gj * gj;
+                ++cnt;
+            }
+        }
+        const double tv = block_sum(v, sh);
+        const double tc = block_sum((double)cnt, sh);
+        if (threadIdx.x == 0) {
+            const size_t o = ((size_t)c * NSTAT + vb.x) * ngm + e;
+            D.statpart[o] = tv;
+            D.cntpart[o] = (int32_t)tc;
+        }
     }
 }
 
@@ -696,27 +788,47 @@ __global__ void __launch_bounds__(256) k_stats(Dev D)
 }
 
 
+// The hyper-parameter draws of a chain, one CTA.  They are bound by the latency of a few FP64 draws, so the
+// three that do not depend on one another run at once: sigma2_g in warp 0, sigma2_e in warp 1, and pi in the
+// others, one thread a group.  With the sums before them and the tables after them spread over the CTA's
+// threads, a chain of BayesR takes 28 us (62 us when one thread did it all).
+constexpr int HYPER_THREADS = 256;
+
 __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
 {
-    __shared__ double s_vara;
-    const int c = vb.x, rep = cur_rep(D);
+    __shared__ double s_rr;
+    tc::pdl_trigger();
+    tc::pdl_wait();
+    const int c = vb.x, rep = cur_rep(D), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int NW = HYPER_THREADS / 32;
     ChainScal *S = &D.scal[c];
     const int ng = D.ngroup, nm = D.nmix, ngm = ng * nm, m = D.method;
-    for (int e = threadIdx.x; e < ngm; e += blockDim.x) {
+    // sums over the CTAs of k_stats: cell e by warp e % NW, sum r^2 by the last warp
+    for (int e = warp; e < ngm; e += NW) {
         double v = 0.0;
         int cnt = 0;
-        for (int t = 0; t < NSTAT; ++t) {
+        for (int t = lane; t < NSTAT; t += 32) {
             const size_t o = ((size_t)c * NSTAT + t) * ngm + e;
             v += D.statpart[o];
             cnt += D.cntpart[o];
         }
-        S->varindist[e] = v;
-        // BayesA tracks no class counts (models.f90:194): its trace shows none
-        S->snpindist[e] = m == SODAGPU_BAYES_A ? 0 : cnt;
+        v = warp_sum(v);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) {
+            S->varindist[e] = v;
+            // BayesA tracks no class counts (models.f90:194): its trace shows none
+            S->snpindist[e] = m == SODAGPU_BAYES_A ? 0 : cnt;
+        }
+    }
+    if (warp == NW - 1) {
+        double rr = 0.0;
+        for (int t = lane; t < mu_grid(D.n); t += 32) rr += D.rpart[(size_t)c * D.nr_ctas + t];
+        rr = warp_sum(rr);
+        if (lane == 0) s_rr = rr;
     }
     __syncthreads();
     int err = 0;
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         if (m == SODAGPU_BAYES_B) {
             S->included = S->snpindist[ng];
             S->varindist[0] = 0.0;
@@ -733,19 +845,15 @@ __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
             S->vara = d_rscinvchi2((double)S->included + D.df_va, scale, R, &err);
             for (int j = 0; j < nm; ++j) S->gp[j] = D.mix[j] * S->vara;
         }
-        double rr = 0.0;
-        for (int t = 0; t < D.nr_ctas; ++t) rr += D.rpart[(size_t)c * D.nr_ctas + t];
+    } else if (tid == 32) {
         const double nn = (double)D.n;
-        const double scale = (rr + D.scale_ve * D.df_ve) / (nn + D.df_ve);
+        const double scale = (s_rr + D.scale_ve * D.df_ve) / (nn + D.df_ve);
         CRng R;
         crng_site(R, D, c, rep, 0, P_VARE);
         S->vare = d_rscinvchi2(nn + D.df_ve, scale, R, &err);
-        s_vara = S->vara;
-    }
-    __syncthreads();
-    // pi ~ Dirichlet(counts + alpha), one thread per group (models.f90:517-522)
-    if (m == SODAGPU_BAYES_CPI || m == SODAGPU_BAYES_R || m == SODAGPU_BAYES_RC) {
-        for (int i = threadIdx.x; i < ng; i += blockDim.x) {
+    } else if (warp >= 2 && (m == SODAGPU_BAYES_CPI || m == SODAGPU_BAYES_R || m == SODAGPU_BAYES_RC)) {
+        // pi ~ Dirichlet(counts + alpha), one thread per group (models.f90:517-522), groups over the warps first
+        for (int i = lane * (NW - 2) + warp - 2; i < ng; i += 32 * (NW - 2)) {
             CRng R;
             crng_site(R, D, c, rep, i, P_PI);
             double x[MAXDIST], sx = 0.0;
@@ -755,32 +863,41 @@ __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
             for (int j = 0; j < nm; ++j) S->p[i + j * ng] = x[j] / sx;
         }
     }
+    if (err) flag_err(D, 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const bool keep = rep > D.burnin && rep % D.thin == 0;
+    const bool keep = rep > D.burnin && rep % D.thin == 0;
+    const double mu = S->mu[rep & 1];
+    for (int e = tid; e < ngm; e += HYPER_THREADS) {
+        if (keep) {
+            // soda_bayes keeps varstore for every method (models.f90:530), regular_bayes
+            // not for BayesA (models.f90:893-896)
+            if (!(D.regular && m == SODAGPU_BAYES_A)) S->varstore[e] = S->varstore[e] + S->varindist[e];
+            if (m != SODAGPU_BAYES_A) {
+                S->snpstore[e] = S->snpstore[e] + S->snpindist[e];
+                if (m != SODAGPU_BAYES_B && m != SODAGPU_BAYES_C) S->pstore[e] = S->pstore[e] + S->p[e];
+            }
+        }
+        // log_p for the next iteration (models.f90:198-199, 330-338)
+        if (m != SODAGPU_BAYES_A) S->log_p[e] = log(S->p[e]);
+    }
+    if (m != SODAGPU_BAYES_A)
+        for (int j = 1 + tid; j < nm; j += HYPER_THREADS) S->vare_gp[j] = S->vare / S->gp[j];
+    if (tid == 0) {
         S->keep = keep;
-        const double mu = S->mu[rep & 1];
         if (keep) {
             S->counter += 1;
             S->mu_store = S->mu_store + mu;
-            // soda_bayes keeps varstore for every method (models.f90:530), regular_bayes
-            // not for BayesA (models.f90:893-896)
-            if (!(D.regular && m == SODAGPU_BAYES_A))
-                for (int e = 0; e < ngm; ++e) S->varstore[e] = S->varstore[e] + S->varindist[e];
             S->vare_store = S->vare_store + S->vare;
-            if (m != SODAGPU_BAYES_A) {
-                S->included_store = S->included_store + S->included;
-                for (int e = 0; e < ngm; ++e) S->snpstore[e] = S->snpstore[e] + S->snpindist[e];
-                if (m != SODAGPU_BAYES_B && m != SODAGPU_BAYES_C)
-                    for (int e = 0; e < ngm; ++e) S->pstore[e] = S->pstore[e] + S->p[e];
-            }
-            if (m != SODAGPU_BAYES_A && m != SODAGPU_BAYES_B) S->vara_store = S->vara_store + s_vara;
+            if (m != SODAGPU_BAYES_A) S->included_store = S->included_store + S->included;
+            if (m != SODAGPU_BAYES_A && m != SODAGPU_BAYES_B) S->vara_store = S->vara_store + S->vara;
         }
-        if (rep % D.thin == 0) {
-            RunCtl *ctl = D.ctl;
-            const int row = (ctl->trace_iter - 1) * D.chains + c;
-            if (ctl->trace && row >= 0 && row < ctl->trace_cap) {
-                sodagpu_trace_row *tr = ctl->trace + row;
+    }
+    if (rep % D.thin == 0) {
+        RunCtl *ctl = D.ctl;
+        const int row = (ctl->trace_iter - 1) * D.chains + c;
+        if (ctl->trace && row >= 0 && row < ctl->trace_cap) {
+            sodagpu_trace_row *tr = ctl->trace + row;
+            if (tid == 0) {
                 tr->chain = c;
                 tr->rep = rep;
                 tr->included = S->included;
@@ -788,22 +905,16 @@ __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
                 tr->mu = mu;
                 tr->vare = S->vare;
                 tr->vara = S->vara;
-                for (int j = 0; j < MAXDIST; ++j) {
-                    tr->snpindist[j] = j < nm ? S->snpindist[j * ng] : 0;
-                    tr->varindist[j] = j < nm ? S->varindist[j * ng] : 0.0;
-                }
+            }
+            for (int j = tid; j < MAXDIST; j += HYPER_THREADS) {
+                tr->snpindist[j] = j < nm ? S->snpindist[j * ng] : 0;
+                tr->varindist[j] = j < nm ? S->varindist[j * ng] : 0.0;
             }
         }
-        // log_p and vare/gp for the next iteration (models.f90:198-199, 330-338)
-        if (m != SODAGPU_BAYES_A) {
-            for (int e = 0; e < ngm; ++e) S->log_p[e] = log(S->p[e]);
-            for (int j = 1; j < nm; ++j) S->vare_gp[j] = S->vare / S->gp[j];
-        }
-        if (err) flag_err(D, 1);
     }
 }
 
-__global__ void __launch_bounds__(128) k_hyper(Dev D)
+__global__ void __launch_bounds__(HYPER_THREADS) k_hyper(Dev D)
 {
     hyper_body(D, vb_native());
 }
@@ -812,11 +923,16 @@ __global__ void __launch_bounds__(128) k_hyper(Dev D)
 // ra redraw (models.f90:523-525) and the per-SNP accumulators (528, 535-538, 544)
 __device__ __forceinline__ void post_body(const Dev &D, const VB &vb)
 {
+    tc::pdl_trigger();
+    tc::pdl_wait();
     const int c = vb.y, rep = cur_rep(D);
     const ChainScal *S = &D.scal[c];
     const int t0 = vb.x * blockDim.x + threadIdx.x, stride = vb.nx * blockDim.x;
     const double sd = sqrt(S->vare);
-    for (int i = t0; i < D.naind; i += stride) {
+    // FP64 draws: one row of every CTA's share after the other, so that the narrow FP64 pipes of all SMs
+    // take part (with CTA-contiguous rows the first CTAs of a chain did all of them: 26 us for 16 x 2000
+    // rows, 23 us like this)
+    for (int i = threadIdx.x * vb.nx + vb.x; i < D.naind; i += stride) {
         CRng R;
         crng_site(R, D, c, rep, i, P_RA);
         store_ra(D, c, i, d_rnorm(0.0, sd, R));
@@ -838,24 +954,32 @@ __global__ void __launch_bounds__(256) k_post(Dev D)
 }
 
 
-// compute_residuals (utilities.f90:609-614), every `recal` iterations
+// compute_residuals (utilities.f90:609-614), every `recal` iterations.  The two kernels are launched every
+// iteration (the iteration is a captured graph) and return at once on the others, so their grids hold
+// RECAL_CTAS CTAs that walk the (rows, column split, chain) tiles: one CTA a tile cost 302 us an iteration in
+// CTA launches alone at n = 50,000 and 16 chains.
 __device__ __forceinline__ void recal_partial_body(const Dev &D, const VB &vb, int force)
 {
+    tc::pdl_trigger();
+    tc::pdl_wait();
     const int rep = cur_rep(D);
     if (!force && (D.recal <= 0 || rep % D.recal != 0)) return;
-    const int c = vb.z, split = vb.y;
-    const int i = vb.x * 256 + threadIdx.x;
-    if (i >= D.n) return;
+    const int tiles = (D.n + 255) / 256, total = tiles * RECAL_SPLIT * D.chains;
     const int per = (D.p + RECAL_SPLIT - 1) / RECAL_SPLIT;
-    const int k0 = split * per, k1 = min(D.p, k0 + per);
-    double acc = 0.0;
-    const double *g = D.g + (size_t)c * D.p;
-    for (int k = k0; k < k1; ++k) {
-        const double gj = g[D.perm[k]];
-        if (gj == 0.0) continue;
-        acc = acc + D.xv[(size_t)k * 4 + D.G[(size_t)k * D.ldx + i]] * gj;
+    for (int t = vb.x; t < total; t += vb.nx) {
+        const int c = t / (tiles * RECAL_SPLIT), split = (t / tiles) % RECAL_SPLIT;
+        const int i = (t % tiles) * 256 + threadIdx.x;
+        if (i >= D.n) continue;
+        const int k0 = split * per, k1 = min(D.p, k0 + per);
+        double acc = 0.0;
+        const double *g = D.g + (size_t)c * D.p;
+        for (int k = k0; k < k1; ++k) {
+            const double gj = g[D.perm[k]];
+            if (gj == 0.0) continue;
+            acc = acc + D.xv[(size_t)k * 4 + D.G[(size_t)k * D.ldx + i]] * gj;
+        }
+        D.recal_part[((size_t)c * RECAL_SPLIT + split) * D.ldr + i] = acc;
     }
-    D.recal_part[((size_t)c * RECAL_SPLIT + split) * D.ldr + i] = acc;
 }
 
 __global__ void __launch_bounds__(256) k_recal_partial(Dev D, int force)
@@ -866,15 +990,19 @@ __global__ void __launch_bounds__(256) k_recal_partial(Dev D, int force)
 
 __device__ __forceinline__ void recal_apply_body(const Dev &D, const VB &vb, int force, int mu_slot)
 {
+    tc::pdl_trigger();
+    tc::pdl_wait();
     const int rep = cur_rep(D);
     if (!force && (D.recal <= 0 || rep % D.recal != 0)) return;
-    const int c = vb.y;
-    const int i = vb.x * 256 + threadIdx.x;
-    if (i >= D.n) return;
-    double d = 0.0;
-    for (int s = 0; s < RECAL_SPLIT; ++s) d = d + D.recal_part[((size_t)c * RECAL_SPLIT + s) * D.ldr + i];
+    const int tiles = (D.n + 255) / 256, total = tiles * D.chains;
     const int slot = mu_slot >= 0 ? mu_slot : (rep & 1);
-    store_r(D, c, i, D.y[i] - d - D.scal[c].mu[slot]);
+    for (int t = vb.x; t < total; t += vb.nx) {
+        const int c = t / tiles, i = (t % tiles) * 256 + threadIdx.x;
+        if (i >= D.n) continue;
+        double d = 0.0;
+        for (int s = 0; s < RECAL_SPLIT; ++s) d = d + D.recal_part[((size_t)c * RECAL_SPLIT + s) * D.ldr + i];
+        store_r(D, c, i, D.y[i] - d - D.scal[c].mu[slot]);
+    }
 }
 
 __global__ void __launch_bounds__(256) k_recal_apply(Dev D, int force, int mu_slot)
@@ -911,6 +1039,7 @@ __global__ void __launch_bounds__(256) k_init_chain(Dev D, double vara0, double 
         S->scale_va = scale_va0;
         S->vara = vara0;
         S->counter = 0;
+        S->mu_ticket = 0;
         S->keep = 0;
         S->err = 0;
         S->included = 0;
@@ -1425,20 +1554,31 @@ cudaError_t sweep_prepare(int bs)
     return e;
 }
 
+// CTAs of k_post per chain, and of the recalibration kernels over all of their tiles.
+static int post_grid(const Dev &D, int sm_count)
+{
+    return std::max(1, std::min((D.p + 255) / 256, 4 * sm_count));
+}
+static int recal_grid(const Dev &D, int splits)
+{
+    return (int)std::min<long long>((long long)((D.n + 255) / 256) * splits * D.chains, RECAL_CTAS);
+}
+
 cudaError_t sweep_enqueue_iteration(const Dev &D, const int *blk_sizes, int sm_count, const TcMaps *maps,
                                     cudaStream_t st, ProfHook *prof)
 {
     if (D.tc && !maps) return cudaErrorInvalidValue;
     const int C = D.chains;
+    cudaError_t e = cudaSuccess;
     {
         ProfScope ps(prof, st, PROF_MU);
         k_iter_begin<<<1, 1, 0, st>>>(D);
-        k_mu_partial<<<dim3(D.nr_ctas, C), ROW_THREADS, 0, st>>>(D);
-        k_mu_apply<<<dim3(D.nr_ctas, C), ROW_THREADS, 0, st>>>(D);
+        e = launch_pdl(k_mu_partial, dim3(mu_grid(D.n), C), dim3(MU_THREADS), 0, st, D);
+        if (e == cudaSuccess) e = launch_pdl(k_mu_apply, dim3(mu_grid(D.n), C), dim3(MU_THREADS), 0, st, D);
+        if (e != cudaSuccess) return e;
     }
     for (int b = 0; b < D.nb; ++b) {
         const int nsnp = blk_sizes[b];
-        cudaError_t e;
         if (D.precision == SODAGPU_FP64) e = launch_block_mode<SODAGPU_FP64>(D, b, nsnp, sm_count, maps, st, prof);
         else if (D.precision == SODAGPU_FP32)
             e = launch_block_mode<SODAGPU_FP32>(D, b, nsnp, sm_count, maps, st, prof);
@@ -1451,14 +1591,13 @@ cudaError_t sweep_enqueue_iteration(const Dev &D, const int *blk_sizes, int sm_c
             const size_t sm = (size_t)D.n * sizeof(double) <= (size_t)SS_SMEM_MAX ? (size_t)D.n * sizeof(double) : 0;
             k_skipped<<<C, SS_THREADS, sm, st>>>(D);
         }
-        k_stats<<<dim3(NSTAT + D.nr_ctas, C), 256, 0, st>>>(D);
-        k_hyper<<<C, 128, 0, st>>>(D);
-        const int pgrid = (D.p + 255) / 256 < 4 * sm_count ? (D.p + 255) / 256 : 4 * sm_count;
-        k_post<<<dim3(pgrid > 0 ? pgrid : 1, C), 256, 0, st>>>(D);
-        k_recal_partial<<<dim3((D.n + 255) / 256, RECAL_SPLIT, C), 256, 0, st>>>(D, 0);
-        k_recal_apply<<<dim3((D.n + 255) / 256, C), 256, 0, st>>>(D, 0, -1);
+        e = launch_pdl(k_stats, dim3(NSTAT + mu_grid(D.n), C), dim3(256), 0, st, D);
+        if (e == cudaSuccess) e = launch_pdl(k_hyper, dim3(C), dim3(HYPER_THREADS), 0, st, D);
+        if (e == cudaSuccess) e = launch_pdl(k_post, dim3(post_grid(D, sm_count), C), dim3(256), 0, st, D);
+        if (e == cudaSuccess) e = launch_pdl(k_recal_partial, dim3(recal_grid(D, RECAL_SPLIT)), dim3(256), 0, st, D, 0);
+        if (e == cudaSuccess) e = launch_pdl(k_recal_apply, dim3(recal_grid(D, 1)), dim3(256), 0, st, D, 0, -1);
     }
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t sweep_enqueue_init(const Dev &D, double vara0, double scale_va0, int sm_count, cudaStream_t st)
@@ -1539,8 +1678,8 @@ cudaError_t sweep_set_state(const Dev &D, int c, const double *g, const int32_t 
 cudaError_t sweep_enqueue_recal(const Dev &D, double mu_slot_unused, cudaStream_t st)
 {
     (void)mu_slot_unused;
-    k_recal_partial<<<dim3((D.n + 255) / 256, RECAL_SPLIT, D.chains), 256, 0, st>>>(D, 1);
-    k_recal_apply<<<dim3((D.n + 255) / 256, D.chains), 256, 0, st>>>(D, 1, -1);
+    k_recal_partial<<<recal_grid(D, RECAL_SPLIT), 256, 0, st>>>(D, 1);
+    k_recal_apply<<<recal_grid(D, 1), 256, 0, st>>>(D, 1, -1);
     return cudaGetLastError();
 }
 
@@ -1561,14 +1700,14 @@ __global__ void k_iter_begin_m(const __grid_constant__ JobGrid G)
     iter_begin_body(G.dev[j], vb);
 }
 
-__global__ void __launch_bounds__(ROW_THREADS) k_mu_partial_m(const __grid_constant__ JobGrid G)
+__global__ void __launch_bounds__(MU_THREADS) k_mu_partial_m(const __grid_constant__ JobGrid G)
 {
     VB vb;
     const int j = jg_locate(G, vb);
     mu_partial_body(G.dev[j], vb);
 }
 
-__global__ void __launch_bounds__(ROW_THREADS) k_mu_apply_m(const __grid_constant__ JobGrid G)
+__global__ void __launch_bounds__(MU_THREADS) k_mu_apply_m(const __grid_constant__ JobGrid G)
 {
     VB vb;
     const int j = jg_locate(G, vb);
@@ -1589,7 +1728,7 @@ __global__ void __launch_bounds__(256) k_stats_m(const __grid_constant__ JobGrid
     stats_body(G.dev[j], vb);
 }
 
-__global__ void __launch_bounds__(128) k_hyper_m(const __grid_constant__ JobGrid G)
+__global__ void __launch_bounds__(HYPER_THREADS) k_hyper_m(const __grid_constant__ JobGrid G)
 {
     VB vb;
     const int j = jg_locate(G, vb);
@@ -1788,16 +1927,17 @@ cudaError_t sweep_enqueue_iteration_multi(const BatchPlan &P, int sm_count, cuda
     for (int j = 0; j < nj; ++j) {
         const Dev &D = P.hdev[j];
         one.set(j, 1, 1, 1);
-        rows.set(j, D.nr_ctas, D.chains, 1);
+        rows.set(j, mu_grid(D.n), D.chains, 1);
         maxnb = std::max(maxnb, D.nb);
     }
     k_iter_begin_m<<<one.total(), 1, 0, st>>>(one.g);
-    k_mu_partial_m<<<rows.total(), ROW_THREADS, 0, st>>>(rows.g);
-    k_mu_apply_m<<<rows.total(), ROW_THREADS, 0, st>>>(rows.g);
+    cudaError_t e = launch_pdl(k_mu_partial_m, dim3(rows.total()), dim3(MU_THREADS), 0, st, rows.g);
+    if (e == cudaSuccess) e = launch_pdl(k_mu_apply_m, dim3(rows.total()), dim3(MU_THREADS), 0, st, rows.g);
+    if (e != cudaSuccess) return e;
     for (int t = 0; t < maxnb; ++t) {
-        cudaError_t e = prec == SODAGPU_FP64   ? multi_step_mode<SODAGPU_FP64>(P, t, st)
-                        : prec == SODAGPU_FP32 ? multi_step_mode<SODAGPU_FP32>(P, t, st)
-                                               : multi_step_mode<SODAGPU_FP8>(P, t, st);
+        e = prec == SODAGPU_FP64   ? multi_step_mode<SODAGPU_FP64>(P, t, st)
+            : prec == SODAGPU_FP32 ? multi_step_mode<SODAGPU_FP32>(P, t, st)
+                                   : multi_step_mode<SODAGPU_FP8>(P, t, st);
         if (e != cudaSuccess) return e;
     }
     GridBuilder skp(P.ddev, nj), stats(P.ddev, nj), hyp(P.ddev, nj), post(P.ddev, nj), rp(P.ddev, nj),
@@ -1809,20 +1949,19 @@ cudaError_t sweep_enqueue_iteration_multi(const BatchPlan &P, int sm_count, cuda
         skp.set(j, D.nskipped > 0 ? C : 0, 1, 1);
         if (D.nskipped > 0 && (size_t)D.n * sizeof(double) <= (size_t)SS_SMEM_MAX)
             ssm = std::max(ssm, (size_t)D.n * sizeof(double));
-        stats.set(j, NSTAT + D.nr_ctas, C, 1);
+        stats.set(j, NSTAT + mu_grid(D.n), C, 1);
         hyp.set(j, C, 1, 1);
-        const int pgrid = (D.p + 255) / 256 < 4 * sm_count ? (D.p + 255) / 256 : 4 * sm_count;
-        post.set(j, pgrid > 0 ? pgrid : 1, C, 1);
-        rp.set(j, (D.n + 255) / 256, RECAL_SPLIT, C);
-        ra.set(j, (D.n + 255) / 256, C, 1);
+        post.set(j, post_grid(D, sm_count), C, 1);
+        rp.set(j, recal_grid(D, RECAL_SPLIT), 1, 1);
+        ra.set(j, recal_grid(D, 1), 1, 1);
     }
     if (skp.total() > 0) k_skipped_m<<<skp.total(), SS_THREADS, ssm, st>>>(skp.g);
-    k_stats_m<<<stats.total(), 256, 0, st>>>(stats.g);
-    k_hyper_m<<<hyp.total(), 128, 0, st>>>(hyp.g);
-    k_post_m<<<post.total(), 256, 0, st>>>(post.g);
-    k_recal_partial_m<<<rp.total(), 256, 0, st>>>(rp.g);
-    k_recal_apply_m<<<ra.total(), 256, 0, st>>>(ra.g);
-    return cudaGetLastError();
+    e = launch_pdl(k_stats_m, dim3(stats.total()), dim3(256), 0, st, stats.g);
+    if (e == cudaSuccess) e = launch_pdl(k_hyper_m, dim3(hyp.total()), dim3(HYPER_THREADS), 0, st, hyp.g);
+    if (e == cudaSuccess) e = launch_pdl(k_post_m, dim3(post.total()), dim3(256), 0, st, post.g);
+    if (e == cudaSuccess) e = launch_pdl(k_recal_partial_m, dim3(rp.total()), dim3(256), 0, st, rp.g);
+    if (e == cudaSuccess) e = launch_pdl(k_recal_apply_m, dim3(ra.total()), dim3(256), 0, st, ra.g);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace soda

@@ -299,10 +299,9 @@ int sodagpu_profile_kernels(sodagpu_ctx *ctx, int32_t iters, double *ms, int32_t
  * and leave their partial sums in it: calls that overlap on the GPU race and
  * must be serialised by the caller.  cudaDeviceReset invalidates the address
  * looked up for that device: after a reset, do not call this again on that
- * device in the same process.  The columns are summed in min(32,
- * SODAGPU_NOALLOC_SCRATCH / nind, nloci) splits: up to nind = 65,536 the same
- * order as sodagpu_predict, above it the last bits may differ.  Codes outside
- * 0..2 count as 1 (a missing call, utilities.f90:446-449), where
+ * device in the same process.  The columns are summed in sodagpu_predict's
+ * splits while nind times their number fits the scratch, in fewer above that
+ * (the last bits may differ then).  Codes outside 0..2 count as 1 (a missing call, utilities.f90:446-449), where
  * sodagpu_predict returns SODAGPU_E_ARG.  Errors are reported by the return
  * code only (sodagpu_last_error is not updated); a launch error the caller
  * left pending is neither reported nor cleared. */

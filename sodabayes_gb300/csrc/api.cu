@@ -1215,18 +1215,17 @@ int sodagpu_compute_dgv(sodagpu_ctx *c, double mu, const double *effects, double
 {
     if (!c || !effects || !pred) return fail(SODAGPU_E_ARG, "null argument");
     if (!c->have_z) return fail(SODAGPU_E_STATE, "no genotypes in subset order (run sodagpu_build_z)");
-    const int nsplit = 32;
-    double *deff = nullptr, *part = nullptr, *dpred = nullptr;
-    TRY(c->alloc(&deff, c->p, false));
-    TRY(c->alloc(&part, (size_t)nsplit * c->ldx, false));
-    TRY(c->alloc(&dpred, c->n, false));
-    CUDA_TRY(cudaMemcpyAsync(deff, effects, sizeof(double) * c->p, cudaMemcpyHostToDevice, c->st));
-    CUDA_TRY(zb_dgv(c->G, c->ldx, c->xv, c->perm, deff, c->n, c->p, mu, part, nsplit, dpred, c->st));
-    CUDA_TRY(cudaMemcpyAsync(pred, dpred, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->st));
-    CUDA_TRY(cudaStreamSynchronize(c->st));
-    c->release(deff);
-    c->release(part);
-    c->release(dpred);
+    // one allocation: effects, predictions, the splits' sums
+    double *buf = nullptr;
+    TRY(c->alloc(&buf, (size_t)c->p + c->n + (size_t)zb_dgv_splits(c->n, c->p) * c->n, false));
+    double *deff = buf, *dpred = deff + c->p, *part = dpred + c->n;
+    cudaError_t e = cudaMemcpyAsync(deff, effects, sizeof(double) * c->p, cudaMemcpyHostToDevice, c->st);
+    if (e == cudaSuccess)
+        e = zb_dgv(c->G, c->ldx, c->xv, nullptr, c->perm, deff, c->n, c->p, mu, part, dpred, c->st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pred, dpred, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
+    c->release(buf);
+    if (e != cudaSuccess) return fail(SODAGPU_E_CUDA, "genomic values: %s", cudaGetErrorString(e));
     return 0;
 }
 
@@ -1239,57 +1238,70 @@ int sodagpu_predict(int32_t nind, int32_t nloci, const void *geno, int32_t layou
         cudaGetLastError();
         return fail(SODAGPU_E_NODEVICE, "no CUDA device visible");
     }
-    cudaStream_t st;
+    cudaStream_t st = nullptr, stc = nullptr;   // kernels, copies of a .bed payload
     CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     const int n = nind, p = nloci;
-    const int ldx = (int)round_up((size_t)n, 128);
-    int8_t *G = nullptr;
-    double *dfreq = nullptr, *xv = nullptr, *deff = nullptr, *part = nullptr, *dpred = nullptr;
-    int32_t *perm = nullptr;
-    uint8_t *tmp = nullptr;
-    const int nsplit = 32;
-    std::vector<int32_t> ident(p);
-    for (int k = 0; k < p; ++k) ident[k] = k;
+    const bool bed = (layout & 0xff) != SODAGPU_GENO_CODES, on_dev = (layout & SODAGPU_GENO_DEVICE_PTR) != 0;
+    const cudaMemcpyKind mk = on_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    const size_t rec = ((size_t)n + 3) / 4, ldx = round_up((size_t)n, 128);
+    // A .bed payload goes over in up to four pieces of at least 8 MB (the copy then runs at nearly its full rate,
+    // 160 GB/s), each used by its kernel while the next is copied; their splits together are twice a single
+    // kernel's, so that the last one still fills half of the SMs.  On the device it is used where it is.
+    const bool copied = !(bed && on_dev);
+    const int pieces = bed && copied ? (int)std::max<size_t>(1, std::min<size_t>({(size_t)4, rec * p >> 23, (size_t)p})) : 1;
+    const int per = (p + pieces - 1) / pieces, base = zb_dgv_splits(n, p);
+    const int splits = pieces == 1 ? base : std::max(1, std::min(2 * base / pieces, zb_dgv_splits(n, per)));
+    // one allocation: the genotypes (a .bed payload is used as it is), then the vectors and the splits' sums
+    const size_t gbytes = copied ? round_up(bed ? rec * p : (size_t)p * ldx, 256) : 0;
+    const size_t nd = (size_t)3 * p + n + (size_t)pieces * splits * n;
+    uint8_t *buf = nullptr;
+    int h_bad = 0;
+    cudaEvent_t ev = nullptr;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    chk(cudaMalloc(&G, (size_t)p * ldx));
-    chk(cudaMalloc(&dfreq, sizeof(double) * p));
-    chk(cudaMalloc(&xv, sizeof(double) * 4 * p));
-    chk(cudaMalloc(&deff, sizeof(double) * p));
-    chk(cudaMalloc(&part, sizeof(double) * nsplit * ldx));
-    chk(cudaMalloc(&dpred, sizeof(double) * n));
-    chk(cudaMalloc(&perm, sizeof(int32_t) * p));
-    if (e == cudaSuccess) chk(cudaMemsetAsync(G, 0, (size_t)p * ldx, st));
-    const bool on_dev = (layout & SODAGPU_GENO_DEVICE_PTR) != 0;
-    const cudaMemcpyKind mk = on_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    chk(cudaMalloc(&buf, gbytes + sizeof(double) * nd + 256));
     if (e == cudaSuccess) {
-        if ((layout & 0xff) == SODAGPU_GENO_CODES) {
-            chk(cudaMemcpy2DAsync(G, ldx, geno, n, n, p, mk, st));
+        double *dfreq = reinterpret_cast<double *>(buf + gbytes), *deff = dfreq + p, *fcodes = deff + p;
+        double *dpred = fcodes + p, *part = dpred + n;
+        int *bad = reinterpret_cast<int *>(buf + gbytes + sizeof(double) * nd);
+        chk(cudaMemcpyAsync(dfreq, freq, sizeof(double) * p, cudaMemcpyHostToDevice, st));
+        chk(cudaMemcpyAsync(deff, effects, sizeof(double) * p, cudaMemcpyHostToDevice, st));
+        if (bed) {
+            chk(cudaStreamCreateWithFlags(&stc, cudaStreamNonBlocking));
+            chk(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+            int nsplit = 0;
+            for (int k = 0; k < p && e == cudaSuccess; k += per) {
+                const int m = std::min(per, p - k);
+                const uint8_t *src = (copied ? buf : (const uint8_t *)geno) + rec * k;
+                if (copied) {
+                    chk(cudaMemcpyAsync(buf + rec * k, (const uint8_t *)geno + rec * k, rec * m, mk, stc));
+                    chk(cudaEventRecord(ev, stc));
+                    chk(cudaStreamWaitEvent(st, ev, 0));
+                    if (e != cudaSuccess) break;
+                }
+                const int s = zb_dgv_bed(src, dfreq + k, deff + k, n, m, part + (size_t)nsplit * n, splits, st);
+                if (s < 0) chk(cudaErrorLaunchFailure);
+                nsplit += s;
+            }
+            if (e == cudaSuccess) chk(zb_dgv_sum(part, n, nsplit, mu, dpred, st));
         } else {
-            const size_t rec = ((size_t)n + 3) / 4;
-            chk(cudaMalloc(&tmp, rec * p));
-            if (e == cudaSuccess) chk(cudaMemcpyAsync(tmp, geno, rec * p, mk, st));
-            if (e == cudaSuccess) chk(zb_decode_bed(tmp, n, p, G, ldx, st));
+            int8_t *G = reinterpret_cast<int8_t *>(buf);
+            chk(cudaMemsetAsync(G, 0, (size_t)p * ldx, st));
+            chk(cudaMemcpy2DAsync(G, ldx, geno, n, n, p, mk, st));
+            // codes outside 0..2 are an error, as in sodagpu_load_genotypes: counted on the device
+            chk(cudaMemsetAsync(bad, 0, sizeof(int), st));
+            if (e == cudaSuccess) chk(zb_freq(G, n, p, (int)ldx, fcodes, bad, st));
+            chk(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+            if (e == cudaSuccess) chk(zb_dgv(G, (int)ldx, nullptr, dfreq, nullptr, deff, n, p, mu, part, dpred, st));
         }
+        if (e == cudaSuccess) chk(cudaMemcpyAsync(pred, dpred, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+        // whatever failed, nothing may still be reading or writing the buffers
+        if (stc) chk(cudaStreamSynchronize(stc));
+        chk(cudaStreamSynchronize(st));
     }
-    // codes outside 0..2 are an error, as in sodagpu_load_genotypes: counted on the device (k_freq, into
-    // the xv buffer, which is written again below)
-    int *bad = nullptr, h_bad = 0;
-    chk(cudaMalloc(&bad, sizeof(int)));
-    if (e == cudaSuccess) chk(cudaMemsetAsync(bad, 0, sizeof(int), st));
-    if (e == cudaSuccess) chk(zb_freq(G, n, p, ldx, xv, bad, st));
-    if (e == cudaSuccess) chk(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (e == cudaSuccess) chk(cudaStreamSynchronize(st));
-    if (e == cudaSuccess) chk(cudaMemcpyAsync(dfreq, freq, sizeof(double) * p, cudaMemcpyHostToDevice, st));
-    if (e == cudaSuccess) chk(cudaMemcpyAsync(deff, effects, sizeof(double) * p, cudaMemcpyHostToDevice, st));
-    if (e == cudaSuccess) chk(cudaMemcpyAsync(perm, ident.data(), sizeof(int32_t) * p, cudaMemcpyHostToDevice, st));
-    if (e == cudaSuccess) chk(zb_xv(dfreq, perm, p, xv, st));
-    if (e == cudaSuccess) chk(zb_dgv(G, ldx, xv, nullptr, deff, n, p, mu, part, nsplit, dpred, st));
-    if (e == cudaSuccess) chk(cudaMemcpyAsync(pred, dpred, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    if (e == cudaSuccess) chk(cudaStreamSynchronize(st));
-    cudaFree(G); cudaFree(dfreq); cudaFree(xv); cudaFree(deff); cudaFree(part); cudaFree(dpred); cudaFree(perm);
-    cudaFree(tmp);
-    cudaFree(bad);
+    cudaFree(buf);
+    if (ev) cudaEventDestroy(ev);
+    if (stc) cudaStreamDestroy(stc);
     cudaStreamDestroy(st);
     if (e != cudaSuccess) return fail(SODAGPU_E_CUDA, "prediction failed: %s", cudaGetErrorString(e));
     if (h_bad) return fail(SODAGPU_E_ARG, "%d genotype codes outside 0..2", h_bad);

@@ -21,9 +21,9 @@
 // that resets a device must not call this entry point on it again in the
 // same process.
 //
-// The columns are summed in nsplit = min(32, SCRATCH / nind, nloci) splits,
-// the same 32 as sodagpu_predict up to nind = 65,536; above that the
-// summation order differs and so can the last bits of the result.  Codes
+// The columns are summed in the splits of dgv_splits (dgv.cuh), the same as
+// sodagpu_predict's while nind times their number fits the scratch, and in
+// fewer above that: the last bits of the result can differ then.  Codes
 // outside 0..2 count as 1, the value load_geno gives a missing call
 // (utilities.f90:446-449); sodagpu_predict rejects them instead.
 #include <cuda_runtime.h>
@@ -32,69 +32,16 @@
 #include <mutex>
 
 #include "../../include/sodagpu.h"
+#include "dgv.cuh"
 
 namespace {
 
-constexpr int kSplitMax = 32;     // column splits of the partial sums
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) double g_dgv_scratch[SODAGPU_NOALLOC_SCRATCH];
 
 std::mutex g_scratch_mu;
 double *g_scratch_ptr[kMaxDevices];   // device address per device, 0 until looked up
-
-// partial[s][i] = sum over the columns of split s of x_ij * effects_j, with
-// x_ij = (code - 2p_j) / sqrt(2p_j(1-p_j)) (0 for monomorphic SNPs); the
-// three values of each column are formed in shared memory per chunk.
-__global__ void __launch_bounds__(256) k_dgv_noalloc_partial(const int8_t *codes, int ldg, const double *freq,
-                                                             const double *eff, int n, int p, int nsplit,
-                                                             double *part)
-{
-    __shared__ double s_x[256][3];
-    __shared__ double s_e[256];
-    const int i = blockIdx.x * 256 + threadIdx.x, s = blockIdx.y;
-    const int per = (p + nsplit - 1) / nsplit;
-    const int k0 = s * per, k1 = min(p, k0 + per);
-    const double eps = 2.220446049250313e-16;
-    double acc = 0.0;
-    for (int c0 = k0; c0 < k1; c0 += 256) {
-        const int cnt = min(256, k1 - c0);
-        __syncthreads();
-        if (threadIdx.x < cnt) {
-            const int k = c0 + threadIdx.x;
-            const double f = freq[k];
-            s_e[threadIdx.x] = eff[k];
-            if (f < eps || (1.0 - f) < eps) {
-                s_x[threadIdx.x][0] = s_x[threadIdx.x][1] = s_x[threadIdx.x][2] = 0.0;
-            } else {
-                const double twop = __dmul_rn(2.0, f);
-                const double sd = sqrt(__dmul_rn(twop, __dsub_rn(1.0, f)));
-                s_x[threadIdx.x][0] = __ddiv_rn(__dsub_rn(0.0, twop), sd);
-                s_x[threadIdx.x][1] = __ddiv_rn(__dsub_rn(1.0, twop), sd);
-                s_x[threadIdx.x][2] = __ddiv_rn(__dsub_rn(2.0, twop), sd);
-            }
-        }
-        __syncthreads();
-        if (i < n) {
-            for (int q = 0; q < cnt; ++q) {
-                const double e = s_e[q];
-                if (e == 0.0) continue;
-                const int code = codes[(size_t)(c0 + q) * ldg + i];
-                acc = acc + s_x[q][code < 0 ? 1 : (code > 2 ? 1 : code)] * e;
-            }
-        }
-    }
-    if (i < n) part[(size_t)s * n + i] = acc;
-}
-
-__global__ void k_dgv_noalloc_final(const double *part, int n, int nsplit, double mu, double *pred)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double d = 0.0;
-    for (int s = 0; s < nsplit; ++s) d = d + part[(size_t)s * n + i];
-    pred[i] = mu + d;
-}
 
 }  // namespace
 
@@ -104,9 +51,9 @@ extern "C" int sodagpu_compute_dgv_noalloc(int32_t nind, int32_t nloci, const in
 {
     if (nind < 1 || nloci < 1 || ldg < nind || !codes || !freq || !effects || !pred) return SODAGPU_E_ARG;
     if ((int64_t)nind > (int64_t)SODAGPU_NOALLOC_SCRATCH) return SODAGPU_E_ARG;   // beyond the scratch maximum
-    int nsplit = (int)((int64_t)SODAGPU_NOALLOC_SCRATCH / nind);
-    nsplit = nsplit > kSplitMax ? kSplitMax : nsplit;
-    nsplit = nsplit > nloci ? nloci : nsplit;
+    int nsplit = soda::dgv_splits(nind, nloci);
+    if ((int64_t)nsplit * nind > (int64_t)SODAGPU_NOALLOC_SCRATCH)
+        nsplit = (int)((int64_t)SODAGPU_NOALLOC_SCRATCH / nind);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
@@ -127,26 +74,11 @@ extern "C" int sodagpu_compute_dgv_noalloc(int32_t nind, int32_t nloci, const in
         }
         scratch = g_scratch_ptr[dev];
     }
-    // cudaLaunchKernel reports a failed launch in its own return value, so an error the caller left
-    // pending from earlier work is neither reported as this call's failure nor cleared
-    cudaStream_t st = (cudaStream_t)stream;
-    {
-        void *args[] = {(void *)&codes, (void *)&ldg, (void *)&freq, (void *)&effects, (void *)&nind,
-                        (void *)&nloci, (void *)&nsplit, (void *)&scratch};
-        if (cudaLaunchKernel((const void *)k_dgv_noalloc_partial, dim3((nind + 255) / 256, nsplit), dim3(256), args,
-                             0, st) != cudaSuccess) {
-            cudaGetLastError();
-            return SODAGPU_E_CUDA;
-        }
-    }
-    {
-        const double *part = scratch;
-        void *args[] = {(void *)&part, (void *)&nind, (void *)&nsplit, (void *)&mu, (void *)&pred};
-        if (cudaLaunchKernel((const void *)k_dgv_noalloc_final, dim3((nind + 255) / 256), dim3(256), args, 0, st) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            return SODAGPU_E_CUDA;
-        }
+    if (soda::dgv_enqueue<soda::DGV_RAW>(reinterpret_cast<const uint8_t *>(codes), (size_t)ldg, nullptr, freq, nullptr,
+                                         effects, nind, nloci, mu, scratch, (size_t)nind, nsplit, pred,
+                                         (cudaStream_t)stream) != cudaSuccess) {
+        cudaGetLastError();
+        return SODAGPU_E_CUDA;
     }
     return 0;
 }

@@ -15,6 +15,7 @@
 // matrix W_b (N x N, column-major, ld N) lives at wofs[b].
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "dgv.cuh"
 #include "rng.cuh"
 #include "state.cuh"
 #include "zbuild.cuh"
@@ -667,33 +668,6 @@ __global__ void k_unpack_dense(const double *U64, const int64_t *uoff, const int
     }
 }
 
-// pred = mu + sum_k xv[k][G[k][i]] * eff[perm[k]], rows split over columns
-__global__ void __launch_bounds__(256) k_dgv_partial(const int8_t *G, int ldx, const double *xv, const int32_t *perm,
-                                                     const double *eff, int n, int p, int nsplit, double *part)
-{
-    const int i = blockIdx.x * 256 + threadIdx.x, s = blockIdx.y;
-    if (i >= n) return;
-    const int per = (p + nsplit - 1) / nsplit;
-    const int k0 = s * per, k1 = min(p, k0 + per);
-    double acc = 0.0;
-    for (int k = k0; k < k1; ++k) {
-        const double e = eff[perm ? perm[k] : k];
-        if (e == 0.0) continue;
-        const int code = G[(size_t)k * ldx + i];
-        acc = acc + xv[(size_t)k * 4 + ((unsigned)code <= 2u ? code : 1)] * e;   // codes are validated on entry
-    }
-    part[(size_t)s * ldx + i] = acc;
-}
-
-__global__ void k_dgv_final(const double *part, int ldx, int n, int nsplit, double mu, double *pred)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double d = 0.0;
-    for (int s = 0; s < nsplit; ++s) d = d + part[(size_t)s * ldx + i];
-    pred[i] = mu + d;
-}
-
 // ---------------------------------------------------------------------------
 // host wrappers
 // ---------------------------------------------------------------------------
@@ -822,12 +796,24 @@ cudaError_t zb_unpack_dense(const double *U64, const int64_t *uoff, const int32_
     return cudaGetLastError();
 }
 
-cudaError_t zb_dgv(const int8_t *G, int ldx, const double *xv, const int32_t *perm, const double *eff, int n, int p,
-                   double mu, double *part, int nsplit, double *pred, cudaStream_t st)
+int zb_dgv_splits(int n, int p) { return dgv_splits(n, p); }
+
+cudaError_t zb_dgv(const int8_t *G, int ldx, const double *xv, const double *freq, const int32_t *perm,
+                   const double *eff, int n, int p, double mu, double *part, double *pred, cudaStream_t st)
 {
-    k_dgv_partial<<<dim3((n + 255) / 256, nsplit), 256, 0, st>>>(G, ldx, xv, perm, eff, n, p, nsplit, part);
-    k_dgv_final<<<(n + 255) / 256, 256, 0, st>>>(part, ldx, n, nsplit, mu, pred);
-    return cudaGetLastError();
+    return dgv_enqueue<DGV_PADDED>(reinterpret_cast<const uint8_t *>(G), ldx, xv, freq, perm, eff, n, p, mu, part, n,
+                                   dgv_splits(n, p), pred, st);
+}
+
+int zb_dgv_bed(const uint8_t *bed, const double *freq, const double *eff, int n, int p, double *part, int nsplit,
+               cudaStream_t st)
+{
+    return dgv_enqueue_tab<DGV_BED>(bed, ((size_t)n + 3) / 4, nullptr, freq, nullptr, eff, n, p, part, n, nsplit, st);
+}
+
+cudaError_t zb_dgv_sum(const double *part, int n, int nsplit, double mu, double *pred, cudaStream_t st)
+{
+    return dgv_enqueue_sum(part, n, n, nsplit, mu, pred, st);
 }
 
 }  // namespace soda

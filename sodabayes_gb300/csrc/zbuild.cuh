@@ -34,7 +34,15 @@ cudaError_t zb_pack(const double *W, const int64_t *wofs, const int32_t *blk_ls,
                     __nv_bfloat16 *Uhi, __nv_bfloat16 *Ulo, cudaStream_t st);
 cudaError_t zb_unpack_dense(const double *U64, const int64_t *uoff, const int32_t *ulen, int p, int bs, double *xa,
                             cudaStream_t st);
-cudaError_t zb_dgv(const int8_t *G, int ldx, const double *xv, const int32_t *perm, const double *eff, int n, int p,
-                   double mu, double *part, int nsplit, double *pred, cudaStream_t st);
+// Genomic values (dgv.cuh): part holds zb_dgv_splits(n, p) * n doubles.  The codes of a context are centred by
+// xv (nullptr: by freq), a .bed payload by freq.
+int zb_dgv_splits(int n, int p);
+cudaError_t zb_dgv(const int8_t *G, int ldx, const double *xv, const double *freq, const int32_t *perm,
+                   const double *eff, int n, int p, double mu, double *part, double *pred, cudaStream_t st);
+// The splits' sums of p SNPs of a .bed payload (their records, frequencies and effects): returns how many were
+// written, at most nsplit, or -1; then mu + the sum of all of them.
+int zb_dgv_bed(const uint8_t *bed, const double *freq, const double *eff, int n, int p, double *part, int nsplit,
+               cudaStream_t st);
+cudaError_t zb_dgv_sum(const double *part, int n, int nsplit, double mu, double *pred, cudaStream_t st);
 
 }  // namespace soda

@@ -75,13 +75,23 @@ __device__ __forceinline__ float code_to_f32(uint32_t w, int k)
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)k)) - 8388608.0f;
 }
 
+// Threads of a draw CTA.  With the CUDA-core rhs a subset has N * CT draws, few for one or two chains, and in the
+// FP64 mode each is some hundred instructions of the FP64 pipe, which takes a warp's instruction 16 cycles: the draws
+// are spread over the SMs, a warp each (two for 4 chains and more, whose CTAs need at least CT threads).  N = 935, one
+// FP64 chain, the kernel by itself: 34 us, against 42 us in four CTAs of 256 threads (most of it now lies before the
+// dependency wait: an iteration of 10 subsets takes 527 us, 636 us without draw_ahead, 745 us with neither).
+// The tensor-core path has C >= 4 and FP32 draws: 256 threads fill the SMs.
+template <int CT, bool TC>
+struct DrawThreads { static constexpr int v = TC ? 256 : (CT <= 2 ? 32 : 64); };
+
 // Per-SNP draws of one subset (models.f90:146-162, 211-256, 350-413) after
 // the rhs kernel left its split partial sums in rpx/rpu: one thread per
-// (SNP, chain) pair; a CTA takes 256/CT consecutive SNPs, its threads
+// (SNP, chain) pair; a CTA takes NT/CT consecutive SNPs, its NT threads
 // SNP-fastest so that the chain-major arrays (partial sums, g, class, delta
 // and its split) are read and written in contiguous runs.
-// Every load a draw needs is issued up front: the SNP's metadata and state,
-// and the partial sums of all splits at once (added in split order).  With
+// What does not depend on the right-hand sides (draw_sub, draw_ahead) runs before
+// the dependency wait; then the partial sums of all splits are loaded at once and
+// added in split order.  With
 // TC the kernel also writes what the tensor-core update reads (and takes the
 // split count of each SNP's tile from D.rtab): the bf16
 // three-way split of delta/sd per chain (dsplit; pairs up to `span`, past the
@@ -89,14 +99,15 @@ __device__ __forceinline__ float code_to_f32(uint32_t w, int k)
 template <int MODE, int CT, bool TC>
 __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int ksplit, int span)
 {
+    constexpr int NT = DrawThreads<CT, TC>::v;
     __shared__ double s_rs[CT];   // sum(r) per chain (FP8 centring)
-    __shared__ double s_k[256];
-    __shared__ float s_kf[256];   // tensor-core path: x0_j delta_j in FP32
-    __shared__ DrawPre s_pre[CT];   // chain constants in FP32 (the FP64 pipe is narrow)
-    __shared__ float s_zzv[CT];
-    __shared__ float s_d32[256];
-    __shared__ int s_nzf[256 / CT];
-    constexpr int SPC = 256 / CT;   // SNPs per CTA
+    __shared__ double s_k[NT];
+    __shared__ float s_kf[NT];    // tensor-core path: x0_j delta_j in FP32
+    typedef typename std::conditional<MODE == SODAGPU_FP64, double, float>::type T;   // of the draws
+    __shared__ DrawSub<T> s_sub[CT];
+    __shared__ float s_d32[NT];
+    constexpr int SPC = NT / CT;    // SNPs per CTA
+    __shared__ int s_nzf[SPC];
     const int tid = threadIdx.x;
     const int jloc = tid % SPC, c = tid / SPC;
     const int jl = vb.x * SPC + jloc;
@@ -106,30 +117,24 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
     const bool act = jl < N;
     const int k = ls + (act ? jl : 0);
     const double zz = D.xxd[b];
-    // prologue, overlapping the rhs kernel: chain constants (fixed within an
-    // iteration), the SNP's metadata and state (not written by the rhs kernel)
-    if (MODE != SODAGPU_FP64 && tid < CT) {
-        draw_prefetch(D, &D.scal[tid], tid, 0, 0, s_pre[tid]);
-        s_zzv[tid] = (float)(zz / D.scal[tid].vare);
-    }
+    // prologue, overlapping the rhs kernel: the chains' constants of this subset (fixed within an iteration), the
+    // SNP's metadata and state (not written by the rhs kernel)
+    if (tid < CT * DRAW_PRE) draw_sub(D, &D.scal[tid / DRAW_PRE], tid % DRAW_PRE, zz, s_sub[tid / DRAW_PRE]);
     const int snp = act && !D.skip[k] ? D.perm[k] : -1;
     double inv = 0.0, x0 = 0.0, gold = 0.0;
     float inv32 = 0.0f;
     int cl = 0, sg = 0;
-    float vs = 0.0f;
+    T vs = (T)1.0;
     if (snp >= 0) {
         if (MODE == SODAGPU_FP8 || TC) {
             inv = D.xv[(size_t)k * 4 + 3];
             x0 = D.xv[(size_t)k * 4 + 0];
             inv32 = D.xv32[(size_t)k * 4 + 3];
         }
-        if (MODE != SODAGPU_FP64) {
-            gold = D.g[(size_t)c * D.p + snp];
-            cl = D.cls[(size_t)c * D.p + snp];
-            sg = D.grp[snp] - 1;
-            if (D.method == SODAGPU_BAYES_A || D.method == SODAGPU_BAYES_B)
-                vs = (float)D.vara_s[(size_t)c * D.p + snp];
-        }
+        gold = D.g[(size_t)c * D.p + snp];
+        cl = D.cls[(size_t)c * D.p + snp];
+        sg = D.grp[snp] - 1;
+        if (D.method == SODAGPU_BAYES_A || D.method == SODAGPU_BAYES_B) vs = (T)D.vara_s[(size_t)c * D.p + snp];
     }
     // the SNP's draw site and its first Philox block, ahead of the dependency wait
     CRng R;
@@ -144,9 +149,9 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
     if (MODE == SODAGPU_FP8 || TC) {
         // sum(r) per chain from the row-tile partial sums of the previous residual update, before
         // the dependency wait: that update is complete once this kernel runs, because the rhs
-        // kernel lets it launch only after its own dependency wait.  256/CT threads per chain
+        // kernel lets it launch only after its own dependency wait.  NT/CT threads per chain
         // take interleaved tiles, loaded 16 at a time in one batch, then added in part order
-        constexpr int PARTS = 256 / CT;
+        constexpr int PARTS = NT / CT;
         const int cc = tid / PARTS, part = tid % PARTS;
         double a = 0.0;
         for (int q0 = part; q0 < D.nr_ctas; q0 += 16 * PARTS) {
@@ -163,12 +168,14 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
     }
     __syncthreads();
     if ((MODE == SODAGPU_FP8 || TC) && tid < CT) {
-        constexpr int PARTS = 256 / CT;
+        constexpr int PARTS = NT / CT;
         double tt = 0.0;
         for (int q = 0; q < PARTS; ++q) tt += s_k[tid * PARTS + q];
         s_rs[tid] = tt;
     }
     __syncthreads();
+    DrawSnp<T> ahead;
+    if (snp >= 0 && !D.rhs_out) draw_ahead(D, s_sub[c], (T)zz, vs, R, ahead);
     // tensor-core path: the rhs is assembled in FP32 (its split sums are FP32; the FP64 pipe of
     // GB300 is narrow and also runs every double <-> float conversion)
     const float x0f = (float)x0, rsf = TC ? (float)s_rs[c] : 0.0f;
@@ -226,22 +233,9 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
     double delta = 0.0;
     if (snp >= 0) {
         if (MODE == SODAGPU_FP8 && !TC) xr = xr * inv + x0 * s_rs[c];
-        const ChainScal *S = &D.scal[c];
-        int err = 0;
-        if (MODE == SODAGPU_FP64) {
-            delta = draw_snp(D, S, c, cur_rep(D), snp, xr + ur, zz, zz / S->vare, R, &err);
-        } else {
-            DrawPre pre = s_pre[c];
-            pre.vs = vs;
-            if (D.ngroup > 1) {
-#pragma unroll
-                for (int q = 0; q < DRAW_PRE; ++q)
-                    pre.logp[q] = q < D.nmix ? (float)S->log_p[sg + q * D.ngroup] : 0.0f;
-            }
-            const float rhs = TC ? xf : (float)(xr + ur);
-            delta = draw_snp_f(D, S, c, snp, rhs, (float)zz, s_zzv[c], R, &err, gold, cl, sg, pre);
-        }
-        if (err) flag_err(D, 1);
+        const T rhs = TC ? (T)xf : (T)(xr + ur);
+        delta = draw_snp(D, &D.scal[c], c, snp, rhs, (T)zz, s_sub[c], ahead, R, gold, cl, sg);
+        if (ahead.err) flag_err(D, 1);
     }
     float delta32 = 0.0f;
     if (act) {
@@ -269,17 +263,17 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
         for (int q = 0; q < SPC; ++q) tt += s_kf[q * CT + tid];
         D.k0part[(size_t)vb.x * CT + tid] = (double)tt;
     }
-    // delta32 chain-contiguous per SNP (the CTA's block of 256 values), and the flags of SNPs whose
+    // delta32 chain-contiguous per SNP (the CTA's block of NT values), and the flags of SNPs whose
     // delta is non-zero in some chain
     if (MODE != SODAGPU_FP64) {
         const int j = vb.x * SPC + tid / CT;
-        if (j < N) D.delta32[(size_t)vb.x * 256 + tid] = s_d32[tid];
+        if (j < N) D.delta32[(size_t)vb.x * NT + tid] = s_d32[tid];
     }
     if (tid < SPC && vb.x * SPC + tid < N) D.nzflag[vb.x * SPC + tid] = s_nzf[tid];
 }
 
 template <int MODE, int CT, bool TC>
-__global__ void __launch_bounds__(256, 1) k_draw(Dev D, int b, int ksplit, int span)
+__global__ void __launch_bounds__(DrawThreads<CT, TC>::v, 1) k_draw(Dev D, int b, int ksplit, int span)
 {
     draw_body<MODE, CT, TC>(D, vb_native(), b, ksplit, span);
 }

@@ -136,61 +136,9 @@ __host__ __device__ __forceinline__ double crng_unit(CRng &s)
 #endif
 }
 
-// rand_normal (parallelrng.f90:264-277)
-__device__ __forceinline__ double d_rnorm(double mean, double sd, CRng &s)
-{
-    if (sd <= 0.0) return mean;
-    const double u1 = crng_unit(s), u2 = crng_unit(s);
-    const double rr = sqrt(-2.0 * log(u1));
-    const double th = 2.0 * SODA_REF_PI * u2;
-    return mean + sd * rr * sin(th);
-}
-
-// rand_gamma (parallelrng.f90:294-333).  The rejection loop is bounded; on
-// the (practically impossible) exhaustion *err is set and the last candidate
-// returned.
-__device__ __forceinline__ double d_rgamma(double shape, double scale, CRng &s, int *err)
-{
-    const bool small = shape < 1.0;
-    const double sh = small ? shape + 1.0 : shape;
-    const double sc = small ? 1.0 : scale;
-    const double d = sh - 1.0 / 3.0;
-    const double c = 1.0 / sqrt(9.0 * d);
-    double res = d;
-    int tries = 0;
-    for (;;) {
-        double x = d_rnorm(0.0, 1.0, s);
-        double v = 1.0 + c * x;
-        while (v <= 0.0 && tries < 100000) {
-            x = d_rnorm(0.0, 1.0, s);
-            v = 1.0 + c * x;
-            ++tries;
-        }
-        v = v * v * v;
-        const double u = crng_unit(s);
-        const double xsq = x * x;
-        res = sc * d * v;
-        if ((u < 1.0 - 0.0331 * xsq * xsq) || (log(u) < 0.5 * xsq + d * (1.0 - v + log(v)))) break;
-        if (++tries >= 100000) { if (err) *err = 1; break; }
-    }
-    if (small) {
-        // shape < 1: g ~ gamma(shape+1, 1), then scale*g*w**(1/shape)
-        const double w = crng_unit(s);
-        return scale * res * pow(w, 1.0 / shape);
-    }
-    return res;
-}
-
-// rand_scaled_inverse_chi_square (parallelrng.f90:348-362)
-__device__ __forceinline__ double d_rscinvchi2(double dof, double scale, CRng &s, int *err)
-{
-    const double shape = 0.5 * dof, sc = 0.5 * dof * scale;
-    return 1.0 / d_rgamma(shape, 1.0 / sc, s, err);
-}
-
 // ---------------------------------------------------------------------------
-// FP32 transforms for the reduced-precision sweeps (same counter streams).
-// Uniforms take the top 24 bits of each word, offset by half a unit so they
+// FP32 uniforms of the reduced-precision sweeps (same counter streams): they
+// take the top 24 bits of each word, offset by half a unit so they
 // lie strictly inside (0,1): log(u) is always finite.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float crng_unit_f(CRng &s)
@@ -199,50 +147,122 @@ __device__ __forceinline__ float crng_unit_f(CRng &s)
     return ((float)(uint32_t)(crng_u64(s) >> 40) + 0.5f) * 5.9604644775390625e-8f;
 }
 
-__device__ __forceinline__ float d_rnorm_f(float mean, float sd, CRng &s)
-{
-    if (sd <= 0.0f) return mean;
-    const float u1 = crng_unit_f(s), u2 = crng_unit_f(s);
-    const float rr = sqrtf(-2.0f * logf(u1));
-    const float th = 6.2831854820251465f * u2;
-    return mean + sd * rr * sinf(th);
-}
+// ---------------------------------------------------------------------------
+// Distribution transforms, FP64 (the reference's) and FP32 with the same
+// streams.  Each is in two parts, so that a kernel can take the uniforms and
+// do the transcendental arithmetic before the mean, the standard deviation
+// or the scale is known: the parts' values together are the plain draw's,
+// bit for bit.
+// ---------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ T crng_unit_t(CRng &s);
+template <>
+__device__ __forceinline__ double crng_unit_t<double>(CRng &s) { return crng_unit(s); }
+template <>
+__device__ __forceinline__ float crng_unit_t<float>(CRng &s) { return crng_unit_f(s); }
 
-__device__ __forceinline__ float d_rgamma_f(float shape, float scale, CRng &s, int *err)
+__device__ __forceinline__ double t_log(double x) { return log(x); }
+__device__ __forceinline__ float t_log(float x) { return logf(x); }
+__device__ __forceinline__ double t_exp(double x) { return exp(x); }
+__device__ __forceinline__ float t_exp(float x) { return expf(x); }
+__device__ __forceinline__ double t_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ float t_sqrt(float x) { return sqrtf(x); }
+__device__ __forceinline__ double t_sin(double x) { return sin(x); }
+__device__ __forceinline__ float t_sin(float x) { return sinf(x); }
+__device__ __forceinline__ double t_pow(double x, double y) { return pow(x, y); }
+__device__ __forceinline__ float t_pow(float x, float y) { return powf(x, y); }
+
+// rand_normal (parallelrng.f90:264-277): mean + sd * rr * sn; takes no
+// uniforms when sd <= 0.
+template <typename T>
+struct NormalPre {
+    T rr, sn;
+};
+template <typename T>
+__device__ __forceinline__ NormalPre<T> normal_pre(CRng &s)
 {
-    const bool small = shape < 1.0f;
-    const float sh = small ? shape + 1.0f : shape;
-    const float sc = small ? 1.0f : scale;
-    const float d = sh - 1.0f / 3.0f;
-    const float c = 1.0f / sqrtf(9.0f * d);
-    float res = d;
+    const T u1 = crng_unit_t<T>(s), u2 = crng_unit_t<T>(s);
+    NormalPre<T> z;
+    z.rr = t_sqrt((T)-2.0 * t_log(u1));
+    z.sn = t_sin((T)(2.0 * SODA_REF_PI) * u2);
+    return z;
+}
+template <typename T>
+__device__ __forceinline__ T normal_from(T mean, T sd, const NormalPre<T> &z)
+{
+    return mean + sd * z.rr * z.sn;
+}
+template <typename T>
+__device__ __forceinline__ T t_rnorm(T mean, T sd, CRng &s)
+{
+    if (sd <= (T)0.0) return mean;
+    return normal_from(mean, sd, normal_pre<T>(s));
+}
+__device__ __forceinline__ double d_rnorm(double mean, double sd, CRng &s) { return t_rnorm<double>(mean, sd, s); }
+
+// rand_gamma (parallelrng.f90:294-333): scale * d * v, times w**(1/shape) for
+// a shape below 1.  The rejection loop is bounded; on the (practically
+// impossible) exhaustion *err is set and the last candidate kept.
+template <typename T>
+struct GammaPre {
+    T d, v, wp;
+    bool small;
+};
+template <typename T>
+__device__ __forceinline__ GammaPre<T> gamma_pre(T shape, CRng &s, int *err)
+{
+    GammaPre<T> g;
+    g.small = shape < (T)1.0;
+    const T sh = g.small ? shape + (T)1.0 : shape;
+    g.d = sh - (T)1.0 / (T)3.0;
+    const T c = (T)1.0 / t_sqrt((T)9.0 * g.d);
     int tries = 0;
     for (;;) {
-        float x = d_rnorm_f(0.0f, 1.0f, s);
-        float v = 1.0f + c * x;
-        while (v <= 0.0f && tries < 100000) {
-            x = d_rnorm_f(0.0f, 1.0f, s);
-            v = 1.0f + c * x;
+        T x = t_rnorm<T>((T)0.0, (T)1.0, s);
+        T v = (T)1.0 + c * x;
+        while (v <= (T)0.0 && tries < 100000) {
+            x = t_rnorm<T>((T)0.0, (T)1.0, s);
+            v = (T)1.0 + c * x;
             ++tries;
         }
         v = v * v * v;
-        const float u = crng_unit_f(s);
-        const float xsq = x * x;
-        res = sc * d * v;
-        if ((u < 1.0f - 0.0331f * xsq * xsq) || (logf(u) < 0.5f * xsq + d * (1.0f - v + logf(v)))) break;
+        const T u = crng_unit_t<T>(s);
+        const T xsq = x * x;
+        g.v = v;
+        if ((u < (T)1.0 - (T)0.0331 * xsq * xsq) ||
+            (t_log(u) < (T)0.5 * xsq + g.d * ((T)1.0 - v + t_log(v))))
+            break;
         if (++tries >= 100000) { if (err) *err = 1; break; }
     }
-    if (small) {
-        const float w = crng_unit_f(s);
-        return scale * res * powf(w, 1.0f / shape);
+    g.wp = (T)1.0;
+    if (g.small) {
+        // shape < 1: g ~ gamma(shape+1, 1), then scale*g*w**(1/shape)
+        const T w = crng_unit_t<T>(s);
+        g.wp = t_pow(w, (T)1.0 / shape);
     }
-    return res;
+    return g;
+}
+template <typename T>
+__device__ __forceinline__ T gamma_from(T scale, const GammaPre<T> &g)
+{
+    return g.small ? scale * (g.d * g.v) * g.wp : scale * g.d * g.v;
+}
+__device__ __forceinline__ double d_rgamma(double shape, double scale, CRng &s, int *err)
+{
+    return gamma_from(scale, gamma_pre<double>(shape, s, err));
 }
 
-__device__ __forceinline__ float d_rscinvchi2_f(float dof, float scale, CRng &s, int *err)
+// rand_scaled_inverse_chi_square (parallelrng.f90:348-362) from the gamma
+// draw of shape dof / 2
+template <typename T>
+__device__ __forceinline__ T scinvchi2_from(T dof, T scale, const GammaPre<T> &g)
 {
-    const float shape = 0.5f * dof, sc = 0.5f * dof * scale;
-    return 1.0f / d_rgamma_f(shape, 1.0f / sc, s, err);
+    const T sc = (T)0.5 * dof * scale;
+    return (T)1.0 / gamma_from((T)1.0 / sc, g);
+}
+__device__ __forceinline__ double d_rscinvchi2(double dof, double scale, CRng &s, int *err)
+{
+    return scinvchi2_from(dof, scale, gamma_pre<double>(0.5 * dof, s, err));
 }
 
 }  // namespace soda

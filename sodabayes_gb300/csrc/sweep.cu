@@ -115,249 +115,199 @@ __device__ __forceinline__ void crng_site(CRng &R, const Dev &D, int c, int rep,
 }
 
 // ---------------------------------------------------------------------------
-// Per-SNP conditional draw inside a subset.  Returns delta = g_old - g_new.
-// Restates models.f90:146-161 (BayesA), 211-255 (BayesB), 350-412 (C/Cpi/R/Rc).
+// Per-SNP conditional draw inside a subset (models.f90:146-161 BayesA, 211-255
+// BayesB, 350-412 C/Cpi/R/Rc), in FP64, or in FP32 arithmetic for the FP32/FP8
+// sweeps (GB300 executes FP64 at a small fraction of its FP32 rate); the state
+// stays FP64.
+//
+// A draw is a chain of dependent transcendental operations on the critical path
+// of every subset, and most of it does not depend on the right-hand side: what
+// a subset's draws share (DrawSub, one per chain) and what is the SNP's own
+// (DrawSnp: its uniforms, the normal and gamma variates, the locus variance's
+// terms) is computed before the rhs kernel has finished.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double draw_snp(const Dev &D, const ChainScal *S, int c, int rep, int snploc,
-                           double rhs, double zz, double zz_vare, CRng &R, int *err)
+constexpr int DRAW_PRE = 4;   // mixture classes with prefetched constants
+
+template <typename T>
+struct DrawSub {
+    T vare, scale_va, zz_vare;
+    // class k: log pi of group 1, log(gamma_k sigma2_g zz / sigma2_e + 1), the denominators of the score and
+    // of the conditional mean, the conditional standard deviation
+    T logp[DRAW_PRE], ld[DRAW_PRE], den[DRAW_PRE], v1[DRAW_PRE], sd[DRAW_PRE];
+};
+
+// Class k of chain S in a subset with d = zz (k = 0 also fills what all classes share).
+template <typename T>
+__device__ __forceinline__ void draw_sub(const Dev &D, const ChainScal *S, int k, double zz, DrawSub<T> &q)
+{
+    const T vare = (T)S->vare, zt = (T)zz;
+    const T zz_vare = (T)(zz / S->vare);
+    if (k == 0) {
+        q.vare = vare;
+        q.scale_va = (T)S->scale_va;
+        q.zz_vare = zz_vare;
+    }
+    const bool in = k < D.nmix;
+    q.logp[k] = in ? (T)S->log_p[k * D.ngroup] : (T)0.0;
+    const T gp = in ? (T)S->gp[k] : (T)0.0;
+    q.ld[k] = t_log(gp * zz_vare + (T)1.0);
+    q.den[k] = zt + (in ? (T)S->vare_gp[k] : (T)0.0);
+    q.v1[k] = zt + vare / gp;
+    q.sd[k] = t_sqrt(vare / q.v1[k]);
+}
+
+template <typename T>
+struct DrawSnp {
+    T u;                   // class uniform (BayesB and the mixtures)
+    NormalPre<T> z;
+    GammaPre<T> gam;       // BayesA/B
+    T ld, den, sd, sdv;    // BayesA/B: from the locus variance
+    bool plain;            // a standard deviation is 0: the draws follow the plain order at their use
+    int err;
+};
+
+// Advances R past the uniforms that the SNP's draw takes (up to the class uniform when `plain`).
+template <typename T>
+__device__ __forceinline__ void draw_ahead(const Dev &D, const DrawSub<T> &q, T zz, T vs, CRng &R, DrawSnp<T> &a)
+{
+    const int m = D.method;
+    a.plain = false;
+    a.err = 0;
+    if (m == SODAGPU_BAYES_A || m == SODAGPU_BAYES_B) {
+        a.den = zz + q.vare / vs;
+        a.sd = t_sqrt(q.vare / a.den);
+        a.plain = a.sd <= (T)0.0;
+        if (m == SODAGPU_BAYES_B) {
+            a.ld = t_log(vs * q.zz_vare + (T)1.0);
+            a.sdv = t_sqrt(vs);
+            a.plain = a.plain || a.sdv <= (T)0.0;
+            a.u = crng_unit_t<T>(R);
+        }
+        if (a.plain) return;
+        a.z = normal_pre<T>(R);
+        a.gam = gamma_pre<T>((T)0.5 * ((T)D.df_va + (T)1.0), R, &a.err);
+        return;
+    }
+    a.u = crng_unit_t<T>(R);
+    a.z = normal_pre<T>(R);
+}
+
+// Returns delta = g_old - g_new; gold = g and cl = class of the SNP in this chain, sg = its group - 1.
+template <typename T>
+__device__ __forceinline__ double draw_snp(const Dev &D, const ChainScal *S, int c, int snploc, T rhs, T zz,
+                                           const DrawSub<T> &q, DrawSnp<T> &a, CRng &R, double gold, int cl, int sg)
 {
     const size_t o = (size_t)c * D.p + snploc;
-    const double vare = S->vare;
-    double gk = D.g[o];
-    const double gold = gk;
-    const int m = D.method;
-    if (m == SODAGPU_BAYES_A) {
-        rhs = rhs + zz * gk;
-        const double vs = D.vara_s[o];
-        const double v1 = zz + vare / vs;
-        gk = d_rnorm(rhs / v1, sqrt(vare / v1), R);
-        D.g[o] = gk;
-        const double scale = (gk * gk + S->scale_va * D.df_va) / (D.df_va + 1.0);
-        D.vara_s[o] = d_rscinvchi2(D.df_va + 1.0, scale, R, err);
-        return gold - gk;
-    }
-    const int cl = D.cls[o];
-    if (cl > 1) rhs = rhs + zz * gk;
-    const int ng = D.ngroup;
-    if (m == SODAGPU_BAYES_B) {
-        const double vs = D.vara_s[o];
-        const double s1 = S->log_p[0];
-        const double logdetV = log(vs * zz_vare + 1.0);
-        const double uhat = rhs / (zz + vare / vs);
-        const double s2 = -0.5 * (logdetV - (rhs * uhat / vare)) + S->log_p[ng];
-        const double clike = s1 - s2;
-        double sk;
-        if (clike > 700) sk = 0.0;
-        else if (clike < -700) sk = 1.0;
-        else sk = 1.0 / (1.0 + exp(clike));
-        const double u = crng_unit(R);
-        const int flag = u < sk ? 2 : 1;
-        double gnew;
-        if (flag == 1) {
-            gk = d_rnorm(0.0, sqrt(vs), R);
-            gnew = 0.0;
-        } else {
-            const double v1 = zz + vare / vs;
-            gk = d_rnorm(rhs / v1, sqrt(vare / v1), R);
-            gnew = gk;
+    const T vare = q.vare;
+    T gk = (T)gold;
+    const int m = D.method, ng = D.ngroup;
+    if (m == SODAGPU_BAYES_A || m == SODAGPU_BAYES_B) {
+        const T df_va = (T)D.df_va;
+        int flag = 2;
+        if (m == SODAGPU_BAYES_A || cl > 1) rhs = rhs + zz * gk;
+        if (m == SODAGPU_BAYES_B) {
+            const T s1 = q.logp[0];
+            const T uhat = rhs / a.den;
+            const T s2 = (T)-0.5 * (a.ld - (rhs * uhat / vare)) + q.logp[1];
+            const T clike = s1 - s2;
+            T sk;
+            if (clike > (T)700.0) sk = (T)0.0;
+            else if (clike < (T)-700.0) sk = (T)1.0;
+            else sk = (T)1.0 / ((T)1.0 + t_exp(clike));
+            flag = a.u < sk ? 2 : 1;
         }
+        const T mean = flag == 1 ? (T)0.0 : rhs / a.den, sd = flag == 1 ? a.sdv : a.sd;
+        if (a.plain) {
+            gk = t_rnorm<T>(mean, sd, R);
+            a.gam = gamma_pre<T>((T)0.5 * (df_va + (T)1.0), R, &a.err);
+        } else {
+            gk = normal_from(mean, sd, a.z);
+        }
+        const double gnew = flag == 1 ? 0.0 : (double)gk;
         D.g[o] = gnew;
-        D.cls[o] = flag;
-        const double scale = (gk * gk + S->scale_va * D.df_va) / (D.df_va + 1.0);
-        D.vara_s[o] = d_rscinvchi2(D.df_va + 1.0, scale, R, err);
+        if (m == SODAGPU_BAYES_B) D.cls[o] = flag;
+        const T scale = (gk * gk + q.scale_va * df_va) / (df_va + (T)1.0);
+        D.vara_s[o] = (double)scinvchi2_from(df_va + (T)1.0, scale, a.gam);
         return gold - gnew;
     }
     // BayesC / Cpi / R / Rc
-    const int nm = D.nmix;
-    const int sg = D.grp[snploc] - 1;
-    double s[MAXDIST];
-    s[0] = S->log_p[sg];
-    for (int kk = 1; kk < nm; ++kk) {
-        const double logdetV = log(S->gp[kk] * zz_vare + 1.0);
-        const double uhat = rhs / (zz + S->vare_gp[kk]);
-        s[kk] = -0.5 * (logdetV - (rhs * uhat / vare)) + S->log_p[sg + kk * ng];
-    }
-    const double u = crng_unit(R);
-    double ssculm = 0.0;
-    int flag = 1;
-    for (int kk = 0; kk < nm; ++kk) {
-        const double skk = s[kk];
-        double sk = 0.0;
-        bool overflow = false;
-        for (int j = 0; j < nm; ++j) {
-            if (j == kk) continue;
-            const double clike = s[j] - skk;
-            if (clike < -700) continue;
-            if (clike > 700) { overflow = true; break; }
-            sk = sk + exp(clike);
-        }
-        const double st = overflow ? 0.0 : 1.0 / (1.0 + sk);
-        ssculm = ssculm + st;
-        if (u < ssculm) { flag = kk + 1; break; }
-    }
-    double gnew = 0.0;
-    if (flag != 1) {
-        const double v1 = zz + vare / S->gp[flag - 1];
-        gnew = d_rnorm(rhs / v1, sqrt(vare / v1), R);
-    }
-    D.cls[o] = flag;
-    D.g[o] = gnew;
-    return gold - gnew;
-}
-
-// The same draw in FP32 arithmetic, for the FP32/FP8 sweeps: GB300 executes
-// FP64 at a small fraction of its FP32 rate, and the draws of a subset sit on
-// the critical path of every subset.  State stays FP64.
-// Chain state a draw reads, loaded by the caller ahead of the draw (for up
-// to DRAW_PRE mixture classes; the state changes only between iterations):
-// the residual variance, the prior scale, the SNP's locus variance (BayesA/B)
-// and, per class k, log pi of the SNP's group, gamma_k sigma2_g and
-// sigma2_e / (gamma_k sigma2_g).
-constexpr int DRAW_PRE = 4;
-struct DrawPre {
-    float vare, scale_va, vs;
-    float logp[DRAW_PRE], gp[DRAW_PRE], vgp[DRAW_PRE];
-};
-
-__device__ __forceinline__ void draw_prefetch(const Dev &D, const ChainScal *S, int c, int snploc, int sg, DrawPre &q)
-{
-    q.vare = (float)S->vare;
-    q.scale_va = (float)S->scale_va;
-    q.vs = (D.method == SODAGPU_BAYES_A || D.method == SODAGPU_BAYES_B) ? (float)D.vara_s[(size_t)c * D.p + snploc]
-                                                                          : 0.0f;
-#pragma unroll
-    for (int k = 0; k < DRAW_PRE; ++k) {
-        const bool in = k < D.nmix;
-        q.logp[k] = in ? (float)S->log_p[sg + k * D.ngroup] : 0.0f;
-        q.gp[k] = in ? (float)S->gp[k] : 0.0f;
-        q.vgp[k] = in ? (float)S->vare_gp[k] : 0.0f;
-    }
-}
-
-// gold = g and cl = class of the SNP in this chain, sg = its group - 1, all
-// loaded by the caller ahead of the draw (they sit on its critical path);
-// pre: the prefetched chain state (used when nmix <= DRAW_PRE).
-__device__ __forceinline__ double draw_snp_f(const Dev &D, const ChainScal *S, int c, int snploc, float rhs, float zz,
-                                             float zz_vare, CRng &R, int *err, double gold, int cl, int sg,
-                                             const DrawPre &pre)
-{
-    const size_t o = (size_t)c * D.p + snploc;
-    const bool use_pre = D.nmix <= DRAW_PRE;
-    const float vare = pre.vare;
-    float gk = (float)gold;
-    const int m = D.method;
-    const float df_va = (float)D.df_va, scale_va = pre.scale_va;
-    if (m == SODAGPU_BAYES_A) {
-        rhs = rhs + zz * gk;
-        const float vs = pre.vs;
-        const float v1 = zz + vare / vs;
-        gk = d_rnorm_f(rhs / v1, sqrtf(vare / v1), R);
-        D.g[o] = (double)gk;
-        const float scale = (gk * gk + scale_va * df_va) / (df_va + 1.0f);
-        D.vara_s[o] = (double)d_rscinvchi2_f(df_va + 1.0f, scale, R, err);
-        return gold - (double)gk;
-    }
     if (cl > 1) rhs = rhs + zz * gk;
-    const int ng = D.ngroup;
-    if (m == SODAGPU_BAYES_B) {
-        const float vs = pre.vs;
-        const float s1 = pre.logp[0];
-        const float logdetV = logf(vs * zz_vare + 1.0f);
-        const float uhat = rhs / (zz + vare / vs);
-        const float s2 = -0.5f * (logdetV - (rhs * uhat / vare)) + pre.logp[1];
-        const float clike = s1 - s2;
-        float sk;
-        if (clike > 700.0f) sk = 0.0f;
-        else if (clike < -700.0f) sk = 1.0f;
-        else sk = 1.0f / (1.0f + expf(clike));
-        const float u = crng_unit_f(R);
-        const int flag = u < sk ? 2 : 1;
-        double gnew;
-        if (flag == 1) {
-            gk = d_rnorm_f(0.0f, sqrtf(vs), R);
-            gnew = 0.0;
-        } else {
-            const float v1 = zz + vare / vs;
-            gk = d_rnorm_f(rhs / v1, sqrtf(vare / v1), R);
-            gnew = (double)gk;
-        }
-        D.g[o] = gnew;
-        D.cls[o] = flag;
-        const float scale = (gk * gk + scale_va * df_va) / (df_va + 1.0f);
-        D.vara_s[o] = (double)d_rscinvchi2_f(df_va + 1.0f, scale, R, err);
-        return gold - gnew;
-    }
     const int nm = D.nmix;
     int flag = 1;
-    if (use_pre) {
-        // up to DRAW_PRE classes with every loop unrolled: the scores stay in registers
-        float sv[DRAW_PRE];
-        sv[0] = pre.logp[0];
+    T v1, sd;
+    if (nm <= DRAW_PRE) {
+        // every loop unrolled: the scores stay in registers
+        T sv[DRAW_PRE];
 #pragma unroll
-        for (int kk = 1; kk < DRAW_PRE; ++kk) {
-            sv[kk] = 0.0f;
-            if (kk < nm) {
-                const float logdetV = logf(pre.gp[kk] * zz_vare + 1.0f);
-                const float uhat = rhs / (zz + pre.vgp[kk]);
-                sv[kk] = -0.5f * (logdetV - (rhs * uhat / vare)) + pre.logp[kk];
+        for (int kk = 0; kk < DRAW_PRE; ++kk) {
+            const T lp = ng > 1 && kk < nm ? (T)S->log_p[sg + kk * ng] : q.logp[kk];
+            sv[kk] = lp;
+            if (kk > 0 && kk < nm) {
+                const T uhat = rhs / q.den[kk];
+                sv[kk] = (T)-0.5 * (q.ld[kk] - (rhs * uhat / vare)) + lp;
             }
         }
-        const float u = crng_unit_f(R);
-        float ssculm = 0.0f;
+        T ssculm = (T)0.0;
         bool done = false;
 #pragma unroll
         for (int kk = 0; kk < DRAW_PRE; ++kk) {
             if (kk < nm && !done) {
-                float sk = 0.0f;
+                T sk = (T)0.0;
                 bool overflow = false;
 #pragma unroll
                 for (int j = 0; j < DRAW_PRE; ++j) {
                     if (j < nm && j != kk && !overflow) {
-                        const float clike = sv[j] - sv[kk];
-                        if (clike > 700.0f) overflow = true;
-                        else if (clike >= -700.0f) sk = sk + expf(clike);
+                        const T clike = sv[j] - sv[kk];
+                        if (clike > (T)700.0) overflow = true;
+                        else if (clike >= (T)-700.0) sk = sk + t_exp(clike);
                     }
                 }
-                ssculm = ssculm + (overflow ? 0.0f : 1.0f / (1.0f + sk));
-                if (u < ssculm) {
+                ssculm = ssculm + (overflow ? (T)0.0 : (T)1.0 / ((T)1.0 + sk));
+                if (a.u < ssculm) {
                     flag = kk + 1;
                     done = true;
                 }
             }
         }
+        v1 = q.v1[1];
+        sd = q.sd[1];
+#pragma unroll
+        for (int k = 2; k < DRAW_PRE; ++k)
+            if (k == flag - 1) {
+                v1 = q.v1[k];
+                sd = q.sd[k];
+            }
+        if (flag == 1) v1 = (T)1.0;
     } else {
-        float sv[MAXDIST];
-        sv[0] = (float)S->log_p[sg];
+        T sv[MAXDIST];
+        sv[0] = (T)S->log_p[sg];
         for (int kk = 1; kk < nm; ++kk) {
-            const float logdetV = logf((float)S->gp[kk] * zz_vare + 1.0f);
-            const float uhat = rhs / (zz + (float)S->vare_gp[kk]);
-            sv[kk] = -0.5f * (logdetV - (rhs * uhat / vare)) + (float)S->log_p[sg + kk * ng];
+            const T logdetV = t_log((T)S->gp[kk] * q.zz_vare + (T)1.0);
+            const T uhat = rhs / (zz + (T)S->vare_gp[kk]);
+            sv[kk] = (T)-0.5 * (logdetV - (rhs * uhat / vare)) + (T)S->log_p[sg + kk * ng];
         }
-        const float u = crng_unit_f(R);
-        float ssculm = 0.0f;
+        T ssculm = (T)0.0;
         for (int kk = 0; kk < nm; ++kk) {
-            const float skk = sv[kk];
-            float sk = 0.0f;
+            const T skk = sv[kk];
+            T sk = (T)0.0;
             bool overflow = false;
             for (int j = 0; j < nm; ++j) {
                 if (j == kk) continue;
-                const float clike = sv[j] - skk;
-                if (clike < -700.0f) continue;
-                if (clike > 700.0f) { overflow = true; break; }
-                sk = sk + expf(clike);
+                const T clike = sv[j] - skk;
+                if (clike < (T)-700.0) continue;
+                if (clike > (T)700.0) { overflow = true; break; }
+                sk = sk + t_exp(clike);
             }
-            ssculm = ssculm + (overflow ? 0.0f : 1.0f / (1.0f + sk));
-            if (u < ssculm) { flag = kk + 1; break; }
+            ssculm = ssculm + (overflow ? (T)0.0 : (T)1.0 / ((T)1.0 + sk));
+            if (a.u < ssculm) { flag = kk + 1; break; }
         }
+        v1 = zz + vare / (flag == 1 ? (T)1.0 : (T)S->gp[flag - 1]);
+        sd = t_sqrt(vare / v1);
     }
     double gnew = 0.0;
     if (flag != 1) {
-        float gsel = 0.0f;
-#pragma unroll
-        for (int k = 0; k < DRAW_PRE; ++k)
-            if (k == flag - 1) gsel = pre.gp[k];
-        const float v1 = zz + vare / (use_pre ? gsel : (float)S->gp[flag - 1]);
-        gnew = (double)d_rnorm_f(rhs / v1, sqrtf(vare / v1), R);
+        const T mean = rhs / v1;
+        gnew = (double)(sd <= (T)0.0 ? mean : normal_from(mean, sd, a.z));
     }
     D.cls[o] = flag;
     D.g[o] = gnew;
@@ -1221,7 +1171,8 @@ static cudaError_t launch_block(const Dev &D, int b, int nblk_snps, int sm_count
     if (e != cudaSuccess) return e;
     {
         ProfScope ps(prof, st, PROF_DRAW);
-        e = launch_pdl(k_draw<MODE, CT, false>, dim3((nblk_snps * CT + 255) / 256), dim3(256), 0, st, D, b, ks,
+        constexpr int NT = DrawThreads<CT, false>::v;
+        e = launch_pdl(k_draw<MODE, CT, false>, dim3((nblk_snps * CT + NT - 1) / NT), dim3(NT), 0, st, D, b, ks,
                        nblk_snps);
     }
     if (e != cudaSuccess || rhs_only) return e != cudaSuccess ? e : cudaGetLastError();
@@ -1765,7 +1716,7 @@ __global__ void __launch_bounds__(256, 1) k_rhs_m(const __grid_constant__ JobGri
 }
 
 template <int MODE, int CT>
-__global__ void __launch_bounds__(256, 1) k_draw_m(const __grid_constant__ JobGrid G)
+__global__ void __launch_bounds__(DrawThreads<CT, false>::v, 1) k_draw_m(const __grid_constant__ JobGrid G)
 {
     VB vb;
     const int j = jg_locate(G, vb);
@@ -1809,7 +1760,7 @@ template <int MODE, int CT>
 static cudaError_t multi_step(const BatchPlan &P, int t, cudaStream_t st)
 {
     const int nj = P.njobs;
-    constexpr int MTS = 8 * SptOf<CT>::v;
+    constexpr int MTS = 8 * SptOf<CT>::v, NT = DrawThreads<CT, false>::v;
     GridBuilder rhs(P.ddev, nj), draw(P.ddev, nj), upd(P.ddev, nj);
     size_t usmem = 0;
     for (int j = 0; j < nj; ++j) {
@@ -1824,13 +1775,13 @@ static cudaError_t multi_step(const BatchPlan &P, int t, cudaStream_t st)
         const int mtiles = (N + MTS - 1) / MTS;
         const int ks = P.ksplit[j];
         rhs.set(j, mtiles * ks, 1, 1, t, ks);
-        draw.set(j, (N * CT + 255) / 256, 1, 1, t, ks, N);
+        draw.set(j, (N * CT + NT - 1) / NT, 1, 1, t, ks, N);
         upd.set(j, D.nr_ctas + (D.bs + UT - 1) / UT, 1, 1, t);
         usmem = std::max(usmem, update_smem_bytes_ct<MODE, CT>(D.bs));
     }
     if (rhs.total() == 0) return cudaSuccess;
     cudaError_t e = launch_pdl(k_rhs_m<MODE, CT>, dim3(rhs.total()), dim3(256), rhs_smem_bytes<MODE, CT>(), st, rhs.g);
-    if (e == cudaSuccess) e = launch_pdl(k_draw_m<MODE, CT>, dim3(draw.total()), dim3(256), 0, st, draw.g);
+    if (e == cudaSuccess) e = launch_pdl(k_draw_m<MODE, CT>, dim3(draw.total()), dim3(NT), 0, st, draw.g);
     if (e == cudaSuccess)
         e = launch_pdl(k_update_m<MODE, CT>, dim3(upd.total()), dim3(32 * UpdWarps<MODE, CT>::v), usmem, st, upd.g);
     return e;

@@ -538,6 +538,12 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     TRY(c->alloc(&W, (size_t)wtot, false));
     TRY(c->alloc(&d_wofs, nb, false));
     CUDA_TRY(cudaMemcpyAsync(d_wofs, wofs.data(), sizeof(int64_t) * nb, cudaMemcpyHostToDevice, c->st));
+    CUtensorMap tm_g;
+    if (make_tmap_2d(&tm_g, CU_TENSOR_MAP_DATA_TYPE_UINT8, c->G, c->ldx, p, c->ldx, 128, 128,
+                     CU_TENSOR_MAP_SWIZZLE_128B) != CUDA_SUCCESS)
+        return fail(SODAGPU_E_CUDA, "cuTensorMapEncodeTiled failed for the genotypes");
+    int *d_err = nullptr, h_err = 0;
+    TRY(c->alloc(&d_err, 1));
     const int BATCH = std::min(nb, 64);
     const int mmax = std::min(maxN, 400);
     CUDA_TRY(zb_lz_prepare(maxN, mmax));
@@ -569,7 +575,8 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
             bmax = std::max(bmax, c->blk_sizes[b0 + i]);
         }
         CUDA_TRY(cudaMemcpyAsync(d_batch, batch_ids.data(), sizeof(int32_t) * nbat, cudaMemcpyHostToDevice, c->st));
-        CUDA_TRY(zb_gram(c->G, c->ldx, c->blk_ls, d_batch, nbat, bmax, d_wofs, c->freq, c->perm, n, W, c->st));
+        CUDA_TRY(zb_gram(&tm_g, c->G, c->ldx, c->blk_ls, d_batch, nbat, bmax, d_wofs, c->freq, c->perm, n, W, nullptr, 0,
+                         d_err, c->st));
         // Lanczos for lambda_max of each subset
         CUDA_TRY(cudaMemsetAsync(d_done, 0, BATCH, c->st));
         CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(double) * BATCH * mmax, c->st));
@@ -618,7 +625,9 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
         CUDA_TRY(cudaStreamSynchronize(c->st));
     }
     CUDA_TRY(cudaMemcpyAsync(h_status.data(), d_status, sizeof(int32_t) * nb, cudaMemcpyDeviceToHost, c->st));
+    CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CUDA_TRY(cudaStreamSynchronize(c->st));
+    if (h_err) return fail(SODAGPU_E_TIMEOUT, "a bounded device wait of the Z build gave up");
     // pivoted fallback for the subsets whose factorisation failed (soda.f90:492-510)
     std::vector<int32_t> h_iskipped;
     int naless = p;
@@ -641,7 +650,8 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
             if (h_status[b] != 0) {
                 int32_t one = b;
                 CUDA_TRY(cudaMemcpyAsync(d_batch, &one, sizeof(int32_t), cudaMemcpyHostToDevice, c->st));
-                CUDA_TRY(zb_gram(c->G, c->ldx, c->blk_ls, d_batch, 1, N, d_wofs, c->freq, c->perm, n, W, c->st));
+                CUDA_TRY(zb_gram(&tm_g, c->G, c->ldx, c->blk_ls, d_batch, 1, N, d_wofs, c->freq, c->perm, n, W, nullptr, 0,
+                                 d_err, c->st));
                 CUDA_TRY(zb_form_m(W, d_wofs, c->blk_ls, d_batch, 1, c->xxd, c->st));
                 CUDA_TRY(cudaMemcpyAsync(M, W + wofs[b], sizeof(double) * N * N, cudaMemcpyDeviceToDevice, c->st));
                 CUDA_TRY(zb_psd_block(W + wofs[b], M, N, c->h_blk_ls[b], c->ulen, c->skip, piv, rank, pst, work, c->st));
@@ -707,6 +717,7 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     c->release(d_status);
     c->release(d_done);
     c->release(d_wofs);
+    c->release(d_err);
     TRY(c->alloc(&c->iskipped, std::max(1, c->nskipped), false));
     TRY(c->alloc(&c->xpx, p));
     if (c->nskipped)

@@ -2,7 +2,7 @@
 //
 // Per subset b of N SNPs (get_aug_matrix, soda.f90:445-518):
 //   A   = X_b'X_b from the exact integer Gram of the 0/1/2 codes, centred and
-//         scaled like xxproduct (soda.f90:520-556)              k_gram
+//         scaled like xxproduct (soda.f90:520-556)              k_gram_tc
 //   d   = lambda_max(A) + 0.001 (soda.f90:484-486); lambda_max from a
 //         fully reorthogonalised Lanczos run (k_lz_*) instead of the
 //         reference's power iteration (soda.f90:378-401): both converge to
@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "dgv.cuh"
+#include "gram_tc.cuh"
 #include "rng.cuh"
 #include "state.cuh"
 #include "zbuild.cuh"
@@ -120,7 +121,9 @@ __global__ void k_x32(const int8_t *G, const double *xv, float *X32, int n, int 
 }
 
 // ---------------------------------------------------------------------------
-// Gram: S = G_b'G_b with dp4a on 64x64 tiles, then the xxproduct scaling
+// Gram: S = G_b'G_b and the xxproduct scaling, on the tensor cores (gram_tc.cuh);
+// with dp4a on 64x64 tiles for more than GR_NMAX individuals, whose counts
+// FP32 sums do not hold
 // ---------------------------------------------------------------------------
 constexpr int GT = 64;   // output tile
 constexpr int GK = 64;   // bytes of K per stage
@@ -128,7 +131,7 @@ constexpr int GK = 64;   // bytes of K per stage
 __global__ void __launch_bounds__(256) k_gram(const int8_t *G, int ldx, const int32_t *blk_ls,
                                               const int32_t *batch_blocks, const int64_t *wofs,
                                               const double *freq, const int32_t *perm, int n,
-                                              double *W)
+                                              double *W, float *W32, int ld32, size_t stride32)
 {
     __shared__ int sA[GT][GK / 4 + 1];
     __shared__ int sB[GT][GK / 4 + 1];
@@ -166,6 +169,7 @@ __global__ void __launch_bounds__(256) k_gram(const int8_t *G, int ldx, const in
     }
     const double ep = 2.220446049250313e-16;
     double *Wb = W + wofs[b];
+    float *Fb = W32 ? W32 + blockIdx.y * stride32 : nullptr;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int j = ti * GT + ty * 4 + q;
@@ -193,6 +197,10 @@ __global__ void __launch_bounds__(256) k_gram(const int8_t *G, int ldx, const in
             }
             Wb[(size_t)j + (size_t)k * N] = res;
             Wb[(size_t)k + (size_t)j * N] = res;
+            if (Fb) {
+                Fb[(size_t)j + (size_t)k * ld32] = (float)res;
+                Fb[(size_t)k + (size_t)j * ld32] = (float)res;
+            }
         }
     }
 }
@@ -708,12 +716,22 @@ cudaError_t zb_x32(const int8_t *G, const double *xv, float *X32, int n, int p, 
     return cudaGetLastError();
 }
 
-cudaError_t zb_gram(const int8_t *G, int ldx, const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch,
-                    int maxN, const int64_t *wofs, const double *freq, const int32_t *perm, int n, double *W,
-                    cudaStream_t st)
+cudaError_t zb_gram(const CUtensorMap *tm_g, const int8_t *G, int ldx, const int32_t *blk_ls,
+                    const int32_t *batch_blocks, int nbatch, int maxN, const int64_t *wofs, const double *freq,
+                    const int32_t *perm, int n, double *W, float *W32, int ld32, int *err, cudaStream_t st)
 {
+    const size_t stride32 = (size_t)ld32 * maxN;
+    if (n <= GR_NMAX) {
+        cudaError_t e = cudaFuncSetAttribute(k_gram_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GR_SMEM);
+        if (e != cudaSuccess) return e;
+        const int nt = (maxN + GR_T - 1) / GR_T;
+        k_gram_tc<<<dim3(nt * (nt + 1) / 2, nbatch), GR_THREADS, GR_SMEM, st>>>(
+            *tm_g, ldx, blk_ls, batch_blocks, wofs, freq, perm, n, W, W32, ld32, stride32, err);
+        return cudaGetLastError();
+    }
     const int nt = (maxN + GT - 1) / GT;
-    k_gram<<<dim3(nt * (nt + 1) / 2, nbatch), 256, 0, st>>>(G, ldx, blk_ls, batch_blocks, wofs, freq, perm, n, W);
+    k_gram<<<dim3(nt * (nt + 1) / 2, nbatch), 256, 0, st>>>(G, ldx, blk_ls, batch_blocks, wofs, freq, perm, n, W, W32,
+                                                            ld32, stride32);
     return cudaGetLastError();
 }
 

@@ -544,25 +544,28 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
         return fail(SODAGPU_E_CUDA, "cuTensorMapEncodeTiled failed for the genotypes");
     int *d_err = nullptr, h_err = 0;
     TRY(c->alloc(&d_err, 1));
-    const int BATCH = std::min(nb, 64);
+    // subsets at a time: at most 64, and at most 4 GB of the FP32 copies that start the Lanczos runs
+    const size_t w32 = round_up((size_t)maxN, 32) * maxN * sizeof(float);
+    const int BATCH = (int)std::min<size_t>({(size_t)nb, (size_t)64, std::max<size_t>(1, ((size_t)4 << 30) / w32)});
     const int mmax = std::min(maxN, 400);
     CUDA_TRY(zb_lz_prepare(maxN, mmax));
-    double *V = nullptr, *wvec = nullptr, *alpha = nullptr, *beta = nullptr;
-    int64_t *d_vofs = nullptr;
+    double *V = nullptr, *wpart = nullptr, *alpha = nullptr, *beta = nullptr;
+    float *W32 = nullptr, *V32 = nullptr, *ab32 = nullptr;   // the Lanczos start's
+    const int ld32 = (int)round_up((size_t)maxN, 32);
+    const size_t vstride = (size_t)mmax * maxN;
     int32_t *d_batch = nullptr, *d_status = nullptr;
     uint8_t *d_done = nullptr;
-    TRY(c->alloc(&V, (size_t)BATCH * mmax * maxN));
-    TRY(c->alloc(&wvec, (size_t)BATCH * maxN));
-    TRY(c->alloc(&alpha, (size_t)BATCH * mmax));
-    TRY(c->alloc(&beta, (size_t)BATCH * mmax));
-    TRY(c->alloc(&d_vofs, BATCH, false));
+    TRY(c->alloc(&V, BATCH * vstride, false));
+    TRY(c->alloc(&wpart, zb_lz_wpart(maxN, BATCH), false));
+    TRY(c->alloc(&W32, (size_t)BATCH * ld32 * maxN, false));
+    TRY(c->alloc(&V32, (size_t)BATCH * zb_lz_pre() * maxN, false));
+    TRY(c->alloc(&ab32, (size_t)2 * BATCH * zb_lz_pre(), false));
+    TRY(c->alloc(&alpha, (size_t)2 * BATCH * mmax));
+    beta = alpha + (size_t)BATCH * mmax;
     TRY(c->alloc(&d_batch, BATCH, false));
     TRY(c->alloc(&d_status, nb));
     TRY(c->alloc(&d_done, BATCH));
-    std::vector<int64_t> vofs(BATCH);
-    for (int i = 0; i < BATCH; ++i) vofs[i] = (int64_t)i * mmax * maxN;
-    CUDA_TRY(cudaMemcpyAsync(d_vofs, vofs.data(), sizeof(int64_t) * BATCH, cudaMemcpyHostToDevice, c->st));
-    std::vector<double> h_xxd(nb), ha((size_t)BATCH * mmax), hb((size_t)BATCH * mmax);
+    std::vector<double> h_xxd(nb), hab((size_t)2 * BATCH * mmax);
     std::vector<int32_t> h_status(nb, 0);
     std::vector<int32_t> batch_ids;
     const float shift_f = 0.001f;   // soda.f90:485 adds a REAL literal
@@ -575,32 +578,32 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
             bmax = std::max(bmax, c->blk_sizes[b0 + i]);
         }
         CUDA_TRY(cudaMemcpyAsync(d_batch, batch_ids.data(), sizeof(int32_t) * nbat, cudaMemcpyHostToDevice, c->st));
-        CUDA_TRY(zb_gram(&tm_g, c->G, c->ldx, c->blk_ls, d_batch, nbat, bmax, d_wofs, c->freq, c->perm, n, W, nullptr, 0,
-                         d_err, c->st));
+        CUDA_TRY(zb_gram(&tm_g, c->G, c->ldx, c->blk_ls, d_batch, nbat, maxN, d_wofs, c->freq, c->perm, n, W, W32,
+                         ld32, d_err, c->st));
         // Lanczos for lambda_max of each subset
         CUDA_TRY(cudaMemsetAsync(d_done, 0, BATCH, c->st));
-        CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(double) * BATCH * mmax, c->st));
-        CUDA_TRY(cudaMemsetAsync(beta, 0, sizeof(double) * BATCH * mmax, c->st));
-        CUDA_TRY(zb_lz_init(c->blk_ls, d_batch, nbat, d_vofs, V, (uint64_t)llabs(c->cfg.seed), c->st));
+        CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(double) * 2 * BATCH * mmax, c->st));
+        CUDA_TRY(zb_lz_start(W32, ld32, c->blk_ls, d_batch, nbat, maxN, vstride, V, V32,
+                             reinterpret_cast<float *>(wpart), ab32, (uint64_t)llabs(c->cfg.seed), c->st));
         std::vector<uint8_t> done(nbat, 0);
-        std::vector<double> theta(nbat, 0.0), theta_prev(nbat, -1.0);
+        // converged: theta has not moved over eight steps, looked at every four
+        std::vector<double> theta(nbat, 0.0), theta4(nbat, -1.0), theta8(nbat, -1.0);
         std::vector<int> steps(nbat, 0);
         const int bmm = std::min(bmax, mmax);
         for (int j = 0; j < bmm; ++j) {
-            CUDA_TRY(zb_lz_step(W, d_wofs, c->blk_ls, d_batch, nbat, bmax, d_vofs, V, wvec, maxN, alpha, beta, mmax,
-                                j, d_done, c->st));
-            const bool check = ((j + 1) % 8 == 0) || j + 1 == bmm;
+            CUDA_TRY(zb_lz_step(W, d_wofs, c->blk_ls, d_batch, nbat, maxN, vstride, V, wpart, alpha, beta, mmax, j,
+                                d_done, c->st));
+            const bool check = ((j + 1) % 4 == 0) || j + 1 == bmm;
             if (!check) continue;
-            CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha, sizeof(double) * nbat * mmax, cudaMemcpyDeviceToHost, c->st));
-            CUDA_TRY(cudaMemcpyAsync(hb.data(), beta, sizeof(double) * nbat * mmax, cudaMemcpyDeviceToHost, c->st));
+            CUDA_TRY(cudaMemcpyAsync(hab.data(), alpha, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->st));
             CUDA_TRY(cudaStreamSynchronize(c->st));
             bool all = true;
             for (int i = 0; i < nbat; ++i) {
                 if (done[i]) continue;
                 const int Nb = c->blk_sizes[b0 + i];
                 const int m = std::min(j + 1, Nb);
-                const double *a = &ha[(size_t)i * mmax];
-                const double *bb = &hb[(size_t)i * mmax];
+                const double *a = &hab[(size_t)i * mmax];
+                const double *bb = &hab[(size_t)(BATCH + i) * mmax];
                 theta[i] = tridiag_max_eig(a, bb, m);
                 steps[i] = m;
                 const double scale = std::max(fabs(theta[i]), 1e-300);
@@ -608,13 +611,14 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
                 if (m >= Nb) conv = true;   // full Krylov space: exact
                 for (int t = 0; t < m && !conv; ++t)
                     if (bb[t] <= 1e-13 * scale) conv = true;   // invariant subspace
-                if (!conv && theta_prev[i] >= 0.0 && fabs(theta[i] - theta_prev[i]) <= 1e-15 * scale) conv = true;
-                theta_prev[i] = theta[i];
+                if (!conv && theta8[i] >= 0.0 && fabs(theta[i] - theta8[i]) <= 1e-15 * scale) conv = true;
+                theta8[i] = theta4[i];
+                theta4[i] = theta[i];
                 if (conv) done[i] = 1;
                 else all = false;
             }
-            CUDA_TRY(cudaMemcpyAsync(d_done, done.data(), nbat, cudaMemcpyHostToDevice, c->st));
             if (all) break;
+            CUDA_TRY(cudaMemcpyAsync(d_done, done.data(), nbat, cudaMemcpyHostToDevice, c->st));
         }
         for (int i = 0; i < nbat; ++i)
             h_xxd[b0 + i] = fabs(theta[i]) + (double)shift_f + c->d_offset;
@@ -709,10 +713,11 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     }
     c->release(W);
     c->release(V);
-    c->release(wvec);
+    c->release(wpart);
+    c->release(W32);
+    c->release(V32);
+    c->release(ab32);
     c->release(alpha);
-    c->release(beta);
-    c->release(d_vofs);
     c->release(d_batch);
     c->release(d_status);
     c->release(d_done);

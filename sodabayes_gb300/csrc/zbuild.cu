@@ -4,7 +4,7 @@
 //   A   = X_b'X_b from the exact integer Gram of the 0/1/2 codes, centred and
 //         scaled like xxproduct (soda.f90:520-556)              k_gram_tc
 //   d   = lambda_max(A) + 0.001 (soda.f90:484-486); lambda_max from a
-//         fully reorthogonalised Lanczos run (k_lz_*) instead of the
+//         fully reorthogonalised Lanczos run (lanczos.cuh) instead of the
 //         reference's power iteration (soda.f90:378-401): both converge to
 //         the same eigenvalue, Lanczos in far fewer products with A.
 //   U   = chol(d I - A), upper (choleskyPD, soda.f90:8-47)     k_chol_*
@@ -15,8 +15,10 @@
 // matrix W_b (N x N, column-major, ld N) lives at wofs[b].
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <algorithm>
 #include "dgv.cuh"
 #include "gram_tc.cuh"
+#include "lanczos.cuh"
 #include "rng.cuh"
 #include "state.cuh"
 #include "zbuild.cuh"
@@ -205,10 +207,6 @@ __global__ void __launch_bounds__(256) k_gram(const int8_t *G, int ldx, const in
     }
 }
 
-// ---------------------------------------------------------------------------
-// Lanczos with full reorthogonalisation (two classical Gram-Schmidt passes)
-// V_b: [mmax][N] at vofs[b]; alpha/beta: [batch][mmax]
-// ---------------------------------------------------------------------------
 __device__ double blk_sum(double v, double *sh)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -225,114 +223,6 @@ __device__ double blk_sum(double v, double *sh)
     }
     __syncthreads();
     return sh[32];
-}
-
-__global__ void __launch_bounds__(1024) k_lz_init(const int32_t *blk_ls, const int32_t *batch_blocks,
-                                                  const int64_t *vofs, double *V, uint64_t seed)
-{
-    __shared__ double sh[33];
-    const int b = batch_blocks[blockIdx.x];
-    const int N = blk_ls[b + 1] - blk_ls[b];
-    double *v = V + vofs[blockIdx.x];
-    double ss = 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        // the i-th uniform of the (seed, subset, P_POWER) stream, like the
-        // reference's random start vector (soda.f90:390)
-        CRng R;
-        crng_init(R, seed, 0, 0, b, P_POWER);
-        R.c3 += (uint32_t)(i >> 1);
-        double x = crng_unit(R);
-        if (i & 1) x = crng_unit(R);
-        v[i] = x;
-        ss += x * x;
-    }
-    ss = blk_sum(ss, sh);
-    const double inv = 1.0 / sqrt(ss);
-    for (int i = threadIdx.x; i < N; i += blockDim.x) v[i] *= inv;
-}
-
-// w = A v_j ; one thread per row, v_j staged in shared memory
-__global__ void __launch_bounds__(128) k_lz_matvec(const double *W, const int64_t *wofs,
-                                                   const int32_t *blk_ls, const int32_t *batch_blocks,
-                                                   const int64_t *vofs, const double *V, double *Wvec,
-                                                   int ldw, int j)
-{
-    extern __shared__ double sv[];
-    const int b = batch_blocks[blockIdx.y];
-    const int N = blk_ls[b + 1] - blk_ls[b];
-    const double *v = V + vofs[blockIdx.y] + (size_t)j * N;
-    for (int k = threadIdx.x; k < N; k += blockDim.x) sv[k] = v[k];
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const double *A = W + wofs[b];
-    double acc0 = 0.0, acc1 = 0.0;
-    int k = 0;
-    for (; k + 1 < N; k += 2) {
-        acc0 += A[(size_t)i + (size_t)k * N] * sv[k];
-        acc1 += A[(size_t)i + (size_t)(k + 1) * N] * sv[k + 1];
-    }
-    if (k < N) acc0 += A[(size_t)i + (size_t)k * N] * sv[k];
-    Wvec[(size_t)blockIdx.y * ldw + i] = acc0 + acc1;
-}
-
-// alpha, three-term recurrence, two CGS passes, beta, v_{j+1}
-__global__ void __launch_bounds__(1024) k_lz_orth(const int32_t *blk_ls, const int32_t *batch_blocks,
-                                                  const int64_t *vofs, double *V, double *Wvec, int ldw,
-                                                  double *alpha, double *beta, int mmax, int j,
-                                                  const uint8_t *done)
-{
-    __shared__ double sh[33];
-    extern __shared__ double sw[];   // [N] w, then [mmax] h
-    const int bi = blockIdx.x;
-    if (done[bi]) return;
-    const int b = batch_blocks[bi];
-    const int N = blk_ls[b + 1] - blk_ls[b];
-    double *Vb = V + vofs[bi];
-    double *h = sw + N;
-    const double *vj = Vb + (size_t)j * N;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) sw[i] = Wvec[(size_t)bi * ldw + i];
-    __syncthreads();
-    double part = 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) part += sw[i] * vj[i];
-    const double a = blk_sum(part, sh);
-    const double bprev = j > 0 ? beta[(size_t)bi * mmax + j - 1] : 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        double x = sw[i] - a * vj[i];
-        if (j > 0) x -= bprev * Vb[(size_t)(j - 1) * N + i];
-        sw[i] = x;
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int t = warp; t <= j; t += nw) {
-            const double *vt = Vb + (size_t)t * N;
-            double s = 0.0;
-            for (int i = lane; i < N; i += 32) s += vt[i] * sw[i];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) h[t] = s;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < N; i += blockDim.x) {
-            double x = sw[i];
-            for (int t = 0; t <= j; ++t) x -= h[t] * Vb[(size_t)t * N + i];
-            sw[i] = x;
-        }
-        __syncthreads();
-    }
-    double ss = 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) ss += sw[i] * sw[i];
-    const double bt = sqrt(blk_sum(ss, sh));
-    if (threadIdx.x == 0) {
-        alpha[(size_t)bi * mmax + j] = a;
-        beta[(size_t)bi * mmax + j] = bt;
-    }
-    if (j + 1 < mmax && j + 1 < N) {
-        double *vn = Vb + (size_t)(j + 1) * N;
-        const double inv = bt > 0.0 ? 1.0 / bt : 0.0;
-        for (int i = threadIdx.x; i < N; i += blockDim.x) vn[i] = sw[i] * inv;
-    }
 }
 
 // M = d I - A in place (soda.f90:487-490)
@@ -735,31 +625,96 @@ cudaError_t zb_gram(const CUtensorMap *tm_g, const int8_t *G, int ldx, const int
     return cudaGetLastError();
 }
 
-cudaError_t zb_lz_init(const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch, const int64_t *vofs,
-                       double *V, uint64_t seed, cudaStream_t st)
+// Launch with programmatic stream serialization (the kernels wait for the one before them by themselves).
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_after(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                Args... args)
 {
-    k_lz_init<<<nbatch, 1024, 0, st>>>(blk_ls, batch_blocks, vofs, V, seed);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <typename T>
+static size_t lz_smem(int maxN, int mmax)
+{
+    return sizeof(T) * (size_t)(3 * mmax + (maxN + LZ_CTAS - 1) / LZ_CTAS);
+}
+
+int zb_lz_pre() { return LZ_PRE; }
+
+// Column splits of a product: about four CTAs an SM (152 of them), at most LZ_VCOLS columns each.
+template <typename T>
+static int lz_splits(int maxN, int nbatch)
+{
+    const int tiles = (maxN + LzTile<T>::v - 1) / LzTile<T>::v * nbatch;
+    return std::max((maxN + LZ_VCOLS - 1) / LZ_VCOLS, std::min(LZ_SPLITS, (608 + tiles - 1) / tiles));
+}
+
+size_t zb_lz_wpart(int maxN, int nbatch)
+{
+    return (size_t)nbatch * std::max(LZ_SPLITS, (maxN + LZ_VCOLS - 1) / LZ_VCOLS) * maxN;
+}
+
+template <typename T>
+static cudaError_t lz_step(const T *A, const int64_t *aofs, size_t astride, int ld, const int32_t *blk_ls,
+                           const int32_t *batch_blocks, int nbatch, int maxN, size_t vstride, T *V, T *wpart, T *alpha,
+                           T *beta, int mmax, int j, const uint8_t *done, cudaStream_t st)
+{
+    const int nsp = lz_splits<T>(maxN, nbatch);
+    cudaError_t e = launch_after(k_lz_matvec<T>, dim3((maxN + LzTile<T>::v - 1) / LzTile<T>::v, nsp, nbatch),
+                                 dim3(LZ_THREADS), 0, st, A, aofs, astride, ld, blk_ls, batch_blocks, vstride,
+                                 (const T *)V, wpart, maxN, j, done);
+    if (e == cudaSuccess)
+        e = launch_after(k_lz_orth<T>, dim3(LZ_CTAS * nbatch), dim3(LZ_THREADS), lz_smem<T>(maxN, mmax), st, blk_ls,
+                         batch_blocks, vstride, V, (const T *)wpart, nsp, maxN, alpha, beta, mmax, j, done);
+    return e;
+}
+
+cudaError_t zb_lz_start(const float *W32, int ld32, const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch,
+                        int maxN, size_t vstride, double *V, float *V32, float *wpart32, float *ab32, uint64_t seed,
+                        cudaStream_t st)
+{
+    const size_t vstride32 = (size_t)LZ_PRE * maxN;
+    float *alpha = ab32, *beta = ab32 + (size_t)nbatch * LZ_PRE;
+    // FP32 steps: about as many as take the vector to FP32's 1e-6 (40 at N = 300, over a hundred at N = 2000); too few
+    // cost FP64 steps, three times as long
+    const int steps = std::min(std::min(LZ_PRE, maxN), 16 + maxN / 12);
+    cudaError_t e = cudaMemsetAsync(ab32, 0, sizeof(float) * 2 * nbatch * LZ_PRE, st);
+    if (e != cudaSuccess) return e;
+    k_lz_init<float><<<nbatch, 1024, 0, st>>>(blk_ls, batch_blocks, vstride32, V32, seed);
+    e = cudaGetLastError();
+    for (int j = 0; j < steps && e == cudaSuccess; ++j)
+        e = lz_step<float>(W32, nullptr, (size_t)ld32 * maxN, ld32, blk_ls, batch_blocks, nbatch, maxN, vstride32, V32,
+                           wpart32, alpha, beta, LZ_PRE, j, nullptr, st);
+    if (e != cudaSuccess) return e;
+    k_lz_ritz<<<nbatch, 1024, 0, st>>>(blk_ls, batch_blocks, vstride32, V32, alpha, beta, steps, vstride, V);
     return cudaGetLastError();
 }
 
 cudaError_t zb_lz_step(const double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks,
-                       int nbatch, int maxN, const int64_t *vofs, double *V, double *wvec, int ldw, double *alpha,
-                       double *beta, int mmax, int j, const uint8_t *done, cudaStream_t st)
+                       int nbatch, int maxN, size_t vstride, double *V, double *wpart, double *alpha, double *beta,
+                       int mmax, int j, const uint8_t *done, cudaStream_t st)
 {
-    k_lz_matvec<<<dim3((maxN + 127) / 128, nbatch), 128, sizeof(double) * maxN, st>>>(W, wofs, blk_ls, batch_blocks,
-                                                                                      vofs, V, wvec, ldw, j);
-    k_lz_orth<<<nbatch, 1024, sizeof(double) * (maxN + mmax), st>>>(blk_ls, batch_blocks, vofs, V, wvec, ldw, alpha,
-                                                                    beta, mmax, j, done);
-    return cudaGetLastError();
+    return lz_step<double>(W, wofs, 0, 0, blk_ls, batch_blocks, nbatch, maxN, vstride, V, wpart, alpha, beta, mmax, j,
+                           done, st);
 }
 
 cudaError_t zb_lz_prepare(int maxN, int mmax)
 {
-    cudaError_t e = cudaFuncSetAttribute(k_lz_matvec, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(double) * maxN));
+    cudaError_t e = cudaFuncSetAttribute(k_lz_orth<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)lz_smem<double>(maxN, mmax));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_lz_orth, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(double) * (maxN + mmax)));
+        e = cudaFuncSetAttribute(k_lz_orth<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)lz_smem<float>(maxN, LZ_PRE));
     return e;
 }
 

@@ -18,12 +18,18 @@ cudaError_t zb_x32(const int8_t *G, const double *xv, float *X32, int n, int p, 
 cudaError_t zb_gram(const CUtensorMap *tm_g, const int8_t *G, int ldx, const int32_t *blk_ls,
                     const int32_t *batch_blocks, int nbatch, int maxN, const int64_t *wofs, const double *freq,
                     const int32_t *perm, int n, double *W, float *W32, int ld32, int *err, cudaStream_t st);
+// Lanczos runs of a batch of subsets (lanczos.cuh).  V: [batch][mmax][N], subsets vstride apart; wpart:
+// zb_lz_wpart() elements.  zb_lz_start fills v_0 from an FP32 run on W32 (V32: batch * zb_lz_pre() * maxN, ab32:
+// 2 * batch * zb_lz_pre()); zb_lz_step is step j of the FP64 run.
+int zb_lz_pre();
+size_t zb_lz_wpart(int maxN, int nbatch);
 cudaError_t zb_lz_prepare(int maxN, int mmax);
-cudaError_t zb_lz_init(const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch, const int64_t *vofs,
-                       double *V, uint64_t seed, cudaStream_t st);
+cudaError_t zb_lz_start(const float *W32, int ld32, const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch,
+                        int maxN, size_t vstride, double *V, float *V32, float *wpart32, float *ab32, uint64_t seed,
+                        cudaStream_t st);
 cudaError_t zb_lz_step(const double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks,
-                       int nbatch, int maxN, const int64_t *vofs, double *V, double *wvec, int ldw, double *alpha,
-                       double *beta, int mmax, int j, const uint8_t *done, cudaStream_t st);
+                       int nbatch, int maxN, size_t vstride, double *V, double *wpart, double *alpha, double *beta,
+                       int mmax, int j, const uint8_t *done, cudaStream_t st);
 cudaError_t zb_form_m(double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch,
                       const double *xxd, cudaStream_t st);
 cudaError_t zb_cholesky(double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks,

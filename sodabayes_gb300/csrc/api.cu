@@ -544,9 +544,24 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
         return fail(SODAGPU_E_CUDA, "cuTensorMapEncodeTiled failed for the genotypes");
     int *d_err = nullptr, h_err = 0;
     TRY(c->alloc(&d_err, 1));
-    // subsets at a time: at most 64, and at most 4 GB of the FP32 copies that start the Lanczos runs
-    const size_t w32 = round_up((size_t)maxN, 32) * maxN * sizeof(float);
-    const int BATCH = (int)std::min<size_t>({(size_t)nb, (size_t)64, std::max<size_t>(1, ((size_t)4 << 30) / w32)});
+    // subsets at a time: at most 64, and at most 4 GB of the factorisation's digits (the FP32 copies that start the
+    // Lanczos runs are a third of that)
+    const size_t digits = zb_chol_digits(maxN);
+    const int BATCH =
+        (int)std::min<size_t>({(size_t)nb, (size_t)64, std::max<size_t>(1, ((size_t)4 << 30) / (digits * 2))});
+    uint16_t *dig = nullptr;
+    double *cwork = nullptr;
+    TRY(c->alloc(&dig, BATCH * digits, false));
+    TRY(c->alloc(&cwork, zb_chol_work(maxN, BATCH), false));
+    CUtensorMap tm_da, tm_db;
+    {
+        const uint64_t cols = zb_chol_ldt(maxN), rows = BATCH * digits / cols;
+        if (make_tmap_2d(&tm_da, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, dig, cols, rows, cols * 2, 32, 128,
+                         CU_TENSOR_MAP_SWIZZLE_64B) != CUDA_SUCCESS ||
+            make_tmap_2d(&tm_db, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, dig, cols, rows, cols * 2, 32, 64,
+                         CU_TENSOR_MAP_SWIZZLE_64B) != CUDA_SUCCESS)
+            return fail(SODAGPU_E_CUDA, "cuTensorMapEncodeTiled failed for the factorisation's digits");
+    }
     const int mmax = std::min(maxN, 400);
     CUDA_TRY(zb_lz_prepare(maxN, mmax));
     double *V = nullptr, *wpart = nullptr, *alpha = nullptr, *beta = nullptr;
@@ -623,8 +638,8 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
         for (int i = 0; i < nbat; ++i)
             h_xxd[b0 + i] = fabs(theta[i]) + (double)shift_f + c->d_offset;
         CUDA_TRY(cudaMemcpyAsync(c->xxd + b0, &h_xxd[b0], sizeof(double) * nbat, cudaMemcpyHostToDevice, c->st));
-        CUDA_TRY(zb_form_m(W, d_wofs, c->blk_ls, d_batch, nbat, c->xxd, c->st));
-        CUDA_TRY(zb_cholesky(W, d_wofs, c->blk_ls, d_batch, nbat, bmax, d_status, c->st));
+        CUDA_TRY(zb_cholesky(&tm_da, &tm_db, W, d_wofs, c->blk_ls, d_batch, nbat, maxN, c->xxd, d_status, dig, cwork,
+                             d_err, c->st));
         CUDA_TRY(zb_pd_lengths(c->blk_ls, d_batch, nbat, d_status, c->ulen, c->skip, c->st));
         CUDA_TRY(cudaStreamSynchronize(c->st));
     }
@@ -723,6 +738,8 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     c->release(d_done);
     c->release(d_wofs);
     c->release(d_err);
+    c->release(dig);
+    c->release(cwork);
     TRY(c->alloc(&c->iskipped, std::max(1, c->nskipped), false));
     TRY(c->alloc(&c->xpx, p));
     if (c->nskipped)

@@ -32,6 +32,18 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr, uint32_t sbo_byte
     return d;
 }
 
+// K-major, 64-byte swizzle: 512-byte atoms of 8 rows by 32 bf16, one after another along the rows.
+__device__ __forceinline__ uint64_t desc_sw64(uint32_t saddr)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1u << 16;
+    d |= (uint64_t)(512u >> 4) << 32;
+    d |= (uint64_t)1u << 46;
+    d |= (uint64_t)4u << 61;                          // 64-byte swizzle
+    return d;
+}
+
 // Descriptor of an MN-major operand with 128-byte swizzle: 1024-byte atoms of
 // 64 bf16 along M/N by 8 rows of K; lbo = byte stride between atoms along
 // M/N, sbo = byte stride between 8-row groups of K.

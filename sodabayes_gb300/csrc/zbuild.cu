@@ -7,7 +7,7 @@
 //         fully reorthogonalised Lanczos run (lanczos.cuh) instead of the
 //         reference's power iteration (soda.f90:378-401): both converge to
 //         the same eigenvalue, Lanczos in far fewer products with A.
-//   U   = chol(d I - A), upper (choleskyPD, soda.f90:8-47)     k_chol_*
+//   U   = chol(d I - A), upper (choleskyPD, soda.f90:8-47)     chol_tc.cuh
 //   fallback for a failed factorisation: the reference's own sequence —
 //         the unpivoted attempt up to the failing row, then the pivoted
 //         factorisation (choleskyPSD, soda.f90:49-124) — in k_psd_block.
@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
+#include "chol_tc.cuh"
 #include "dgv.cuh"
 #include "gram_tc.cuh"
 #include "lanczos.cuh"
@@ -238,133 +239,6 @@ __global__ void k_form_m(double *W, const int64_t *wofs, const int32_t *blk_ls,
         const int i = (int)(t % N), j = (int)(t / N);
         const double v = -A[t];
         A[t] = i == j ? d + v : v;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// blocked right-looking Cholesky M = U'U (upper), batched over subsets
-// ---------------------------------------------------------------------------
-constexpr int CB = 32;   // panel width
-
-// factor the diagonal tile of panel kb; status[b] = failing row (1-based)
-__global__ void __launch_bounds__(1024) k_chol_diag(double *W, const int64_t *wofs, const int32_t *blk_ls,
-                                                    const int32_t *batch_blocks, int32_t *status, int kb)
-{
-    __shared__ double T[CB][CB + 1];
-    __shared__ int s_fail;
-    const int b = batch_blocks[blockIdx.x];
-    const int N = blk_ls[b + 1] - blk_ls[b];
-    if (kb >= N || status[b] != 0) return;
-    const int nbk = min(CB, N - kb);
-    double *A = W + wofs[b];
-    const int r = threadIdx.x >> 5, c = threadIdx.x & 31;
-    if (r < nbk && c < nbk) T[r][c] = A[(size_t)(kb + r) + (size_t)(kb + c) * N];
-    if (threadIdx.x == 0) s_fail = 0;
-    __syncthreads();
-    for (int j = 0; j < nbk; ++j) {
-        if (threadIdx.x == 0) {
-            const double v = T[j][j];
-            if (!(v > 0.0)) s_fail = kb + j + 1;
-            else T[j][j] = sqrt(v);
-        }
-        __syncthreads();
-        if (s_fail) break;
-        if (r == 0 && c > j && c < nbk) T[j][c] = T[j][c] / T[j][j];
-        __syncthreads();
-        if (r > j && c >= r && c < nbk) T[r][c] -= T[j][r] * T[j][c];
-        __syncthreads();
-    }
-    if (s_fail) {
-        if (threadIdx.x == 0) status[b] = s_fail;
-        return;
-    }
-    if (r < nbk && c < nbk && c >= r) A[(size_t)(kb + r) + (size_t)(kb + c) * N] = T[r][c];
-}
-
-// row panel: U[kb:kb+nbk, c] = U_kk'^{-1} M[kb:kb+nbk, c] for c >= kb+nbk
-__global__ void __launch_bounds__(256) k_chol_trsm(double *W, const int64_t *wofs, const int32_t *blk_ls,
-                                                   const int32_t *batch_blocks, const int32_t *status, int kb)
-{
-    __shared__ double T[CB][CB + 1];
-    const int b = batch_blocks[blockIdx.y];
-    const int N = blk_ls[b + 1] - blk_ls[b];
-    if (kb >= N || status[b] != 0) return;
-    const int nbk = min(CB, N - kb);
-    double *A = W + wofs[b];
-    for (int t = threadIdx.x; t < CB * CB; t += blockDim.x) {
-        const int r = t % CB, c = t / CB;
-        if (r < nbk && c < nbk) T[r][c] = A[(size_t)(kb + r) + (size_t)(kb + c) * N];
-    }
-    __syncthreads();
-    const int col = kb + nbk + blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= N) return;
-    double x[CB];
-    double *ac = A + (size_t)col * N + kb;
-#pragma unroll
-    for (int r = 0; r < CB; ++r) x[r] = r < nbk ? ac[r] : 0.0;
-#pragma unroll
-    for (int r = 0; r < CB; ++r) {
-        if (r < nbk) {
-            double s = x[r];
-#pragma unroll
-            for (int t = 0; t < r; ++t) s -= T[t][r] * x[t];
-            x[r] = s / T[r][r];
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < CB; ++r)
-        if (r < nbk) ac[r] = x[r];
-}
-
-// trailing update of the upper triangle: M[i,j] -= sum_t U[t,i] U[t,j]
-constexpr int UT = 64;
-__global__ void __launch_bounds__(256) k_chol_update(double *W, const int64_t *wofs, const int32_t *blk_ls,
-                                                     const int32_t *batch_blocks, const int32_t *status, int kb)
-{
-    __shared__ double Pi[CB][UT + 1];
-    __shared__ double Pj[CB][UT + 1];
-    const int b = batch_blocks[blockIdx.y];
-    const int N = blk_ls[b + 1] - blk_ls[b];
-    if (status[b] != 0) return;
-    const int k1 = kb + CB;
-    if (k1 >= N) return;
-    const int M = N - k1;
-    const int nt = (M + UT - 1) / UT;
-    int t = blockIdx.x, ti = 0;
-    while (ti < nt && t >= nt - ti) { t -= nt - ti; ++ti; }
-    if (ti >= nt) return;
-    const int tj = ti + t;
-    double *A = W + wofs[b];
-    const int i0 = k1 + ti * UT, j0 = k1 + tj * UT;
-    for (int q = threadIdx.x; q < CB * UT; q += blockDim.x) {
-        const int r = q % CB, c = q / CB;
-        const int ci = i0 + c, cj = j0 + c;
-        Pi[r][c] = ci < N ? A[(size_t)(kb + r) + (size_t)ci * N] : 0.0;
-        Pj[r][c] = cj < N ? A[(size_t)(kb + r) + (size_t)cj * N] : 0.0;
-    }
-    __syncthreads();
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-#pragma unroll 4
-    for (int r = 0; r < CB; ++r) {
-        double a[4], bb[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) { a[q] = Pi[r][ty + 16 * q]; bb[q] = Pj[r][tx + 16 * q]; }
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int s = 0; s < 4; ++s) acc[q][s] += a[q] * bb[s];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int i = i0 + ty + 16 * q;
-        if (i >= N) continue;
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const int j = j0 + tx + 16 * s;
-            if (j >= N || j < i) continue;
-            A[(size_t)i + (size_t)j * N] -= acc[q][s];
-        }
     }
 }
 
@@ -725,19 +599,31 @@ cudaError_t zb_form_m(double *W, const int64_t *wofs, const int32_t *blk_ls, con
     return cudaGetLastError();
 }
 
-cudaError_t zb_cholesky(double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks,
-                        int nbatch, int maxN, int32_t *status, cudaStream_t st)
+int zb_chol_np(int maxN) { return (maxN + CH_M - 1) / CH_M * CH_M; }
+int zb_chol_ldt(int maxN) { return (maxN + CH_P - 1) / CH_P * CH_P; }
+size_t zb_chol_digits(int maxN) { return (size_t)CH_DIG * zb_chol_np(maxN) * zb_chol_ldt(maxN); }
+size_t zb_chol_work(int maxN, int nbatch) { return (size_t)nbatch * (2 * zb_chol_np(maxN) + CH_P); }
+
+cudaError_t zb_cholesky(const CUtensorMap *tm_a, const CUtensorMap *tm_b, double *W, const int64_t *wofs,
+                        const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch, int maxN, const double *xxd,
+                        int32_t *status, uint16_t *dig, double *work, int *err, cudaStream_t st)
 {
-    for (int kb = 0; kb < maxN; kb += CB) {
-        k_chol_diag<<<nbatch, 1024, 0, st>>>(W, wofs, blk_ls, batch_blocks, status, kb);
-        const int rest = maxN - kb - CB;
-        if (rest > 0) {
-            k_chol_trsm<<<dim3((rest + 255) / 256, nbatch), 256, 0, st>>>(W, wofs, blk_ls, batch_blocks, status, kb);
-            const int nt = (rest + UT - 1) / UT;
-            k_chol_update<<<dim3(nt * (nt + 1) / 2, nbatch), 256, 0, st>>>(W, wofs, blk_ls, batch_blocks, status, kb);
-        }
+    const int np = zb_chol_np(maxN), ldt = zb_chol_ldt(maxN);
+    double *sc = work, *nrm = sc + (size_t)nbatch * np, *piv = nrm + (size_t)nbatch * np;
+    cudaError_t e = cudaFuncSetAttribute(k_ch_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM);
+    if (e != cudaSuccess) return e;
+    k_ch_init<<<nbatch, 256, 0, st>>>(W, wofs, blk_ls, batch_blocks, xxd, sc, nrm, np, status);
+    e = cudaGetLastError();
+    for (int i0 = 0; i0 < maxN && e == cudaSuccess; i0 += CH_P) {
+        e = launch_after(k_ch_update, dim3((maxN - i0 + CH_M - 1) / CH_M, nbatch), dim3(CH_THREADS), CH_SMEM, st, *tm_a,
+                         *tm_b, W, wofs, blk_ls, batch_blocks, xxd, (const double *)sc, np, status, i0, err);
+        if (e == cudaSuccess)
+            e = launch_after(k_ch_diag, dim3(nbatch), dim3(256), 0, st, W, wofs, blk_ls, batch_blocks, status, i0, piv);
+        if (e == cudaSuccess && maxN - i0 > CH_P)
+            e = launch_after(k_ch_trsm, dim3((maxN - i0 - CH_P + 31) / 32, nbatch), dim3(32), 0, st, W, wofs, blk_ls,
+                             batch_blocks, xxd, (const double *)sc, nrm, np, status, i0, (const double *)piv, dig, ldt);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t zb_pd_lengths(const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch, const int32_t *status,

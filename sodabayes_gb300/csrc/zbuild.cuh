@@ -32,8 +32,16 @@ cudaError_t zb_lz_step(const double *W, const int64_t *wofs, const int32_t *blk_
                        int mmax, int j, const uint8_t *done, cudaStream_t st);
 cudaError_t zb_form_m(double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch,
                       const double *xxd, cudaStream_t st);
-cudaError_t zb_cholesky(double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks,
-                        int nbatch, int maxN, int32_t *status, cudaStream_t st);
+// Cholesky of d I - A of a batch of subsets (chol_tc.cuh), A in W on entry, U's upper triangle there on return.
+// dig: nbatch * zb_chol_digits() digits, seen by tm_a and tm_b as rows of zb_chol_ldt() bf16 in boxes of 32 x 128 and
+// 32 x 64, 64-byte swizzle; work: zb_chol_work() doubles.
+int zb_chol_np(int maxN);
+int zb_chol_ldt(int maxN);
+size_t zb_chol_digits(int maxN);
+size_t zb_chol_work(int maxN, int nbatch);
+cudaError_t zb_cholesky(const CUtensorMap *tm_a, const CUtensorMap *tm_b, double *W, const int64_t *wofs,
+                        const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch, int maxN, const double *xxd,
+                        int32_t *status, uint16_t *dig, double *work, int *err, cudaStream_t st);
 cudaError_t zb_pd_lengths(const int32_t *blk_ls, const int32_t *batch_blocks, int nbatch, const int32_t *status,
                           int32_t *ulen, uint8_t *skip, cudaStream_t st);
 cudaError_t zb_psd_block(double *Wb, double *M, int N, int ls, int32_t *ulen, uint8_t *skip, int32_t *piv,

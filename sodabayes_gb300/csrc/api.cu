@@ -173,7 +173,9 @@ struct sodagpu_ctx {
     // staging of sodagpu_set_state and the output of sodagpu_subset_rhs
     double *st_g = nullptr, *st_vs = nullptr, *st_r = nullptr, *st_ra = nullptr, *st_pi = nullptr;
     int32_t *st_cls = nullptr;
-    double *rhs_buf = nullptr;
+    unsigned char *pinned = nullptr;     // page-locked host memory the device writes results to (host_buffer)
+    size_t pinned_bytes = 0;
+    double *dgv_buf = nullptr;           // sodagpu_compute_dgv: effects, predictions, the splits' sums
     double *tape = nullptr;              // injected-draw tape (sodagpu_set_tape)
     int tape_reps = 0;
     cudaGraphExec_t graph = nullptr;
@@ -198,6 +200,24 @@ struct sodagpu_ctx {
         *ptr = (T *)p_;
         return 0;
     }
+    // At least `bytes` of page-locked host memory, kept by the context (it grows to the largest result read so far,
+    // at most HOST_BUFFER_MAX for states); its contents last until the context's next call.
+    int host_buffer(size_t bytes)
+    {
+        if (bytes <= pinned_bytes) return 0;
+        if (pinned) cudaFreeHost(pinned);
+        pinned = nullptr;
+        pinned_bytes = 0;
+        void *p_ = nullptr;
+        const cudaError_t e = cudaHostAlloc(&p_, bytes, cudaHostAllocDefault);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(SODAGPU_E_NOMEM, "cudaHostAlloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+        }
+        pinned = (unsigned char *)p_;
+        pinned_bytes = bytes;
+        return 0;
+    }
     void release(void *p_)
     {
         if (!p_) return;
@@ -212,6 +232,10 @@ struct sodagpu_ctx {
         int _rc = (expr);         \
         if (_rc != 0) return _rc; \
     } while (0)
+
+// A chain's state is gathered by one kernel up to this size; larger ones are copied array by array (the copies then
+// run at their full rate, and the context need not keep so much page-locked memory).
+constexpr size_t HOST_BUFFER_MAX = (size_t)4 << 20;
 
 extern "C" {
 
@@ -1023,22 +1047,27 @@ int sodagpu_run(sodagpu_ctx *c, int32_t iters, sodagpu_trace_cb cb, void *user)
     if (iters == 0) return 0;
     const auto t0 = std::chrono::steady_clock::now();
     RunCtl h{};
-    CUDA_TRY(cudaMemcpyAsync(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost, c->st));
-    CUDA_TRY(cudaStreamSynchronize(c->st));
-    const int rep0 = h.rep;
-    const int thin = c->cfg.thin;
-    const int rows = (cb ? ((rep0 + iters) / thin - rep0 / thin) : 0) * c->C;
-    if (rows > c->trace_cap) {
-        if (c->trace) c->release(c->trace);
-        c->trace = nullptr;
-        TRY(c->alloc(&c->trace, rows, false));
-        c->trace_cap = rows;
+    int rows = 0;
+    if (cb) {   // the trace needs room for the iterations' rows, so the host needs the iteration counter
+        CUDA_TRY(cudaMemcpyAsync(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost, c->st));
+        CUDA_TRY(cudaStreamSynchronize(c->st));
+        const int rep0 = h.rep;
+        const int thin = c->cfg.thin;
+        rows = ((rep0 + iters) / thin - rep0 / thin) * c->C;
+        if (rows > c->trace_cap) {
+            if (c->trace) c->release(c->trace);
+            c->trace = nullptr;
+            TRY(c->alloc(&c->trace, rows, false));
+            c->trace_cap = rows;
+        }
+        h.trace_iter = 0;
+        h.trace_cap = rows;
+        h.trace_count = 0;
+        h.trace = c->trace;
+        CUDA_TRY(cudaMemcpyAsync(c->ctl, &h, sizeof h, cudaMemcpyHostToDevice, c->st));
+    } else {
+        CUDA_TRY(sweep_run_begin(c->D, c->st));
     }
-    h.trace_iter = 0;
-    h.trace_cap = cb ? rows : 0;
-    h.trace_count = 0;
-    h.trace = cb ? c->trace : nullptr;
-    CUDA_TRY(cudaMemcpyAsync(c->ctl, &h, sizeof h, cudaMemcpyHostToDevice, c->st));
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
@@ -1118,26 +1147,30 @@ int sodagpu_get_state(sodagpu_ctx *c, int32_t chain, double *g, int32_t *cls, do
     if (chain < 0 || chain >= c->C) return fail(SODAGPU_E_ARG, "chain out of range");
     const int p = c->p;
     const size_t off = (size_t)chain * p;
-    if (g) CUDA_TRY(cudaMemcpy(g, c->g + off, sizeof(double) * p, cudaMemcpyDeviceToHost));
-    if (cls) CUDA_TRY(cudaMemcpy(cls, c->cls + off, sizeof(int32_t) * p, cudaMemcpyDeviceToHost));
-    if (vara_s) CUDA_TRY(cudaMemcpy(vara_s, c->vara_s + off, sizeof(double) * p, cudaMemcpyDeviceToHost));
-    if (yadj) CUDA_TRY(cudaMemcpy(yadj, c->r + (size_t)chain * c->ldr, sizeof(double) * c->n, cudaMemcpyDeviceToHost));
-    if (yaadj) CUDA_TRY(cudaMemcpy(yaadj, c->ra + (size_t)chain * c->ldra, sizeof(double) * c->bs, cudaMemcpyDeviceToHost));
-    if (scalars) {
-        ChainScal *S = new ChainScal;
-        RunCtl h{};
-        cudaError_t e = cudaMemcpy(S, c->scal + chain, sizeof(ChainScal), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) {
-            delete S;
-            return fail(SODAGPU_E_CUDA, "reading chain scalars: %s", cudaGetErrorString(e));
-        }
-        scalars[0] = S->mu[h.rep & 1];
-        scalars[1] = S->vare;
-        scalars[2] = S->vara;
-        scalars[3] = S->included;
-        delete S;
+    unsigned want = (g ? STATE_G : 0) | (vara_s ? STATE_VARA_S : 0) | (yadj ? STATE_R : 0) | (yaadj ? STATE_RA : 0) |
+                    (cls ? STATE_CLS : 0);
+    StateLayout L = sweep_state_layout(c->D, want);
+    const bool copies = L.bytes > HOST_BUFFER_MAX;   // the arrays one by one, only the scalars through the kernel
+    if (copies) L = sweep_state_layout(c->D, 0);
+    TRY(c->host_buffer(L.bytes));
+    CUDA_TRY(sweep_get_state(c->D, chain, L, c->pinned, c->st));
+    CUDA_TRY(cudaStreamSynchronize(c->st));
+    if (copies) {
+        if (g) CUDA_TRY(cudaMemcpy(g, c->g + off, sizeof(double) * p, cudaMemcpyDeviceToHost));
+        if (cls) CUDA_TRY(cudaMemcpy(cls, c->cls + off, sizeof(int32_t) * p, cudaMemcpyDeviceToHost));
+        if (vara_s) CUDA_TRY(cudaMemcpy(vara_s, c->vara_s + off, sizeof(double) * p, cudaMemcpyDeviceToHost));
+        if (yadj)
+            CUDA_TRY(cudaMemcpy(yadj, c->r + (size_t)chain * c->ldr, sizeof(double) * c->n, cudaMemcpyDeviceToHost));
+        if (yaadj)
+            CUDA_TRY(cudaMemcpy(yaadj, c->ra + (size_t)chain * c->ldra, sizeof(double) * c->bs, cudaMemcpyDeviceToHost));
+    } else {
+        if (g) memcpy(g, c->pinned + L.g, sizeof(double) * p);
+        if (cls) memcpy(cls, c->pinned + L.cls, sizeof(int32_t) * p);
+        if (vara_s) memcpy(vara_s, c->pinned + L.vara_s, sizeof(double) * p);
+        if (yadj) memcpy(yadj, c->pinned + L.r, sizeof(double) * c->n);
+        if (yaadj) memcpy(yaadj, c->pinned + L.ra, sizeof(double) * c->bs);
     }
+    if (scalars) memcpy(scalars, c->pinned + L.scalars, 4 * sizeof(double));
     return 0;
 }
 
@@ -1196,13 +1229,13 @@ int subset_call(sodagpu_ctx *c, int32_t b, bool rhs_only)
     if (!c->have_chain) return fail(SODAGPU_E_STATE, "call sodagpu_init_chains first");
     if (c->regular) return fail(SODAGPU_E_UNSUPPORTED, "the regular sampler has no subsets");
     if (b < 0 || b >= c->nb) return fail(SODAGPU_E_ARG, "subset %d out of range 0..%d", b, c->nb - 1);
+    // the draw kernel writes the right-hand sides, chain c's at c * bs, to page-locked host memory
     Dev D = c->D;
-    if (rhs_only) {
-        if (!c->rhs_buf) TRY(c->alloc(&c->rhs_buf, (size_t)c->C * c->bs));
-        D.rhs_out = c->rhs_buf;
-    }
+    const size_t rhs_bytes = rhs_only ? round_up(sizeof(double) * c->C * c->bs, 16) : 0;
+    TRY(c->host_buffer(rhs_bytes + sizeof(RunCtl)));
+    RunCtl &h = *reinterpret_cast<RunCtl *>(c->pinned + rhs_bytes);
+    if (rhs_only) D.rhs_out = reinterpret_cast<double *>(c->pinned);
     CUDA_TRY(sweep_enqueue_subset(D, b, c->blk_sizes[b], c->sm_count, &c->maps, c->st, rhs_only));
-    RunCtl h{};
     CUDA_TRY(cudaMemcpyAsync(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost, c->st));
     CUDA_TRY(cudaStreamSynchronize(c->st));
     if (h.err) return fail(SODAGPU_E_TIMEOUT, "a bounded device loop gave up (code %d)", h.err);
@@ -1216,8 +1249,8 @@ int sodagpu_subset_rhs(sodagpu_ctx *c, int32_t b, double *rhs)
     TRY(subset_call(c, b, true));
     const int N = c->blk_sizes[b];
     for (int ch = 0; ch < c->C; ++ch)
-        CUDA_TRY(cudaMemcpy(rhs + (size_t)ch * N, c->rhs_buf + (size_t)ch * c->bs, sizeof(double) * N,
-                            cudaMemcpyDeviceToHost));
+        memcpy(rhs + (size_t)ch * N, reinterpret_cast<const double *>(c->pinned) + (size_t)ch * c->bs,
+               sizeof(double) * N);
     return 0;
 }
 
@@ -1248,16 +1281,14 @@ int sodagpu_compute_dgv(sodagpu_ctx *c, double mu, const double *effects, double
 {
     if (!c || !effects || !pred) return fail(SODAGPU_E_ARG, "null argument");
     if (!c->have_z) return fail(SODAGPU_E_STATE, "no genotypes in subset order (run sodagpu_build_z)");
-    // one allocation: effects, predictions, the splits' sums
-    double *buf = nullptr;
-    TRY(c->alloc(&buf, (size_t)c->p + c->n + (size_t)zb_dgv_splits(c->n, c->p) * c->n, false));
-    double *deff = buf, *dpred = deff + c->p, *part = dpred + c->n;
+    // kept by the context: p + (splits + 1) n doubles, at most about 20 MB more than effects and predictions
+    if (!c->dgv_buf) TRY(c->alloc(&c->dgv_buf, (size_t)c->p + c->n + (size_t)zb_dgv_splits(c->n, c->p) * c->n, false));
+    double *deff = c->dgv_buf, *dpred = deff + c->p, *part = dpred + c->n;
     cudaError_t e = cudaMemcpyAsync(deff, effects, sizeof(double) * c->p, cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess)
         e = zb_dgv(c->G, c->ldx, c->xv, nullptr, c->perm, deff, c->n, c->p, mu, part, dpred, c->st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(pred, dpred, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-    c->release(buf);
     if (e != cudaSuccess) return fail(SODAGPU_E_CUDA, "genomic values: %s", cudaGetErrorString(e));
     return 0;
 }
@@ -1394,6 +1425,7 @@ struct sodagpu_batch {
     cudaStream_t st = nullptr;
     cudaGraphExec_t graph = nullptr;
     Dev *ddev = nullptr;
+    int32_t *derr = nullptr;             // the jobs' error flags after a run
     double last_ms = 0.0;
 };
 
@@ -1405,6 +1437,7 @@ void sodagpu_batch_destroy(sodagpu_batch *b)
     if (b->st) cudaStreamSynchronize(b->st);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->ddev) cudaFree(b->ddev);
+    if (b->derr) cudaFree(b->derr);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
 }
@@ -1462,6 +1495,7 @@ int sodagpu_batch_create(sodagpu_batch **out, sodagpu_ctx *const *jobs, int32_t 
     }
     cudaError_t e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&b->ddev, sizeof(Dev) * njobs);
+    if (e == cudaSuccess) e = cudaMalloc(&b->derr, sizeof(int32_t) * njobs);
     if (e == cudaSuccess) e = cudaMemcpy(b->ddev, hdev.data(), sizeof(Dev) * njobs, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         sodagpu_batch_destroy(b);
@@ -1493,35 +1527,26 @@ int sodagpu_batch_run(sodagpu_batch *b, int32_t iters)
     if (iters < 0) return fail(SODAGPU_E_ARG, "iters < 0");
     if (iters == 0) return 0;
     CUDA_TRY(cudaSetDevice(b->dev));
-    // each job's control block: no trace rows; the job's own stream drained first
-    for (auto *c : b->jobs) {
-        RunCtl h{};
-        CUDA_TRY(cudaMemcpyAsync(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost, c->st));
-        CUDA_TRY(cudaStreamSynchronize(c->st));
-        h.trace_iter = 0;
-        h.trace_cap = 0;
-        h.trace_count = 0;
-        h.trace = nullptr;
-        CUDA_TRY(cudaMemcpyAsync(c->ctl, &h, sizeof h, cudaMemcpyHostToDevice, c->st));
-        CUDA_TRY(cudaStreamSynchronize(c->st));
-    }
+    // no trace rows; every job's own stream drained first
+    for (auto *c : b->jobs) CUDA_TRY(cudaStreamSynchronize(c->st));
+    CUDA_TRY(sweep_batch_begin(b->ddev, (int)b->jobs.size(), b->st));
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     CUDA_TRY(cudaEventRecord(e0, b->st));
     for (int t = 0; t < iters; ++t) CUDA_TRY(cudaGraphLaunch(b->graph, b->st));
     CUDA_TRY(cudaEventRecord(e1, b->st));
+    int32_t errs[MAXJOBS] = {0};
+    CUDA_TRY(sweep_batch_errors(b->ddev, (int)b->jobs.size(), b->derr, b->st));
+    CUDA_TRY(cudaMemcpyAsync(errs, b->derr, sizeof(int32_t) * b->jobs.size(), cudaMemcpyDeviceToHost, b->st));
     CUDA_TRY(cudaStreamSynchronize(b->st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     b->last_ms = ms;
-    for (size_t j = 0; j < b->jobs.size(); ++j) {
-        RunCtl h{};
-        CUDA_TRY(cudaMemcpy(&h, b->jobs[j]->ctl, sizeof h, cudaMemcpyDeviceToHost));
-        if (h.err) return fail(SODAGPU_E_TIMEOUT, "job %zu: a bounded device loop gave up (code %d)", j, h.err);
-    }
+    for (size_t j = 0; j < b->jobs.size(); ++j)
+        if (errs[j]) return fail(SODAGPU_E_TIMEOUT, "job %zu: a bounded device loop gave up (code %d)", j, errs[j]);
     return 0;
 }
 
@@ -1590,6 +1615,7 @@ void sodagpu_destroy(sodagpu_ctx *c)
     if (c->graph) cudaGraphExecDestroy(c->graph);
     for (void *p_ : c->allocs) cudaFree(p_);
     c->allocs.clear();
+    if (c->pinned) cudaFreeHost(c->pinned);
     if (c->st) cudaStreamDestroy(c->st);
     delete c;
 }

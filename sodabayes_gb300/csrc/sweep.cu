@@ -1626,6 +1626,104 @@ cudaError_t sweep_set_state(const Dev &D, int c, const double *g, const int32_t 
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Reading one chain's state and starting a run: one launch in place of a copy per array.  A copy of a few hundred
+// bytes to the host takes 11 us, and one chain's state was seven of them (one of 100 KB for four scalars): 87 us at
+// p = 20,000, 48 us through one kernel that writes to page-locked host memory, which the GPU reaches coherently.
+// ---------------------------------------------------------------------------
+// out: g, vara_s (nloci each), yadj (nind), yaadj (bs), {mu, vare, vara, included}, then cls (int32); an array whose
+// bit of `want` is 0 is left out (sweep_state_layout gives the places).
+__global__ void __launch_bounds__(256) k_get_state(Dev D, int c, StateLayout L, unsigned char *out)
+{
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    auto put = [&](size_t at, const double *src, int n) {
+        double *dst = reinterpret_cast<double *>(out + at);
+        for (int i = t0; i < n; i += stride) dst[i] = src[i];
+    };
+    if (L.want & STATE_G) put(L.g, D.g + (size_t)c * D.p, D.p);
+    if (L.want & STATE_VARA_S) put(L.vara_s, D.vara_s + (size_t)c * D.p, D.p);
+    if (L.want & STATE_R) put(L.r, D.r + (size_t)c * D.ldr, D.n);
+    if (L.want & STATE_RA) put(L.ra, D.ra + (size_t)c * D.ldra, D.bs);
+    if (L.want & STATE_CLS) {
+        int32_t *dst = reinterpret_cast<int32_t *>(out + L.cls);
+        for (int i = t0; i < D.p; i += stride) dst[i] = D.cls[(size_t)c * D.p + i];
+    }
+    if (t0 == 0) {
+        const ChainScal *S = &D.scal[c];
+        double *dst = reinterpret_cast<double *>(out + L.scalars);
+        dst[0] = S->mu[D.ctl->rep & 1];
+        dst[1] = S->vare;
+        dst[2] = S->vara;
+        dst[3] = (double)S->included;
+    }
+}
+
+StateLayout sweep_state_layout(const Dev &D, unsigned want)
+{
+    StateLayout L{};
+    L.want = want;
+    auto take = [&](unsigned bit, size_t bytes) {
+        const size_t at = L.bytes;
+        if (want & bit) L.bytes += (bytes + 15) & ~(size_t)15;
+        return at;
+    };
+    L.g = take(STATE_G, sizeof(double) * (size_t)D.p);
+    L.vara_s = take(STATE_VARA_S, sizeof(double) * (size_t)D.p);
+    L.r = take(STATE_R, sizeof(double) * (size_t)D.n);
+    L.ra = take(STATE_RA, sizeof(double) * (size_t)D.bs);
+    L.scalars = L.bytes;
+    L.bytes += 4 * sizeof(double);
+    L.cls = take(STATE_CLS, sizeof(int32_t) * (size_t)D.p);
+    return L;
+}
+
+cudaError_t sweep_get_state(const Dev &D, int c, const StateLayout &L, unsigned char *out, cudaStream_t st)
+{
+    const int grid = std::max(1, std::min((std::max(D.p, D.n) + 255) / 256, 152));
+    k_get_state<<<grid, 256, 0, st>>>(D, c, L, out);
+    return cudaGetLastError();
+}
+
+// No trace rows for the next iterations of a job (or of every job of a batch).
+__global__ void k_run_begin(Dev D)
+{
+    D.ctl->trace_iter = 0;
+    D.ctl->trace_cap = 0;
+    D.ctl->trace_count = 0;
+    D.ctl->trace = nullptr;
+}
+__global__ void k_run_begin_m(const Dev *dev, int njobs)
+{
+    const int j = threadIdx.x;
+    if (j >= njobs) return;
+    RunCtl *ctl = dev[j].ctl;
+    ctl->trace_iter = 0;
+    ctl->trace_cap = 0;
+    ctl->trace_count = 0;
+    ctl->trace = nullptr;
+}
+__global__ void k_batch_errors(const Dev *dev, int njobs, int32_t *out)
+{
+    const int j = threadIdx.x;
+    if (j < njobs) out[j] = dev[j].ctl->err;
+}
+
+cudaError_t sweep_run_begin(const Dev &D, cudaStream_t st)
+{
+    k_run_begin<<<1, 1, 0, st>>>(D);
+    return cudaGetLastError();
+}
+cudaError_t sweep_batch_begin(const Dev *ddev, int njobs, cudaStream_t st)
+{
+    k_run_begin_m<<<1, MAXJOBS, 0, st>>>(ddev, njobs);
+    return cudaGetLastError();
+}
+cudaError_t sweep_batch_errors(const Dev *ddev, int njobs, int32_t *out, cudaStream_t st)
+{
+    k_batch_errors<<<1, MAXJOBS, 0, st>>>(ddev, njobs, out);
+    return cudaGetLastError();
+}
+
 cudaError_t sweep_enqueue_recal(const Dev &D, double mu_slot_unused, cudaStream_t st)
 {
     (void)mu_slot_unused;

@@ -84,6 +84,18 @@ cudaError_t sweep_enqueue_subset(const Dev &D, int b, int nsnp, int sm_count, co
 cudaError_t sweep_set_state(const Dev &D, int c, const double *g, const int32_t *cls, const double *vs,
                             const double *r, const double *ra, const double *pi, double mu, double vare, double vara,
                             int included, cudaStream_t st);
+// One chain's state gathered into a buffer the device can write (page-locked host memory): which arrays, where.
+enum { STATE_G = 1, STATE_VARA_S = 2, STATE_R = 4, STATE_RA = 8, STATE_CLS = 16 };
+struct StateLayout {
+    unsigned want;
+    size_t g, vara_s, r, ra, scalars, cls, bytes;
+};
+StateLayout sweep_state_layout(const Dev &D, unsigned want);
+cudaError_t sweep_get_state(const Dev &D, int c, const StateLayout &L, unsigned char *out, cudaStream_t st);
+// Resets the trace fields of a job's (every job's of a batch) control block; the jobs' error flags.
+cudaError_t sweep_run_begin(const Dev &D, cudaStream_t st);
+cudaError_t sweep_batch_begin(const Dev *ddev, int njobs, cudaStream_t st);
+cudaError_t sweep_batch_errors(const Dev *ddev, int njobs, int32_t *out, cudaStream_t st);
 cudaError_t sweep_enqueue_recal(const Dev &D, double unused, cudaStream_t st);
 
 // Several jobs per launch (CUDA-core kernels; the jobs share precision and

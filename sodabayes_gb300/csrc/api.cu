@@ -148,9 +148,9 @@ struct sodagpu_ctx {
     uint32_t *indist = nullptr;
     ChainScal *scal = nullptr;
     RunCtl *ctl = nullptr;
-    double *delta = nullptr, *rpart = nullptr, *rsum = nullptr, *statpart = nullptr, *recal_part = nullptr,
+    double *delta = nullptr, *rpart = nullptr, *rsum = nullptr, *statpart = nullptr, *recal_part = nullptr, *ssrec = nullptr,
            *upart = nullptr, *rpx = nullptr, *rpu = nullptr;
-    int32_t *cntpart = nullptr, *ucount = nullptr;
+    int32_t *cntpart = nullptr, *ucount = nullptr, *ssdense = nullptr;
     uint8_t *nzflag = nullptr;
     int tc = 0, ldd = 0;                 // tensor-core sweep
     uint16_t *dsplit = nullptr;
@@ -876,6 +876,8 @@ int build_dev(sodagpu_ctx *c)
     D.statpart = c->statpart;
     D.cntpart = c->cntpart;
     D.recal_part = c->recal_part;
+    D.ssrec = c->ssrec;
+    D.ssdense = c->ssdense;
     D.rpx = c->rpx;
     D.rpu = c->rpu;
     D.tc = c->tc;
@@ -953,6 +955,10 @@ int sodagpu_init_chains(sodagpu_ctx *c)
         TRY(c->alloc(&c->statpart, (size_t)C * NSTAT * ngm));
         TRY(c->alloc(&c->cntpart, (size_t)C * NSTAT * ngm));
         TRY(c->alloc(&c->recal_part, (size_t)C * RECAL_SPLIT * c->ldr));
+        if (c->nskipped) {
+            TRY(c->alloc(&c->ssrec, sweep_skip_records(c->nskipped, C, nm), false));
+            TRY(c->alloc(&c->ssdense, C));
+        }
         TRY(c->alloc(&c->rpx, (size_t)RHS_KSPLIT_MAX * C * c->bs));
         TRY(c->alloc(&c->rpu, (size_t)RHS_KSPLIT_MAX * C * c->bs));
         c->tc = !c->regular && c->cfg.kernels == SODAGPU_KERNELS_AUTO &&

@@ -109,6 +109,8 @@ struct Dev {
     double *statpart;          // [C][NSTAT][ngroup*nmix] sum g^2
     int32_t *cntpart;          // [C][NSTAT][ngroup*nmix] counts
     double *recal_part;        // [C][RECAL_SPLIT][ldr]
+    double *ssrec;             // [C][min(nskipped, SS_CHUNK)][SS_HEAD + 2 nmix] single-site draws' constants
+    int32_t *ssdense;          // [C] SNPs of the current chunk that are in the model
     double *rpx, *rpu;         // [RHS_KSPLIT_MAX][C][bs] rhs partial sums (genotype / augmented part)
     // tensor-core sweep (FP8 mode, 4/8/16 chains)
     int tc;                    // 1 when the tensor-core kernels run

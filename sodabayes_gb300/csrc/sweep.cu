@@ -12,6 +12,7 @@
 //   ra redraw, posterior accumulators    k_post                      (models.f90:523-548)
 //   residual recalibration               k_recal_partial/_apply      (models.f90:571-573)
 // All chains of the context advance together inside each launch.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "rng.cuh"
@@ -449,189 +450,428 @@ namespace soda {
 // ---------------------------------------------------------------------------
 // Single-site updates, one CTA per chain, SNPs in order: the SNPs the pivoted
 // fallback skips (models.f90:178-193, 276-320, 433-495) and, for the regular
-// sampler, every SNP (regular_bayes, models.f90:717-859).  The residual is
-// held in shared memory when it fits (each thread owns the same individuals
-// in the dot product and in the update, so only the reduction and the draw
-// need barriers); the mixture-class scores and the exponentials of their
-// differences are computed by parallel lanes of warp 0 and added by lane 0 in
-// the reference's order.  The reference reads module copies of log_p /
-// vare_gp for skipped SNPs that its parallel regions never assign; the
-// current values are used.
+// sampler, every SNP (regular_bayes, models.f90:717-859).  The reference reads
+// module copies of log_p / vare_gp for skipped SNPs that its parallel regions
+// never assign; the current values are used.
+//
+// The SNPs are a serial chain, so what counts is the latency of one: GB300's FP64
+// pipe takes 64 cycles for a warp's instruction (a quarter of the SM each), and a
+// logarithm is thirty of them.  All that does not depend on the residual - the
+// uniforms, the normal and gamma variates, the class scores' constants - is
+// computed beforehand by k_skipped_pre, in parallel over the SNPs; k_skipped is
+// left with the dot product (four warps, one on each quarter; the residual in
+// shared memory, the next SNP's codes and constants loaded ahead), one
+// multiply-add and one exponential per class, in parallel lanes, and a comparison.
+// n = 2,326, BayesR: 3.4 us a SNP, against 7.1 us when the draw did it all.
+//
+// The chain is serial only where a SNP changes the residual.  A SNP outside the
+// model that stays outside leaves it as it is, and after burn-in that is nearly all
+// of them; so k_skipped_spec draws SS_SPEC consecutive SNPs at once against the same
+// residual, keeps the draws up to and including the first that changes it, applies
+// that change and goes on behind it: the draws of the serial chain exactly, 24 SNPs
+// a round at 2% in the model.  The same data: 0.54 us a SNP.  Chains with more than a
+// quarter of the SNPs in the model (and BayesA's, with all of them) go one by one.
 // ---------------------------------------------------------------------------
-constexpr int SS_THREADS = 512;
 constexpr int SS_SMEM_MAX = 200 * 1024;   // residual in shared memory up to 25,600 individuals
+constexpr int SS_CHUNK = 16384;           // SNPs per pair of launches: bounds the records
+constexpr int SS_HEAD = 12;               // a record's doubles before the (c_k, b_k) pairs of the classes
+enum { SS_U = 0, SS_POS, SS_SNP, SS_RR, SS_SN, SS_DEN, SS_SD, SS_SDV, SS_GD, SS_GV, SS_GW, SS_FLAGS };
+constexpr int SS_CTAS = 8;                // CTAs of a chain's cluster in k_skipped_spec, four warps each
+constexpr int SS_SPEC = 4 * SS_CTAS;      // SNPs a round
+constexpr double SS_SMALL = 1.0, SS_PLAIN = 2.0;   // SS_FLAGS: gamma shape below 1; a standard deviation is 0
 
-// Lane 0 returns the update delta = g_old - g_new of SNP snploc of chain c
-// (its new effect, class and locus variance written); all 32 lanes enter.
-__device__ __forceinline__ double single_site_draw(const Dev &D, ChainScal *S, int c, int rep, int snploc, double dot)
+int sweep_skip_stride(int nmix) { return SS_HEAD + 2 * nmix; }
+size_t sweep_skip_records(int nskipped, int chains, int nmix)
 {
-    const int lane = threadIdx.x & 31;
-    const size_t o = (size_t)c * D.p + snploc;
-    const double vare = S->vare, zz = D.xpx[snploc], zz_vare = zz / vare;
-    const int m = D.method, ng = D.ngroup, nm = D.nmix;
-    double rhs = dot, upd = 0.0;
-    int err = 0;
-    if (m != SODAGPU_BAYES_A && m != SODAGPU_BAYES_B) {
-        // BayesC/Cpi/R/Rc: scores by lanes 0..nm-1, exponentials of their differences by lanes (kk, j)
-        const double gk = D.g[o];
-        const int cl = D.cls[o];
-        if (cl > 1) rhs = rhs + zz * gk;
-        const int sg = D.grp[snploc] - 1;
-        double sv = 0.0;
-        if (lane == 0) sv = S->log_p[sg];
-        else if (lane < nm) {
-            const double logdetV = log(S->gp[lane] * zz_vare + 1.0);
-            const double uhat = rhs / (zz + S->vare_gp[lane]);
-            sv = -0.5 * (logdetV - (rhs * uhat / vare)) + S->log_p[sg + lane * ng];
-        }
-        const bool par = nm * nm <= 32;
-        const int kq = lane / (nm > 0 ? nm : 1), jq = lane % (nm > 0 ? nm : 1);
-        const double skq = __shfl_sync(0xffffffffu, sv, par ? kq : 0);
-        const double sjq = __shfl_sync(0xffffffffu, sv, par ? jq : 0);
-        double ev = 0.0;
-        if (par && lane < nm * nm && kq != jq) {
-            const double clike = sjq - skq;
-            if (clike >= -700 && clike <= 700) ev = exp(clike);
-        }
-        double s[MAXDIST];
-        double e[MAXDIST * MAXDIST > 32 ? 32 : MAXDIST * MAXDIST];
-#pragma unroll
-        for (int t = 0; t < MAXDIST; ++t) s[t] = __shfl_sync(0xffffffffu, sv, t < 32 ? t : 0);
-#pragma unroll
-        for (int t = 0; t < 32; ++t) {
-            const double v = __shfl_sync(0xffffffffu, ev, t);
-            if (t < (int)(sizeof(e) / sizeof(e[0]))) e[t] = v;
-        }
-        if (lane == 0) {
-            CRng R;
-            crng_site(R, D, c, rep, snploc, P_SKIP);
-            const double u = crng_unit(R);
-            double ssculm = 0.0;
-            int flag = 1;
-            for (int kk = 0; kk < nm; ++kk) {
-                const double skk = s[kk];
-                double sk = 0.0;
-                bool overflow = false;
-                for (int j = 0; j < nm; ++j) {
-                    if (j == kk) continue;
-                    const double clike = s[j] - skk;
-                    if (clike < -700) continue;
-                    if (clike > 700) { overflow = true; break; }
-                    sk = sk + (par ? e[kk * nm + j] : exp(clike));
-                }
-                ssculm = ssculm + (overflow ? 0.0 : 1.0 / (1.0 + sk));
-                if (u < ssculm) { flag = kk + 1; break; }
-            }
-            double gt = 0.0;
-            if (flag == 1) {
-                upd = cl > 1 ? gk : 0.0;
-            } else {
-                const double v1 = zz + vare / S->gp[flag - 1];
-                gt = d_rnorm(rhs / v1, sqrt(vare / v1), R);
-                upd = gk - gt;
-            }
-            D.g[o] = gt;
-            D.cls[o] = flag;
-        }
-        return upd;
-    }
-    if (lane == 0) {
-        const double gk = D.g[o];
-        double gt = 0.0;
-        CRng R;
-        crng_site(R, D, c, rep, snploc, P_SKIP);
-        if (m == SODAGPU_BAYES_A) {
-            rhs = rhs + zz * gk;
-            const double v1 = zz + vare / D.vara_s[o];
-            gt = d_rnorm(rhs / v1, sqrt(vare / v1), R);
-            upd = gk - gt;
-            D.g[o] = gt;
-        } else {
-            if (D.cls[o] > 1) rhs = rhs + zz * gk;
-            const double vs = D.vara_s[o];
-            const double s1 = S->log_p[0];
-            const double logdetV = log(vs * zz_vare + 1.0);
-            const double uhat = rhs / (zz + vare / vs);
-            const double s2 = -0.5 * (logdetV - (rhs * uhat / vare)) + S->log_p[ng];
-            const double clike = s1 - s2;
-            double sk;
-            if (clike > 700) sk = 0.0;
-            else if (clike < -700) sk = 1.0;
-            else sk = 1.0 / (1.0 + exp(clike));
-            const double u = crng_unit(R);
-            const int flag = u < sk ? 2 : 1;
-            if (flag == 1) {
-                gt = d_rnorm(0.0, sqrt(vs), R);
-                upd = D.cls[o] > 1 ? gk : 0.0;
-                D.g[o] = 0.0;
-            } else {
-                const double v1 = zz + vare / vs;
-                gt = d_rnorm(rhs / v1, sqrt(vare / v1), R);
-                upd = gk - gt;
-                D.g[o] = gt;
-            }
-            D.cls[o] = flag;
-        }
-        const double scale = (gt * gt + S->scale_va * D.df_va) / (D.df_va + 1.0);
-        D.vara_s[o] = d_rscinvchi2(D.df_va + 1.0, scale, R, &err);
-        if (err) flag_err(D, 1);
-    }
-    return upd;
+    return (size_t)std::min(nskipped, SS_CHUNK) * chains * sweep_skip_stride(nmix);
 }
 
-__device__ __forceinline__ void skipped_body(const Dev &D, const VB &vb)
+// Record of skipped SNP t0 + t (of cnt) of chain c.  Class k's score, for right-hand side rhs, is b_k + c_k rhs^2
+// (models.f90:362-366 with the quotient rhs^2 / ((zz + sigma2_e / gamma) sigma2_e) as one factor).
+__device__ __forceinline__ void skipped_pre_body(const Dev &D, const VB &vb, int t0, int cnt)
 {
-    extern __shared__ double s_r[];
-    __shared__ double s_part[SS_THREADS / 32];
+    const int t = vb.x * 64 + threadIdx.x, c = vb.y;
+    if (t >= cnt) return;
+    const int rep = cur_rep(D), snp = D.iskipped[t0 + t], m = D.method, nm = D.nmix, ng = D.ngroup;
+    const ChainScal *S = &D.scal[c];
+    const double vare = S->vare, zz = D.xpx[snp], zz_vare = zz / vare;
+    const int stride = SS_HEAD + 2 * nm;
+    double *q = D.ssrec + ((size_t)c * min(D.nskipped, SS_CHUNK) + t) * stride;
+    CRng R;
+    crng_site(R, D, c, rep, snp, P_SKIP);
+    q[SS_POS] = (double)D.pos_of[snp];
+    q[SS_SNP] = (double)snp;
+    // how many of the chunk's SNPs are in the model (cleared before the launch)
+    if (m != SODAGPU_BAYES_A && D.cls[(size_t)c * D.p + snp] > 1) atomicAdd(&D.ssdense[c], 1);
+    if (m == SODAGPU_BAYES_A || m == SODAGPU_BAYES_B) {
+        const double vs = D.vara_s[(size_t)c * D.p + snp];
+        DrawSub<double> sub;
+        sub.vare = vare;
+        sub.zz_vare = zz_vare;
+        DrawSnp<double> a;
+        a.u = a.ld = a.sdv = 0.0;
+        draw_ahead(D, sub, zz, vs, R, a);
+        q[SS_U] = a.u;
+        q[SS_DEN] = a.den;
+        q[SS_SD] = a.sd;
+        q[SS_SDV] = a.sdv;
+        q[SS_FLAGS] = a.plain ? SS_PLAIN : (a.gam.small ? SS_SMALL : 0.0);
+        if (!a.plain) {
+            q[SS_RR] = a.z.rr;
+            q[SS_SN] = a.z.sn;
+            q[SS_GD] = a.gam.d;
+            q[SS_GV] = a.gam.v;
+            q[SS_GW] = a.gam.wp;
+        }
+        if (m == SODAGPU_BAYES_B) {
+            q[SS_HEAD] = 0.0;
+            q[SS_HEAD + 1] = S->log_p[0];
+            q[SS_HEAD + 2] = 0.5 / (a.den * vare);
+            q[SS_HEAD + 3] = S->log_p[ng] - 0.5 * a.ld;
+        }
+        if (a.err) flag_err(D, 1);
+        return;
+    }
+    const int sg = D.grp[snp] - 1;
+    q[SS_U] = crng_unit(R);
+    const NormalPre<double> z = normal_pre<double>(R);
+    q[SS_RR] = z.rr;
+    q[SS_SN] = z.sn;
+    q[SS_HEAD] = 0.0;
+    q[SS_HEAD + 1] = S->log_p[sg];
+    for (int k = 1; k < nm; ++k) {
+        q[SS_HEAD + 2 * k] = 0.5 / ((zz + S->vare_gp[k]) * vare);
+        q[SS_HEAD + 2 * k + 1] = S->log_p[sg + k * ng] - 0.5 * log(S->gp[k] * zz_vare + 1.0);
+    }
+}
+
+__global__ void __launch_bounds__(64) k_skipped_pre(Dev D, int t0, int cnt)
+{
+    skipped_pre_body(D, vb_native(), t0, cnt);
+}
+
+// The class of a SNP (1-based) from its uniform u and this lane's class score s (lanes 0 .. nm-1; all 32 enter): the
+// first class whose cumulative weight exceeds u times their sum, weights exp(s_k - s_0), or relative to the largest
+// score where that could overflow.
+__device__ __forceinline__ int skipped_class(double s, double u, int nm)
+{
+    const int lane = threadIdx.x & 31;
+    const double d = s - __shfl_sync(0xffffffffu, s, 0);
+    double w = d;
+    if (__ballot_sync(0xffffffffu, lane < nm && d > 700.0)) {
+        double top = lane < nm ? s : -1e308;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+        w = s - top;
+    }
+    w = lane < nm ? exp(w) : 0.0;
+    for (int o = 1; o < nm; o <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += v;
+    }
+    const double sum = __shfl_sync(0xffffffffu, w, nm - 1);
+    const unsigned hit = __ballot_sync(0xffffffffu, lane < nm && u * sum < w);
+    return hit ? __ffs(hit) : 1;
+}
+
+// The draws of a record whose standard deviation is 0, in the plain order (A/B; practically never).
+static __device__ __noinline__ void skipped_plain(const Dev &D, int c, int rep, int snp, double mean, double sd,
+                                                  double &gt, GammaPre<double> &gam)
+{
+    CRng R;
+    int err = 0;
+    crng_site(R, D, c, rep, snp, P_SKIP);
+    if (D.method == SODAGPU_BAYES_B) crng_unit(R);
+    gt = t_rnorm<double>(mean, sd, R);
+    gam = gamma_pre<double>(0.5 * (D.df_va + 1.0), R, &err);
+    if (err) flag_err(D, 1);
+}
+
+// The draw of SNP snp of chain c from its dot product, by a warp (the same in every lane): its new effect and class and
+// upd = g_old - g_new.  gk, cl: the SNP's effect and class; cb: this lane's class constants; q: its record, u its
+// uniform.
+struct SkippedDraw {
+    double upd, gt;
+    int flag;
+    GammaPre<double> gam;
+};
+__device__ __forceinline__ SkippedDraw skipped_draw(const Dev &D, const ChainScal *S, int c, int rep, int snp,
+                                                    double dot, double gk, int cl, double zz, double2 cb,
+                                                    const double *q, double u)
+{
+    const int lane = threadIdx.x & 31, m = D.method, nm = D.nmix;
+    SkippedDraw x;
+    double rhs = dot;
+    if (m == SODAGPU_BAYES_A || cl > 1) rhs = rhs + zz * gk;
+    x.flag = 2;
+    if (m != SODAGPU_BAYES_A) {
+        const double s = lane == 0 ? cb.y : fma(rhs * rhs, cb.x, cb.y);
+        if (m == SODAGPU_BAYES_B)   // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2))
+            x.flag = u * (1.0 + exp(__shfl_sync(0xffffffffu, s, 0) - __shfl_sync(0xffffffffu, s, 1))) < 1.0 ? 2 : 1;
+        else x.flag = skipped_class(s, u, nm);
+    }
+    x.upd = x.gt = 0.0;
+    if (m == SODAGPU_BAYES_A || m == SODAGPU_BAYES_B) {
+        const double mean = x.flag == 1 ? 0.0 : rhs / q[SS_DEN], sd = x.flag == 1 ? q[SS_SDV] : q[SS_SD];
+        x.gam = {q[SS_GD], q[SS_GV], q[SS_GW], q[SS_FLAGS] == SS_SMALL};
+        if (q[SS_FLAGS] == SS_PLAIN) {
+            skipped_plain(D, c, rep, snp, mean, sd, x.gt, x.gam);
+        } else {
+            const NormalPre<double> z = {q[SS_RR], q[SS_SN]};
+            x.gt = normal_from(mean, sd, z);
+        }
+        x.upd = x.flag == 1 ? (cl > 1 ? gk : 0.0) : gk - x.gt;
+    } else if (x.flag != 1) {
+        const double vare = S->vare, v1 = zz + vare / S->gp[x.flag - 1], sd = sqrt(vare / v1), mean = rhs / v1;
+        const NormalPre<double> z = {q[SS_RR], q[SS_SN]};
+        x.gt = sd <= 0.0 ? mean : normal_from(mean, sd, z);
+        x.upd = gk - x.gt;
+    } else if (cl > 1) {
+        x.upd = gk;
+    }
+    return x;
+}
+
+// Writes the draw (one thread).
+__device__ __forceinline__ void skipped_commit(const Dev &D, const ChainScal *S, int c, int snp, const SkippedDraw &x)
+{
+    const int m = D.method;
+    const size_t o = (size_t)c * D.p + snp;
+    if (m == SODAGPU_BAYES_A || m == SODAGPU_BAYES_B) {
+        D.g[o] = x.flag == 1 ? 0.0 : x.gt;
+        if (m == SODAGPU_BAYES_B) D.cls[o] = x.flag;
+        const double scale = (x.gt * x.gt + S->scale_va * D.df_va) / (D.df_va + 1.0);
+        D.vara_s[o] = scinvchi2_from(D.df_va + 1.0, scale, x.gam);
+        return;
+    }
+    D.g[o] = x.gt;
+    D.cls[o] = x.flag;
+}
+
+// Whether chain c's chunk of cnt SNPs goes through k_skipped_spec (residual in shared memory, few SNPs in the model).
+__device__ __forceinline__ bool skipped_speculates(const Dev &D, int c, int cnt)
+{
+    return D.method != SODAGPU_BAYES_A && 4 * D.ssdense[c] <= cnt;
+}
+
+// NT threads: 128 with the residual in shared memory, 512 (for the loads in flight) with it in global memory.
+template <int NT>
+__device__ __forceinline__ void skipped_body(const Dev &D, const VB &vb, int t0, int cnt)
+{
+    constexpr bool SMEM = NT == 128;
+    constexpr int NW = NT / 32, AHEAD = 8;   // words of codes a thread loads ahead (four individuals each)
+    extern __shared__ __align__(16) double s_r[];
+    __shared__ double s_part[NW];
     __shared__ double s_upd;
     const int c = vb.x, rep = cur_rep(D);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    ChainScal *S = &D.scal[c];
-    double *rg = D.r + (size_t)c * D.ldr;
-    const bool in_smem = (size_t)D.n * sizeof(double) <= (size_t)SS_SMEM_MAX;
-    double *r = in_smem ? s_r : rg;
-    if (in_smem) {
-        for (int i = tid; i < D.n; i += SS_THREADS) s_r[i] = rg[i];
-        __syncthreads();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nm = D.nmix;
+    if (SMEM && skipped_speculates(D, c, cnt)) return;
+    const ChainScal *S = &D.scal[c];
+    double *rg = D.r + (size_t)c * D.ldr, *r = SMEM ? s_r : rg;
+    // four consecutive individuals a word; rows n .. ldr-1 of the residual are zero, and stay so
+    const int words = (D.n + 3) / 4;
+    if (SMEM) {
+        for (int i = tid; i < 4 * words; i += NT) s_r[i] = rg[i];
     }
-    for (int t = 0; t < D.nskipped; ++t) {
-        const int snploc = D.iskipped[t];
-        const int k = D.pos_of[snploc];
-        const int8_t *col = D.G + (size_t)k * D.ldx;
-        const double *xv = D.xv + (size_t)k * 4;
-        const double x0 = xv[0], x1 = xv[1], x2 = xv[2];
-        double part = 0.0;
-        for (int i = tid; i < D.n; i += SS_THREADS) {
-            const int g = col[i];
-            part += r[i] * (g == 0 ? x0 : (g == 1 ? x1 : x2));
+    const int stride = SS_HEAD + 2 * nm;
+    const double *rec = D.ssrec + (size_t)c * min(D.nskipped, SS_CHUNK) * stride;
+    // what a SNP needs besides the residual, loaded while the SNP before it is drawn
+    struct Next {
+        uint32_t code[AHEAD];
+        const uint32_t *col;
+        double x0, x1, x2, gk, zz, u;
+        double2 cb;
+        int snp, cl;
+    };
+    // (the SNP's id and position come in one and two turns before that: no load waits for another's address)
+    auto fetch = [&](int t, int snp, int k, Next &x) {
+        if (t >= cnt) return;
+        x.snp = snp;
+        x.col = reinterpret_cast<const uint32_t *>(D.G + (size_t)k * D.ldx);
+#pragma unroll
+        for (int w = 0; w < AHEAD; ++w) x.code[w] = tid + w * NT < words ? __ldg(x.col + tid + w * NT) : 0u;
+        const double2 xa = *reinterpret_cast<const double2 *>(D.xv + (size_t)k * 4);
+        x.x0 = xa.x;
+        x.x1 = xa.y;
+        x.x2 = D.xv[(size_t)k * 4 + 2];
+        if (warp == 0) {
+            const size_t o = (size_t)c * D.p + x.snp;
+            x.gk = D.g[o];
+            x.cl = D.cls[o];
+            x.zz = D.xpx[x.snp];
+            x.u = rec[(size_t)t * stride + SS_U];
+            x.cb = lane < nm ? make_double2(rec[(size_t)t * stride + SS_HEAD + 2 * lane],
+                                            rec[(size_t)t * stride + SS_HEAD + 2 * lane + 1])
+                             : make_double2(0.0, 0.0);
         }
-        part = warp_sum(part);
-        if (lane == 0) s_part[warp] = part;
+    };
+    Next cur, nxt;
+    auto snp_at = [&](int t) { return D.iskipped[t0 + min(t, cnt - 1)]; };
+    int snp1 = snp_at(1), pos1 = D.pos_of[snp1], snp2 = snp_at(2);
+    fetch(0, snp_at(0), D.pos_of[snp_at(0)], cur);
+    if (SMEM) __syncthreads();
+    for (int t = 0; t < cnt; ++t) {
+        fetch(t + 1, snp1, pos1, nxt);
+        const int pos2 = D.pos_of[snp2], snp3 = snp_at(t + 3);
+        auto pick = [&](uint32_t g) { return g == 0u ? cur.x0 : (g == 1u ? cur.x1 : cur.x2); };
+        double p0 = 0.0;
+        auto dot4 = [&](int i, uint32_t cw) {
+            const double2 a = *reinterpret_cast<const double2 *>(r + i), b = *reinterpret_cast<const double2 *>(r + i + 2);
+            p0 = fma(a.x, pick(cw & 3u), p0);
+            p0 = fma(a.y, pick(cw >> 8 & 3u), p0);
+            p0 = fma(b.x, pick(cw >> 16 & 3u), p0);
+            p0 = fma(b.y, pick(cw >> 24 & 3u), p0);
+        };
+#pragma unroll
+        for (int w = 0; w < AHEAD; ++w)
+            if (tid + w * NT < words) dot4(4 * (tid + w * NT), cur.code[w]);
+#pragma unroll 4
+        for (int w = AHEAD; tid + w * NT < words; ++w) dot4(4 * (tid + w * NT), __ldg(cur.col + tid + w * NT));
+        p0 = warp_sum(p0);
+        if (lane == 0) s_part[warp] = p0;
         __syncthreads();
         if (warp == 0) {
-            double d = lane < SS_THREADS / 32 ? s_part[lane] : 0.0;
-            d = warp_sum(d);
-            const double upd = single_site_draw(D, S, c, rep, snploc, d);
-            if (lane == 0) s_upd = upd;
+            double d;
+            if (NW == 4) {
+                d = (s_part[0] + s_part[1]) + (s_part[2] + s_part[3]);
+            } else {
+                d = warp_sum(lane < NW ? s_part[lane] : 0.0);
+            }
+            const SkippedDraw x = skipped_draw(D, S, c, rep, cur.snp, d, cur.gk, cur.cl, cur.zz, cur.cb,
+                                               rec + (size_t)t * stride, cur.u);
+            if (lane == 0) {
+                s_upd = x.upd;
+                skipped_commit(D, S, c, cur.snp, x);
+            }
         }
         __syncthreads();
         const double upd = s_upd;
         if (upd != 0.0) {
-            for (int i = tid; i < D.n; i += SS_THREADS) {
-                const int g = col[i];
-                r[i] = r[i] + (g == 0 ? x0 : (g == 1 ? x1 : x2)) * upd;
-            }
+            auto add4 = [&](int i, uint32_t cw) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (i + e < D.n) r[i + e] = fma(pick(cw >> (8 * e) & 3u), upd, r[i + e]);
+            };
+#pragma unroll
+            for (int w = 0; w < AHEAD; ++w)
+                if (tid + w * NT < words) add4(4 * (tid + w * NT), cur.code[w]);
+            for (int w = AHEAD; tid + w * NT < words; ++w) add4(4 * (tid + w * NT), __ldg(cur.col + tid + w * NT));
         }
+        cur = nxt;
+        snp1 = snp2;
+        pos1 = pos2;
+        snp2 = snp3;
     }
-    if (in_smem) {
+    if (SMEM) {
         __syncthreads();
-        for (int i = tid; i < D.n; i += SS_THREADS) rg[i] = s_r[i];
+        for (int i = tid; i < D.n; i += NT) rg[i] = s_r[i];
     }
 }
 
-__global__ void __launch_bounds__(SS_THREADS) k_skipped(Dev D)
+// Rounds of SS_SPEC SNPs, a warp each, over a cluster of SS_CTAS CTAs that all hold the residual; the warps exchange
+// their updates through distributed shared memory.  Bound by a warp's FP64 pipe: n / 32 multiply-adds of 64 cycles a
+// round, and the draw's exponential.
+__device__ __forceinline__ void skipped_spec_body(const Dev &D, int c, int t0, int cnt)
 {
-    skipped_body(D, vb_native());
+    namespace cg = cooperative_groups;
+    constexpr int NT = 128, AHEAD = 8;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) double s_r[];
+    __shared__ double s_upd[2][4];            // this CTA's warps' updates, by the round's parity
+    if (!skipped_speculates(D, c, cnt)) return;   // the same for the whole cluster
+    const int rep = cur_rep(D), rank = (int)cl.block_rank();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nm = D.nmix, mine = 4 * rank + warp;
+    const ChainScal *S = &D.scal[c];
+    double *rg = D.r + (size_t)c * D.ldr;
+    const int words = (D.n + 3) / 4, stride = SS_HEAD + 2 * nm;
+    for (int i = tid; i < 4 * words; i += NT) s_r[i] = rg[i];
+    const double *rec = D.ssrec + (size_t)c * min(D.nskipped, SS_CHUNK) * stride;
+    __syncthreads();
+    int par = 0;
+    for (int t = 0; t < cnt; par ^= 1) {
+        const bool in = t + mine < cnt;
+        SkippedDraw x;
+        x.upd = 0.0;
+        int snp = 0;
+        if (in) {
+            const double *q = rec + (size_t)(t + mine) * stride;
+            snp = (int)q[SS_SNP];
+            const int k = (int)q[SS_POS];
+            const double u = q[SS_U];
+            const double2 cb = lane < nm ? make_double2(q[SS_HEAD + 2 * lane], q[SS_HEAD + 2 * lane + 1])
+                                         : make_double2(0.0, 0.0);
+            const uint32_t *col = reinterpret_cast<const uint32_t *>(D.G + (size_t)k * D.ldx);
+            const double x0 = D.xv[(size_t)k * 4], x1 = D.xv[(size_t)k * 4 + 1], x2 = D.xv[(size_t)k * 4 + 2];
+            const size_t o = (size_t)c * D.p + snp;
+            const double gk = D.g[o], zz = D.xpx[snp];
+            const int cls = D.cls[o];
+            double p0 = 0.0;
+            for (int w0 = lane; w0 < words; w0 += 32 * AHEAD) {
+                uint32_t cw[AHEAD];
+#pragma unroll
+                for (int v = 0; v < AHEAD; ++v) cw[v] = w0 + 32 * v < words ? __ldg(col + w0 + 32 * v) : 0u;
+#pragma unroll
+                for (int v = 0; v < AHEAD; ++v) {
+                    const int i = 4 * (w0 + 32 * v);
+                    if (w0 + 32 * v >= words) break;
+                    const double2 a = *reinterpret_cast<const double2 *>(s_r + i);
+                    const double2 b = *reinterpret_cast<const double2 *>(s_r + i + 2);
+                    auto pick = [&](uint32_t g) { return g == 0u ? x0 : (g == 1u ? x1 : x2); };
+                    p0 = fma(a.x, pick(cw[v] & 3u), p0);
+                    p0 = fma(a.y, pick(cw[v] >> 8 & 3u), p0);
+                    p0 = fma(b.x, pick(cw[v] >> 16 & 3u), p0);
+                    p0 = fma(b.y, pick(cw[v] >> 24 & 3u), p0);
+                }
+            }
+            x = skipped_draw(D, S, c, rep, snp, warp_sum(p0), gk, cls, zz, cb, q, u);
+        }
+        if (lane == 0) s_upd[par][warp] = in ? x.upd : 0.0;
+        cl.sync();
+        // every warp looks at all updates: SNP t + l's lies in CTA l / 4.  (The other parity's slots are written only
+        // after the next barrier.)
+        const double ul = cl.map_shared_rank(&s_upd[par][0], lane >> 2)[lane & 3];
+        const unsigned hit = __ballot_sync(0xffffffffu, ul != 0.0);
+        const int f = hit ? __ffs(hit) - 1 : SS_SPEC - 1;   // the last SNP of the round whose draw stands
+        if (in && mine <= f && lane == 0) skipped_commit(D, S, c, snp, x);
+        if (hit) {
+            const double upd = __shfl_sync(0xffffffffu, ul, f);
+            const int k = (int)rec[(size_t)(t + f) * stride + SS_POS];
+            const uint32_t *col = reinterpret_cast<const uint32_t *>(D.G + (size_t)k * D.ldx);
+            const double x0 = D.xv[(size_t)k * 4], x1 = D.xv[(size_t)k * 4 + 1], x2 = D.xv[(size_t)k * 4 + 2];
+            __syncthreads();   // every warp has read the residual of this round
+            for (int w = tid; w < words; w += NT) {
+                const uint32_t cw = __ldg(col + w);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint32_t g = cw >> (8 * e) & 3u;
+                    if (4 * w + e < D.n) s_r[4 * w + e] = fma(g == 0u ? x0 : (g == 1u ? x1 : x2), upd, s_r[4 * w + e]);
+                }
+            }
+            __syncthreads();
+        }
+        t += f + 1;
+    }
+    if (rank == 0)
+        for (int i = tid; i < D.n; i += NT) rg[i] = s_r[i];
+    cl.sync();   // no CTA leaves while another still reads its shared memory
+}
+
+__global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(128) k_skipped_spec(Dev D, int t0, int cnt)
+{
+    skipped_spec_body(D, blockIdx.x / SS_CTAS, t0, cnt);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT) k_skipped(Dev D, int t0, int cnt)
+{
+    skipped_body<NT>(D, vb_native(), t0, cnt);
+}
+
+// Shared memory of k_skipped<128>, 0 when the residual does not fit (then k_skipped<512> runs).
+static size_t skipped_smem(int n)
+{
+    const size_t b = sizeof(double) * 4 * (size_t)((n + 3) / 4);
+    return b <= (size_t)SS_SMEM_MAX ? b : 0;
 }
 
 
@@ -1234,8 +1474,14 @@ static cudaError_t carve_all()
     if (e == cudaSuccess) e = max_carveout(k_iter_begin);
     if (e == cudaSuccess) e = max_carveout(k_mu_partial);
     if (e == cudaSuccess) e = max_carveout(k_mu_apply);
-    if (e == cudaSuccess) e = max_carveout(k_skipped);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_skipped, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX);
+    if (e == cudaSuccess) e = max_carveout(k_skipped_pre);
+    if (e == cudaSuccess) e = max_carveout(k_skipped_spec);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_skipped_spec, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX);
+    if (e == cudaSuccess) e = max_carveout(k_skipped<128>);
+    if (e == cudaSuccess) e = max_carveout(k_skipped<512>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_skipped<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX);
     if (e == cudaSuccess) e = max_carveout(k_stats);
     if (e == cudaSuccess) e = max_carveout(k_hyper);
     if (e == cudaSuccess) e = max_carveout(k_post);
@@ -1538,9 +1784,18 @@ cudaError_t sweep_enqueue_iteration(const Dev &D, const int *blk_sizes, int sm_c
     }
     {
         ProfScope ps(prof, st, PROF_OTHER);
-        if (D.nskipped > 0) {
-            const size_t sm = (size_t)D.n * sizeof(double) <= (size_t)SS_SMEM_MAX ? (size_t)D.n * sizeof(double) : 0;
-            k_skipped<<<C, SS_THREADS, sm, st>>>(D);
+        for (int t0 = 0; t0 < D.nskipped; t0 += SS_CHUNK) {
+            const int cnt = std::min(SS_CHUNK, D.nskipped - t0);
+            const size_t sm = skipped_smem(D.n);
+            e = cudaMemsetAsync(D.ssdense, 0, sizeof(int32_t) * C, st);
+            if (e != cudaSuccess) return e;
+            k_skipped_pre<<<dim3((cnt + 63) / 64, C), 64, 0, st>>>(D, t0, cnt);
+            if (sm) {   // each chain goes through one of the two
+                k_skipped_spec<<<SS_CTAS * C, 128, sm, st>>>(D, t0, cnt);
+                k_skipped<128><<<C, 128, sm, st>>>(D, t0, cnt);
+            } else {
+                k_skipped<512><<<C, 512, 0, st>>>(D, t0, cnt);
+            }
         }
         e = launch_pdl(k_stats, dim3(NSTAT + mu_grid(D.n), C), dim3(256), 0, st, D);
         if (e == cudaSuccess) e = launch_pdl(k_hyper, dim3(C), dim3(HYPER_THREADS), 0, st, D);
@@ -1763,11 +2018,34 @@ __global__ void __launch_bounds__(MU_THREADS) k_mu_apply_m(const __grid_constant
     mu_apply_body(G.dev[j], vb);
 }
 
-__global__ void __launch_bounds__(SS_THREADS) k_skipped_m(const __grid_constant__ JobGrid G)
+__global__ void __launch_bounds__(64) k_skipped_pre_m(const __grid_constant__ JobGrid G)
 {
     VB vb;
     const int j = jg_locate(G, vb);
-    skipped_body(G.dev[j], vb);
+    skipped_pre_body(G.dev[j], vb, G.arg[j][0], G.arg[j][1]);
+}
+
+// One dense-count entry per chain; every job's before k_skipped_pre_m.
+__global__ void k_skipped_clear_m(const Dev *dev, int njobs)
+{
+    const int j = blockIdx.x;
+    if (j < njobs && dev[j].ssdense && (int)threadIdx.x < dev[j].chains) dev[j].ssdense[threadIdx.x] = 0;
+}
+
+// (the jobs' grids are multiples of a cluster)
+__global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(128) k_skipped_spec_m(const __grid_constant__ JobGrid G)
+{
+    VB vb;
+    const int j = jg_locate(G, vb);
+    skipped_spec_body(G.dev[j], vb.x / SS_CTAS, G.arg[j][0], G.arg[j][1]);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT) k_skipped_m(const __grid_constant__ JobGrid G)
+{
+    VB vb;
+    const int j = jg_locate(G, vb);
+    skipped_body<NT>(G.dev[j], vb, G.arg[j][0], G.arg[j][1]);
 }
 
 __global__ void __launch_bounds__(256) k_stats_m(const __grid_constant__ JobGrid G)
@@ -1929,7 +2207,10 @@ static cudaError_t multi_attrs_mode(int chains, int max_bs)
 cudaError_t sweep_multi_prepare(int precision, int chains, int max_bs)
 {
     cudaError_t e = sweep_prepare(max_bs);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_skipped_m, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_skipped_m<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_skipped_spec_m, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_SMEM_MAX);
     if (e != cudaSuccess) return e;
     if (precision == SODAGPU_FP64) return multi_attrs_mode<SODAGPU_FP64>(chains, max_bs);
     if (precision == SODAGPU_FP32) return multi_attrs_mode<SODAGPU_FP32>(chains, max_bs);
@@ -1989,22 +2270,39 @@ cudaError_t sweep_enqueue_iteration_multi(const BatchPlan &P, int sm_count, cuda
                                    : multi_step_mode<SODAGPU_FP8>(P, t, st);
         if (e != cudaSuccess) return e;
     }
-    GridBuilder skp(P.ddev, nj), stats(P.ddev, nj), hyp(P.ddev, nj), post(P.ddev, nj), rp(P.ddev, nj),
+    GridBuilder stats(P.ddev, nj), hyp(P.ddev, nj), post(P.ddev, nj), rp(P.ddev, nj),
         ra(P.ddev, nj);
-    size_t ssm = 0;
+    int nskip = 0;
     for (int j = 0; j < nj; ++j) {
         const Dev &D = P.hdev[j];
         const int C = D.chains;
-        skp.set(j, D.nskipped > 0 ? C : 0, 1, 1);
-        if (D.nskipped > 0 && (size_t)D.n * sizeof(double) <= (size_t)SS_SMEM_MAX)
-            ssm = std::max(ssm, (size_t)D.n * sizeof(double));
+        nskip = std::max(nskip, D.nskipped);
         stats.set(j, NSTAT + mu_grid(D.n), C, 1);
         hyp.set(j, C, 1, 1);
         post.set(j, post_grid(D, sm_count), C, 1);
         rp.set(j, recal_grid(D, RECAL_SPLIT), 1, 1);
         ra.set(j, recal_grid(D, 1), 1, 1);
     }
-    if (skp.total() > 0) k_skipped_m<<<skp.total(), SS_THREADS, ssm, st>>>(skp.g);
+    for (int t0 = 0; t0 < nskip; t0 += SS_CHUNK) {
+        // by where the residual is held; a small one's chains each go through one of two kernels
+        GridBuilder pre(P.ddev, nj), spec(P.ddev, nj), small(P.ddev, nj), large(P.ddev, nj);
+        size_t ssm = 0;
+        for (int j = 0; j < nj; ++j) {
+            const Dev &D = P.hdev[j];
+            const int cnt = std::max(0, std::min(SS_CHUNK, D.nskipped - t0));
+            const size_t sm = skipped_smem(D.n);
+            pre.set(j, (cnt + 63) / 64, D.chains, 1, t0, cnt);
+            spec.set(j, cnt > 0 && sm ? SS_CTAS * D.chains : 0, 1, 1, t0, cnt);
+            small.set(j, cnt > 0 && sm ? D.chains : 0, 1, 1, t0, cnt);
+            large.set(j, cnt > 0 && !sm ? D.chains : 0, 1, 1, t0, cnt);
+            if (cnt > 0) ssm = std::max(ssm, sm);
+        }
+        k_skipped_clear_m<<<nj, 32, 0, st>>>(P.ddev, nj);
+        k_skipped_pre_m<<<pre.total(), 64, 0, st>>>(pre.g);
+        if (spec.total() > 0) k_skipped_spec_m<<<spec.total(), 128, ssm, st>>>(spec.g);
+        if (small.total() > 0) k_skipped_m<128><<<small.total(), 128, ssm, st>>>(small.g);
+        if (large.total() > 0) k_skipped_m<512><<<large.total(), 512, 0, st>>>(large.g);
+    }
     e = launch_pdl(k_stats_m, dim3(stats.total()), dim3(256), 0, st, stats.g);
     if (e == cudaSuccess) e = launch_pdl(k_hyper_m, dim3(hyp.total()), dim3(HYPER_THREADS), 0, st, hyp.g);
     if (e == cudaSuccess) e = launch_pdl(k_post_m, dim3(post.total()), dim3(256), 0, st, post.g);

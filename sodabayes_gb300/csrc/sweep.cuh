@@ -49,6 +49,8 @@ constexpr int TC_PACKED_BLOCK = 4 * 128 * 16;   // bytes of one packed code bloc
 int sweep_tc_code_blocks(const int *blk_sizes, int nb, int32_t *qoff);
 cudaError_t sweep_tc_tile_codes(const int8_t *G, const Dev &D, uint8_t *Gt, uint8_t *Gu, long long nblocks,
                                 int sm_count, cudaStream_t st);
+// Doubles of the single-site draws' records (Dev::ssrec).
+size_t sweep_skip_records(int nskipped, int chains, int nmix);
 // Optional per-launch event recording (eager profiling, never inside a graph):
 // before/after every launch an event pair is recorded and its kernel class
 // stored.  Classes: 0 rhs, 1 residual update, 2 mu, 3 everything else, 4 draws.

@@ -47,7 +47,7 @@ enum sodagpu_method {
 
 /* Arithmetic of the per-iteration sweep.  The Z build is FP64 in every mode.
  *   FP64: genotypes as centred/scaled FP64 columns, U in FP64 — the parity mode.
- *   FP32: genotypes as centred/scaled FP32 columns, U in FP32 — the plain path.
+ *   FP32: genotypes as centred/scaled FP32 values, U in FP32 — the plain path.
  *   FP8 : genotypes as exact 8-bit 0/1/2 codes with the centring applied as an
  *         FP32 rank-1 correction, U as BF16 hi+lo pairs.                      */
 enum sodagpu_precision { SODAGPU_FP64 = 0, SODAGPU_FP32 = 1, SODAGPU_FP8 = 2 };

@@ -128,7 +128,6 @@ struct sodagpu_ctx {
     std::vector<int32_t> blk_sizes, h_blk_ls;
     // device
     int8_t *Gsnp = nullptr, *G = nullptr;
-    float *X32 = nullptr;
     double *xv = nullptr, *freq = nullptr, *y = nullptr;
     int64_t *uoff = nullptr;
     int32_t *ulen = nullptr;
@@ -544,10 +543,6 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     CUDA_TRY(cudaStreamSynchronize(c->st));
     c->release(c->Gsnp);
     c->Gsnp = nullptr;
-    if (c->cfg.precision == SODAGPU_FP32) {
-        TRY(c->alloc(&c->X32, (size_t)p * c->ldx, false));
-        CUDA_TRY(zb_x32(c->G, c->xv, c->X32, n, p, c->ldx, c->st));
-    }
     // FP64 work matrices of every subset
     std::vector<int64_t> wofs(nb);
     int64_t wtot = 0;
@@ -836,7 +831,6 @@ int build_dev(sodagpu_ctx *c)
         D.alpha[j] = c->cfg.alpha[j];
     }
     D.G = c->G;
-    D.X32 = c->X32;
     D.xv = c->xv;
     D.xv32 = c->xv32;
     D.delta32 = c->delta32;

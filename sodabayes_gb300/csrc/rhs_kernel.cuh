@@ -6,15 +6,26 @@
 //
 // is a tall-skinny GEMM: M = the subset's SNPs, N = chains, K = individuals
 // followed by the augmented rows.  The grid is (M tiles of 8*SPT SNPs) x
-// (K splits), sized to one wave.  Each CTA streams its share of both K
-// ranges through shared memory in one NS-stage cp.async pipeline — genotype
-// stages (codes or FP32 columns with r) first, then augmenting-matrix stages
-// (U columns with ra; the factor is upper triangular, so a tile needs only
-// the rows up to its last column) — keeping an SPT x CT accumulator block per
-// thread.  Partial sums go to scratch (one slice per K split), which k_draw
-// adds in split order before the draws.  FP8 mode: codes 0/1/2 are exact in
-// FP32 and the centring is applied once per SNP, x'r = (G'r)/sd - 2p/sd *
-// sum(r).
+// (K splits), about one wave.  Each CTA streams its share of both K ranges
+// through shared memory in one NS-stage cp.async pipeline - genotype stages
+// (codes with r) first, then augmenting-matrix stages (U columns with ra; the
+// factor is upper triangular, so a tile needs only the rows up to its last
+// column) - keeping an SPT x CT accumulator block per thread.  Codes and U do
+// not change during the sweep: the first stages' are loaded before the
+// dependency wait, while the previous residual update runs.  Partial sums go to
+// scratch (one slice per K split), which k_draw adds in split order before the
+// draws.  Codes become the column's exact x values (FP64, FP32) or stay 0/1/2,
+// exact in FP32, with the centring applied once per SNP (FP8), x'r = (G'r)/sd -
+// 2p/sd * sum(r).
+//
+// For one chain these kernels are latency, not bandwidth: a subset of 1000 SNPs x
+// 5,000 individuals is 5 MB of codes.  Two CTAs share an SM, FP64 stages are of 256
+// individuals so that every SM has a share, and a warp's sums are reduced eight at a time (nine exchanges in
+// place of forty; in FP64 the forty took longer than the products).  Measured by
+// itself, its loads not early: FP64, N = 935, n = 2,326: 15.5 us (26.7 with stages
+// of 512 and two reductions); an FP32 iteration of 50 subsets of N = 1000, n =
+// 5,000: 0.90 ms (1.21 with FP32 columns of four times the bytes, one CTA an SM and
+// no early loads); a step of eight FP8 analyses: 31.5 us (36.5).
 #pragma once
 #include <cuda_pipeline_primitives.h>
 
@@ -25,21 +36,18 @@ struct RhsCfg;
 template <>
 struct RhsCfg<SODAGPU_FP8> {       // int8 codes, FP32 residual, FP32 U
     static constexpr int KST = 512;            // genotype elements per row per stage
-    static constexpr int XB = 1;               // bytes per genotype element
     static constexpr int RB = 4;               // bytes per residual element
     static constexpr int UB = 4;               // bytes per U / ra element
 };
 template <>
-struct RhsCfg<SODAGPU_FP32> {      // FP32 columns, FP32 residual, FP32 U
-    static constexpr int KST = 256;
-    static constexpr int XB = 4;
+struct RhsCfg<SODAGPU_FP32> {      // int8 codes looked up as FP32, FP32 residual, FP32 U
+    static constexpr int KST = 512;
     static constexpr int RB = 4;
     static constexpr int UB = 4;
 };
 template <>
 struct RhsCfg<SODAGPU_FP64> {      // int8 codes looked up as FP64, FP64 residual and U
-    static constexpr int KST = 512;
-    static constexpr int XB = 1;
+    static constexpr int KST = 256;
     static constexpr int RB = 8;
     static constexpr int UB = 8;
 };
@@ -48,10 +56,10 @@ template <int CT>
 struct SptOf { static constexpr int v = CT >= 8 ? 4 : 8; };
 
 template <int MODE>
-constexpr int rhs_ku() { return RhsCfg<MODE>::KST * RhsCfg<MODE>::XB / RhsCfg<MODE>::UB; }   // U rows per stage
+constexpr int rhs_ku() { return RhsCfg<MODE>::KST / RhsCfg<MODE>::UB; }   // U rows per stage
 
 template <int MODE, int CT>
-constexpr size_t rhs_xpart_bytes() { return (size_t)8 * SptOf<CT>::v * RhsCfg<MODE>::KST * RhsCfg<MODE>::XB; }
+constexpr size_t rhs_xpart_bytes() { return (size_t)8 * SptOf<CT>::v * RhsCfg<MODE>::KST; }
 template <int MODE, int CT>
 constexpr size_t rhs_rpart_bytes()
 {
@@ -61,13 +69,24 @@ constexpr size_t rhs_rpart_bytes()
 }
 template <int MODE, int CT>
 constexpr size_t rhs_stage_bytes() { return rhs_xpart_bytes<MODE, CT>() + rhs_rpart_bytes<MODE, CT>(); }
+// Stages in flight: for one or two chains three, so that two CTAs share an SM (one's products run while the other waits
+// for its stage; the accumulators of more chains do not fit half of the registers), else as many as fit up to four.
 template <int MODE, int CT>
 constexpr int rhs_nstage()
 {
-    return 4 * rhs_stage_bytes<MODE, CT>() <= 200 * 1024 ? 4 : (3 * rhs_stage_bytes<MODE, CT>() <= 200 * 1024 ? 3 : 2);
+    return CT <= 2                                         ? 3
+           : 4 * rhs_stage_bytes<MODE, CT>() <= 200 * 1024 ? 4
+           : 3 * rhs_stage_bytes<MODE, CT>() <= 200 * 1024 ? 3
+                                                           : 2;
 }
 template <int MODE, int CT>
 constexpr size_t rhs_smem_bytes() { return rhs_nstage<MODE, CT>() * rhs_stage_bytes<MODE, CT>(); }
+template <int MODE, int CT>
+constexpr int rhs_per_sm()
+{
+    static_assert(CT > 2 || rhs_smem_bytes<MODE, CT>() <= 110 * 1024, "two CTAs an SM");
+    return CT <= 2 ? 2 : 1;
+}
 
 __device__ __forceinline__ float code_to_f32(uint32_t w, int k)
 {
@@ -206,14 +225,14 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
             if (act && sp < ksplit) {
                 const size_t o = ((size_t)sp * CT + c) * D.bs + jl;
                 px[sp] = __ldcg(D.rpx + o);
-                pu[sp] = __ldcg(D.rpu + o);
+                if (MODE == SODAGPU_FP8) pu[sp] = __ldcg(D.rpu + o);   // the other modes add both into one sum
             }
         }
 #pragma unroll
         for (int sp = 0; sp < RHS_KSPLIT_MAX; ++sp) {
             if (sp < ksplit) {
                 xr += px[sp];
-                ur += pu[sp];
+                if (MODE == SODAGPU_FP8) ur += pu[sp];
             }
         }
     }
@@ -294,10 +313,6 @@ __device__ __forceinline__ void rhs_body(const Dev &D, const VB &vb, int b, int 
     extern __shared__ __align__(16) unsigned char smem[];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // the draw kernel launches only after this wait (its prologue reads what the previous
-    // residual update wrote)
-    tc::pdl_wait();
-    tc::pdl_trigger();
     const int ls = D.blk_ls[b];
     const int N = D.blk_ls[b + 1] - ls;
     const int mt = vb.x / ksplit, ks = vb.x % ksplit;
@@ -312,127 +327,126 @@ __device__ __forceinline__ void rhs_body(const Dev &D, const VB &vb, int b, int 
     const int u0 = (int)(((long long)nU * ks) / ksplit), u1 = (int)(((long long)nU * (ks + 1)) / ksplit);
     const int ng = g1 - g0, nv = ng + (u1 - u0);
 
-    auto issue = [&](int v, int buf) {
+    // a stage's codes or U columns (constant during the sweep), and its residuals
+    auto issue_x = [&](int v, int buf) {
         unsigned char *dx = smem + (size_t)buf * SBYTES;
-        unsigned char *dr = dx + XPART;
-        if (v < ng) {     // genotype stage
-            const int k0 = (g0 + v) * KST;
-            constexpr int XCH = KST * Cfg::XB / 16;
-            for (int t = tid; t < MTS * XCH; t += 256) {
-                const int row = t / XCH, ch = t % XCH;
-                unsigned char *dst = dx + (size_t)row * KST * Cfg::XB + ch * 16;
-                const int jk = j0 + row;
-                const int e0 = k0 + ch * (16 / Cfg::XB);
-                if (jk < N && e0 + 16 / Cfg::XB <= D.ldx) {
-                    const void *src = MODE == SODAGPU_FP32
-                                          ? (const void *)(D.X32 + (size_t)(ls + jk) * D.ldx + e0)
-                                          : (const void *)(D.G + (size_t)(ls + jk) * D.ldx + e0);
-                    __pipeline_memcpy_async(dst, src, 16);
-                } else {
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-                }
-            }
-            constexpr int RCH = KST * Cfg::RB / 16;
-            for (int t = tid; t < CT * RCH; t += 256) {
-                const int c = t / RCH, ch = t % RCH;
-                unsigned char *dst = dr + (size_t)c * KST * Cfg::RB + ch * 16;
-                const int e0 = k0 + ch * (16 / Cfg::RB);
-                if (e0 + 16 / Cfg::RB <= D.ldr) {
-                    const void *src = MODE == SODAGPU_FP64 ? (const void *)(D.r + (size_t)c * D.ldr + e0)
-                                                           : (const void *)(D.r32 + (size_t)c * D.ldr + e0);
-                    __pipeline_memcpy_async(dst, src, 16);
-                } else {
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-                }
-            }
-        } else {          // augmenting-matrix stage: rows [i0, i0+KU) of the tile's U columns
-            const int i0 = (u0 + v - ng) * KU;
-            constexpr int UCH = KU * Cfg::UB / 16;
-            for (int t = tid; t < MTS * UCH; t += 256) {
-                const int row = t / UCH, ch = t % UCH;
-                unsigned char *dst = dx + (size_t)row * KU * Cfg::UB + ch * 16;
-                const int jk = j0 + row;
-                const int e0 = i0 + ch * (16 / Cfg::UB);
+        constexpr int XCH = KST / 16;
+        for (int t = tid; t < MTS * XCH; t += 256) {
+            const int row = t / XCH, ch = t % XCH;
+            unsigned char *dst = dx + (size_t)row * KST + ch * 16;
+            const int jk = j0 + row;
+            const void *src = nullptr;
+            if (v < ng) {
+                const int e0 = (g0 + v) * KST + ch * 16;
+                if (jk < N && e0 + 16 <= D.ldx) src = D.G + (size_t)(ls + jk) * D.ldx + e0;
+            } else {     // rows [i0, i0+KU) of the tile's U columns
+                const int e0 = (u0 + v - ng) * KU + ch * (16 / Cfg::UB);
                 if (jk < N && e0 + 16 / Cfg::UB <= npad) {
                     const int64_t off = D.uoff[ls + jk] + e0;
-                    const void *src = MODE == SODAGPU_FP64 ? (const void *)(D.U64 + off) : (const void *)(D.U32 + off);
-                    __pipeline_memcpy_async(dst, src, 16);
-                } else {
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
+                    src = MODE == SODAGPU_FP64 ? (const void *)(D.U64 + off) : (const void *)(D.U32 + off);
                 }
             }
-            constexpr int RCH = KU * Cfg::UB / 16;
-            for (int t = tid; t < CT * RCH; t += 256) {
-                const int c = t / RCH, ch = t % RCH;
-                unsigned char *dst = dr + (size_t)c * KU * Cfg::UB + ch * 16;
-                const int e0 = i0 + ch * (16 / Cfg::UB);
-                if (e0 + 16 / Cfg::UB <= D.ldra) {
-                    const void *src = MODE == SODAGPU_FP64 ? (const void *)(D.ra + (size_t)c * D.ldra + e0)
-                                                           : (const void *)(D.ra32 + (size_t)c * D.ldra + e0);
-                    __pipeline_memcpy_async(dst, src, 16);
-                } else {
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-                }
+            if (src) __pipeline_memcpy_async(dst, src, 16);
+            else *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
+        }
+    };
+    auto issue_r = [&](int v, int buf) {
+        unsigned char *dr = smem + (size_t)buf * SBYTES + XPART;
+        const int len = v < ng ? KST : KU, lim = v < ng ? D.ldr : D.ldra;
+        const int k0 = v < ng ? (g0 + v) * KST : (u0 + v - ng) * KU;
+        const int rch = len * Cfg::RB / 16;
+        for (int t = tid; t < CT * rch; t += 256) {
+            const int c = t / rch, ch = t - c * rch;
+            unsigned char *dst = dr + (size_t)c * len * Cfg::RB + ch * 16;
+            const int e0 = k0 + ch * (16 / Cfg::RB);
+            if (e0 + 16 / Cfg::RB <= lim) {
+                const size_t o = (size_t)c * lim + e0;
+                const void *src = MODE == SODAGPU_FP64 ? (v < ng ? (const void *)(D.r + o) : (const void *)(D.ra + o))
+                                                       : (v < ng ? (const void *)(D.r32 + o) : (const void *)(D.ra32 + o));
+                __pipeline_memcpy_async(dst, src, 16);
+            } else {
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
             }
         }
         __pipeline_commit();
     };
+    static_assert(Cfg::RB == Cfg::UB, "r and ra have one type");
 
     acc_t acc[SPT][CT];
 #pragma unroll
     for (int s = 0; s < SPT; ++s)
 #pragma unroll
         for (int c = 0; c < CT; ++c) acc[s][c] = 0;
-    double xl[SPT][3];
-    if (MODE == SODAGPU_FP64) {
+    acc_t xl[SPT][3];   // the x values of this warp's SNPs
+    if (MODE != SODAGPU_FP8) {
 #pragma unroll
         for (int s = 0; s < SPT; ++s) {
             const int jk = j0 + warp * SPT + s;
             const int k = ls + (jk < N ? jk : 0);
-            xl[s][0] = D.xv[(size_t)k * 4 + 0];
-            xl[s][1] = D.xv[(size_t)k * 4 + 1];
-            xl[s][2] = D.xv[(size_t)k * 4 + 2];
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                xl[s][q] = MODE == SODAGPU_FP64 ? (acc_t)D.xv[(size_t)k * 4 + q] : (acc_t)D.xv32[(size_t)k * 4 + q];
         }
     }
-    // publishes the accumulators as this split's genotype (is_u = false) or
-    // augmenting (is_u = true) partial sums and clears them
+    // publishes the accumulators as this split's genotype (is_u = false) or augmenting (is_u = true) partial sums and
+    // clears them; the FP64 and FP32 modes add both kinds into one sum.  The SPT sums of a chain are reduced together:
+    // at each exchange a lane keeps half of them, so lane l ends with sum (l >> LOG) of SPT
     auto publish = [&](bool is_u) {
         double *dstp = is_u ? D.rpu : D.rpx;
+        constexpr int LOG = SPT == 8 ? 2 : 3;   // 32 lanes / SPT sums = 2^LOG lanes a sum
+        static_assert(SPT == 8 || SPT == 4, "the reduction halves SPT sums");
 #pragma unroll
-        for (int s = 0; s < SPT; ++s) {
-            const int jk = j0 + warp * SPT + s;
+        for (int c = 0; c < CT; ++c) {
+            acc_t v[SPT];
 #pragma unroll
-            for (int c = 0; c < CT; ++c) {
-                // FP32 modes reduce in FP32; only lane 0 widens (the FP64 pipe is narrow)
-                if (MODE == SODAGPU_FP64) {
-                    const double a = warp_sum((double)acc[s][c]);
-                    if (lane == 0 && jk < N) dstp[((size_t)ks * CT + c) * D.bs + jk] = a;
-                } else {
-                    const float a = warp_sumf((float)acc[s][c]);
-                    if (lane == 0 && jk < N) dstp[((size_t)ks * CT + c) * D.bs + jk] = (double)a;
-                }
+            for (int s = 0; s < SPT; ++s) {
+                v[s] = acc[s][c];
                 acc[s][c] = 0;
             }
+#pragma unroll
+            for (int h = SPT / 2, o = 16; h >= 1; h /= 2, o /= 2) {
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int s = 0; s < h; ++s) {
+                    const acc_t keep = up ? v[s + h] : v[s], give = up ? v[s] : v[s + h];
+                    v[s] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            }
+#pragma unroll
+            for (int o = 1 << (LOG - 1); o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            const int jk = j0 + warp * SPT + (lane >> LOG);
+            // only one lane widens FP32 sums (the FP64 pipe is narrow)
+            if ((lane & ((1 << LOG) - 1)) == 0 && jk < N) dstp[((size_t)ks * CT + c) * D.bs + jk] = (double)v[0];
         }
     };
 
 #pragma unroll
+    for (int pp = 0; pp < NS - 1; ++pp)
+        if (pp < nv) issue_x(pp, pp);
+    // the draw kernel launches only after this wait (its prologue reads what the previous residual update wrote)
+    tc::pdl_wait();
+    tc::pdl_trigger();
+#pragma unroll
     for (int pp = 0; pp < NS - 1; ++pp) {
-        if (pp < nv) issue(pp, pp);
+        if (pp < nv) issue_r(pp, pp);
         else __pipeline_commit();
     }
     for (int v = 0; v < nv; ++v) {
         const int buf = v % NS;
         // the buffer of stage v+NS-1 was last read in iteration v-1, which
         // ended with a barrier: refill it before waiting for stage v
-        if (v + NS - 1 < nv) issue(v + NS - 1, (v + NS - 1) % NS);
-        else __pipeline_commit();
+        if (v + NS - 1 < nv) {
+            issue_x(v + NS - 1, (v + NS - 1) % NS);
+            issue_r(v + NS - 1, (v + NS - 1) % NS);
+        } else {
+            __pipeline_commit();
+        }
         __pipeline_wait_prior(NS - 1);
         __syncthreads();
-        if (v == ng) publish(false);
+        if (MODE == SODAGPU_FP8 && v == ng) publish(false);
         const unsigned char *bx = smem + (size_t)buf * SBYTES;
         const unsigned char *br = bx + XPART;
-        if (v < ng && MODE == SODAGPU_FP8) {
+        if (v < ng && MODE != SODAGPU_FP64) {
             // lane covers individuals q*128 + 4*lane + {0..3}: genotype words
             // and residual float4s are contiguous across lanes
 #pragma unroll
@@ -442,10 +456,15 @@ __device__ __forceinline__ void rhs_body(const Dev &D, const VB &vb, int b, int 
                 for (int s = 0; s < SPT; ++s) {
                     const uint32_t w = *reinterpret_cast<const uint32_t *>(bx + (size_t)(warp * SPT + s) * KST +
                                                                            q * 128 + lane * 4);
-                    x[s][0] = code_to_f32(w, 0);
-                    x[s][1] = code_to_f32(w, 1);
-                    x[s][2] = code_to_f32(w, 2);
-                    x[s][3] = code_to_f32(w, 3);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if constexpr (MODE == SODAGPU_FP32) {
+                            const uint32_t g = w >> (8 * e) & 3u;
+                            x[s][e] = g == 0u ? xl[s][0] : (g == 1u ? xl[s][1] : xl[s][2]);
+                        } else {
+                            x[s][e] = code_to_f32(w, e);
+                        }
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < CT; ++c) {
@@ -460,25 +479,21 @@ __device__ __forceinline__ void rhs_body(const Dev &D, const VB &vb, int b, int 
                 }
             }
         } else if (MODE != SODAGPU_FP64) {
-            // FP32 columns (FP32 mode genotype stages) or FP32 U columns (both modes)
-            constexpr int KF = KST * Cfg::XB / 4;    // floats per row of the stage
-            const int rstride = v < ng ? KST : KU;
+            // FP32 U columns: KU = 128 rows a stage, four a lane
+            static_assert(MODE == SODAGPU_FP64 || KU == 128, "four rows of U a lane");
+            float4 xx[SPT];
 #pragma unroll
-            for (int q = 0; q < KF / 128; ++q) {
-                float4 xx[SPT];
+            for (int s = 0; s < SPT; ++s)
+                xx[s] = *reinterpret_cast<const float4 *>(bx + ((size_t)(warp * SPT + s) * KU + lane * 4) * 4);
 #pragma unroll
-                for (int s = 0; s < SPT; ++s)
-                    xx[s] = *reinterpret_cast<const float4 *>(bx + ((size_t)(warp * SPT + s) * KF + q * 128 + lane * 4) * 4);
+            for (int c = 0; c < CT; ++c) {
+                const float4 rr = *reinterpret_cast<const float4 *>(br + ((size_t)c * KU + lane * 4) * 4);
 #pragma unroll
-                for (int c = 0; c < CT; ++c) {
-                    const float4 rr = *reinterpret_cast<const float4 *>(br + ((size_t)c * rstride + q * 128 + lane * 4) * 4);
-#pragma unroll
-                    for (int s = 0; s < SPT; ++s) {
-                        acc[s][c] = fmaf(xx[s].x, rr.x, acc[s][c]);
-                        acc[s][c] = fmaf(xx[s].y, rr.y, acc[s][c]);
-                        acc[s][c] = fmaf(xx[s].z, rr.z, acc[s][c]);
-                        acc[s][c] = fmaf(xx[s].w, rr.w, acc[s][c]);
-                    }
+                for (int s = 0; s < SPT; ++s) {
+                    acc[s][c] = fmaf(xx[s].x, rr.x, acc[s][c]);
+                    acc[s][c] = fmaf(xx[s].y, rr.y, acc[s][c]);
+                    acc[s][c] = fmaf(xx[s].z, rr.z, acc[s][c]);
+                    acc[s][c] = fmaf(xx[s].w, rr.w, acc[s][c]);
                 }
             }
         } else if (v < ng) {   // FP64 genotype stage: codes looked up in the column's exact x values
@@ -517,13 +532,17 @@ __device__ __forceinline__ void rhs_body(const Dev &D, const VB &vb, int b, int 
         __syncthreads();
     }
     __pipeline_wait_prior(0);
-    if (nv == ng) publish(false);   // no augmenting stage in this split
-    publish(true);
+    if (MODE == SODAGPU_FP8) {
+        if (nv == ng) publish(false);   // no augmenting stage in this split
+        publish(true);
+    } else {
+        publish(false);
+    }
 
 }
 
 template <int MODE, int CT>
-__global__ void __launch_bounds__(256, 1) k_rhs(Dev D, int b, int ksplit)
+__global__ void __launch_bounds__(256, rhs_per_sm<MODE, CT>()) k_rhs(Dev D, int b, int ksplit)
 {
     rhs_body<MODE, CT>(D, vb_native(), b, ksplit);
 }

@@ -3,7 +3,6 @@
 // HBM layout (all arrays 256-byte aligned):
 //   G      int8   [nloci][ldx]   genotype codes 0/1/2, one column per subset
 //                                position k (SNP perm[k]), padded to ldx
-//   X32    float  [nloci][ldx]   centred/scaled columns (FP32 mode only)
 //   xv     double [nloci][4]     the three values (code - 2p)/sqrt(2p(1-p))
 //                                of each column and 1/sqrt(2p(1-p)); all 0
 //                                for monomorphic SNPs
@@ -57,7 +56,7 @@ struct RunCtl {
 struct Dev {
     // sizes
     int n, p, bs, nb, bt, method, nmix, ngroup, chains, precision;
-    int ldx;                   // column stride of G / X32 (elements)
+    int ldx;                   // column stride of G (elements)
     int ldr;                   // chain stride of r / r32
     int nskipped, naind;
     int nr_ctas;               // row tiles (ROW_TILE rows) of the residual kernels
@@ -69,7 +68,6 @@ struct Dev {
     double mix[MAXDIST], alpha[MAXDIST];
     // data (shared by chains)
     const int8_t *G;
-    const float *X32;
     const double *xv;          // [p][4]: x for codes 0,1,2 and 1/sd (0 if monomorphic)
     const float *xv32;         // the same table in FP32 (FP32/FP8 inner loops)
     const double *y;

@@ -1389,6 +1389,15 @@ static cudaError_t launch_block_tc(const Dev &D, int b, int nblk_snps, int sm_co
     return cudaGetLastError();
 }
 
+// K splits of a subset's rhs tiles: `ctas` CTAs in all, but no more than give every split the same number of
+// genotype stages (a split with one stage fewer only waits for the others).
+static int rhs_splits(int ctas, int mtiles, int nst)
+{
+    int ks = std::max(1, std::min({ctas / std::max(1, mtiles), RHS_KSPLIT_MAX, nst}));
+    const int per = (nst + ks - 1) / ks;
+    return (nst + per - 1) / per;
+}
+
 template <int MODE, int CT>
 static cudaError_t launch_block(const Dev &D, int b, int nblk_snps, int sm_count, const TcMaps *maps, cudaStream_t st,
                                ProfHook *prof, bool rhs_only)
@@ -1399,10 +1408,7 @@ static cudaError_t launch_block(const Dev &D, int b, int nblk_snps, int sm_count
     constexpr int MTS = 8 * SptOf<CT>::v;
     const int mtiles = (nblk_snps + MTS - 1) / MTS;
     const int nst = (D.ldx + RhsCfg<MODE>::KST - 1) / RhsCfg<MODE>::KST;
-    // one wave: a CTA per SM (the pipeline fills most of its shared memory)
-    int ks = sm_count / mtiles;
-    ks = ks < 1 ? 1 : (ks > RHS_KSPLIT_MAX ? RHS_KSPLIT_MAX : ks);
-    ks = ks > nst ? nst : ks;
+    const int ks = rhs_splits(sm_count * rhs_per_sm<MODE, CT>(), mtiles, nst);
     cudaError_t e;
     {
         ProfScope ps(prof, st, PROF_RHS);
@@ -2084,7 +2090,7 @@ __global__ void __launch_bounds__(256) k_recal_apply_m(const __grid_constant__ J
 }
 
 template <int MODE, int CT>
-__global__ void __launch_bounds__(256, 1) k_rhs_m(const __grid_constant__ JobGrid G)
+__global__ void __launch_bounds__(256, rhs_per_sm<MODE, CT>()) k_rhs_m(const __grid_constant__ JobGrid G)
 {
     VB vb;
     const int j = jg_locate(G, vb);
@@ -2223,9 +2229,7 @@ static int multi_split(int N, int ldx, int cta_share)
     constexpr int MTS = 8 * SptOf<CT>::v;
     const int mtiles = (N + MTS - 1) / MTS;
     const int nst = (ldx + RhsCfg<MODE>::KST - 1) / RhsCfg<MODE>::KST;
-    int ks = cta_share / std::max(1, mtiles);
-    ks = std::max(1, std::min(ks, RHS_KSPLIT_MAX));
-    return std::min(ks, std::max(1, nst));
+    return rhs_splits(cta_share * rhs_per_sm<MODE, CT>(), mtiles, std::max(1, nst));
 }
 
 template <int MODE>

@@ -97,10 +97,7 @@ __device__ __forceinline__ void update_body(const Dev &D, const VB &vb, int b)
             if (kk[u] < 0 || i0 >= nrow) continue;
             const int k = ls + kk[u];
             if (rows) {
-                if (MODE == SODAGPU_FP32) {
-                    const float4 v = *reinterpret_cast<const float4 *>(D.X32 + (size_t)k * D.ldx + i0);
-                    x[u][0] = v.x; x[u][1] = v.y; x[u][2] = v.z; x[u][3] = v.w;
-                } else {
+                {
                     const uint32_t wv = *reinterpret_cast<const uint32_t *>(D.G + (size_t)k * D.ldx + i0);
                     acc_t x0, x1, x2;
                     if (MODE == SODAGPU_FP64) {
@@ -155,7 +152,8 @@ __device__ __forceinline__ void update_body(const Dev &D, const VB &vb, int b)
                 for (int e = 0; e < 4; ++e) acc[e][c] += x[u][e] * dl[c];
         }
     }
-    // the warps' partial sums, added in warp order
+    // the warps' partial sums, added in warp order (a warp past the list has none)
+    const int nwarp = min(NW, nlist);
 #pragma unroll
     for (int c = 0; c < CT; ++c)
 #pragma unroll
@@ -167,8 +165,8 @@ __device__ __forceinline__ void update_body(const Dev &D, const VB &vb, int b)
         const int i = t0 + rl;
         if (tid < UT && i < nrow) {
             acc_t dsum = 0;   // the warps' partial sums, in warp order
-#pragma unroll
-            for (int ww = 0; ww < NW; ++ww) dsum += s_red[((size_t)ww * CT + c) * UT + rl];
+#pragma unroll 8
+            for (int ww = 0; ww < nwarp; ++ww) dsum += s_red[((size_t)ww * CT + c) * UT + rl];
             const double d = (double)dsum;
             if (rows) {
                 v = D.r[(size_t)c * D.ldr + i] + d;

@@ -113,16 +113,6 @@ __global__ void k_xv(const double *freq, const int32_t *perm, int p, double *xv)
     o[3] = __ddiv_rn(1.0, sd);
 }
 
-__global__ void k_x32(const int8_t *G, const double *xv, float *X32, int n, int p, int ldx)
-{
-    const size_t tot = (size_t)p * ldx;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < tot; t += (size_t)gridDim.x * blockDim.x) {
-        const int k = (int)(t / ldx);
-        const int i = (int)(t % ldx);
-        X32[t] = i < n ? (float)xv[(size_t)k * 4 + G[t]] : 0.0f;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Gram: S = G_b'G_b and the xxproduct scaling, on the tensor cores (gram_tc.cuh);
 // with dp4a on 64x64 tiles for more than GR_NMAX individuals, whose counts
@@ -471,12 +461,6 @@ cudaError_t zb_xv(const double *freq, const int32_t *perm, int p, double *xv, cu
 cudaError_t zb_xv32(const double *xv, int p, float *xv32, cudaStream_t st)
 {
     k_xv32<<<(4 * p + 255) / 256, 256, 0, st>>>(xv, p, xv32);
-    return cudaGetLastError();
-}
-
-cudaError_t zb_x32(const int8_t *G, const double *xv, float *X32, int n, int p, int ldx, cudaStream_t st)
-{
-    k_x32<<<4096, 256, 0, st>>>(G, xv, X32, n, p, ldx);
     return cudaGetLastError();
 }
 

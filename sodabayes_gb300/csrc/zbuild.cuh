@@ -12,7 +12,6 @@ cudaError_t zb_freq(int8_t *G, int n, int p, int ldx, double *freq, int *bad, cu
 cudaError_t zb_gather(const int8_t *Gsnp, int8_t *Gpos, const int32_t *perm, int p, int ldx, cudaStream_t st);
 cudaError_t zb_xv(const double *freq, const int32_t *perm, int p, double *xv, cudaStream_t st);
 cudaError_t zb_xv32(const double *xv, int p, float *xv32, cudaStream_t st);
-cudaError_t zb_x32(const int8_t *G, const double *xv, float *X32, int n, int p, int ldx, cudaStream_t st);
 // tm_g: the codes G as [p][ldx] bytes in 128 x 128 boxes, 128-byte swizzle.  W32 (or nullptr): an FP32 copy of each
 // subset of the batch, columns ld32 apart, subsets ld32 * maxN.  *err is set when a device wait gave up.
 cudaError_t zb_gram(const CUtensorMap *tm_g, const int8_t *G, int ldx, const int32_t *blk_ls,

@@ -102,6 +102,16 @@ __host__ __device__ __forceinline__ void crng_warm(CRng &s)
     s.have = 2;
 }
 
+__host__ __device__ __forceinline__ uint64_t crng_u64(CRng &s);
+
+// Steps over the first n uniforms of a fresh stream.
+__device__ __forceinline__ void crng_skip(CRng &s, int n)
+{
+    s.tpos += n;
+    s.c3 += (uint32_t)(n >> 1);
+    if (!s.tape && (n & 1)) crng_u64(s);
+}
+
 __host__ __device__ __forceinline__ uint64_t crng_u64(CRng &s)
 {
     if (s.have == 2) {
@@ -207,6 +217,7 @@ template <typename T>
 struct GammaPre {
     T d, v, wp;
     bool small;
+    int taken;   // uniforms used: three when the first candidate is accepted and the shape is at least 1
 };
 template <typename T>
 __device__ __forceinline__ GammaPre<T> gamma_pre(T shape, CRng &s, int *err)
@@ -217,12 +228,15 @@ __device__ __forceinline__ GammaPre<T> gamma_pre(T shape, CRng &s, int *err)
     g.d = sh - (T)1.0 / (T)3.0;
     const T c = (T)1.0 / t_sqrt((T)9.0 * g.d);
     int tries = 0;
+    g.taken = 0;
     for (;;) {
         T x = t_rnorm<T>((T)0.0, (T)1.0, s);
         T v = (T)1.0 + c * x;
+        g.taken += 3;
         while (v <= (T)0.0 && tries < 100000) {
             x = t_rnorm<T>((T)0.0, (T)1.0, s);
             v = (T)1.0 + c * x;
+            g.taken += 2;
             ++tries;
         }
         v = v * v * v;
@@ -238,6 +252,7 @@ __device__ __forceinline__ GammaPre<T> gamma_pre(T shape, CRng &s, int *err)
     if (g.small) {
         // shape < 1: g ~ gamma(shape+1, 1), then scale*g*w**(1/shape)
         const T w = crng_unit_t<T>(s);
+        ++g.taken;
         g.wp = t_pow(w, (T)1.0 / shape);
     }
     return g;

@@ -980,8 +980,8 @@ __global__ void __launch_bounds__(256) k_stats(Dev D)
 
 // The hyper-parameter draws of a chain, one CTA.  They are bound by the latency of a few FP64 draws, so the
 // three that do not depend on one another run at once: sigma2_g in warp 0, sigma2_e in warp 1, and pi in the
-// others, one thread a group.  With the sums before them and the tables after them spread over the CTA's
-// threads, a chain of BayesR takes 28 us (62 us when one thread did it all).
+// others, a lane for each of its gamma variates.  With the sums before them and the tables after them spread over
+// the CTA's threads, a chain of BayesR takes 18 us (62 us when one thread did it all, 28 us with one thread a group).
 constexpr int HYPER_THREADS = 256;
 
 __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
@@ -1042,15 +1042,45 @@ __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
         crng_site(R, D, c, rep, 0, P_VARE);
         S->vare = d_rscinvchi2(nn + D.df_ve, scale, R, &err);
     } else if (warp >= 2 && (m == SODAGPU_BAYES_CPI || m == SODAGPU_BAYES_R || m == SODAGPU_BAYES_RC)) {
-        // pi ~ Dirichlet(counts + alpha), one thread per group (models.f90:517-522), groups over the warps first
-        for (int i = lane * (NW - 2) + warp - 2; i < ng; i += 32 * (NW - 2)) {
+        // pi ~ Dirichlet(counts + alpha) of each group (models.f90:517-522).  The nm gamma variates of a group come from
+        // one stream, one after another, 5 us each; nearly always each takes exactly three uniforms, so nm lanes draw
+        // them at once from those places, and where one but the last took more, its group's first lane draws them in turn
+        const int per = 32 / nm, sub = lane / nm, j = lane - sub * nm, first = sub * nm;
+        for (int i0 = (warp - 2) * per; i0 < ng; i0 += (NW - 2) * per) {
+            const int i = i0 + sub;
+            const bool in = sub < per && i < ng;
             CRng R;
-            crng_site(R, D, c, rep, i, P_PI);
-            double x[MAXDIST], sx = 0.0;
-            for (int j = 0; j < nm; ++j)
-                x[j] = d_rgamma((double)S->snpindist[i + j * ng] + D.alpha[j], 1.0, R, &err);
-            for (int j = 0; j < nm; ++j) sx = sx + x[j];
-            for (int j = 0; j < nm; ++j) S->p[i + j * ng] = x[j] / sx;
+            GammaPre<double> gam;
+            gam.taken = 3;
+            double x = 0.0;
+            int gerr = 0;
+            if (in) {
+                crng_site(R, D, c, rep, i, P_PI);
+                crng_skip(R, 3 * j);
+                gam = gamma_pre<double>((double)S->snpindist[i + j * ng] + D.alpha[j], R, &gerr);
+                x = gamma_from(1.0, gam);
+            }
+            const unsigned odd = __ballot_sync(0xffffffffu, in && j < nm - 1 && gam.taken != 3);
+            const bool redo = in && (odd >> first & ((1u << nm) - 1u)) != 0;
+            double y[MAXDIST];
+            if (redo) {
+                gerr = 0;
+                if (j == 0) {
+                    crng_site(R, D, c, rep, i, P_PI);
+                    for (int q = 0; q < nm; ++q)
+                        y[q] = d_rgamma((double)S->snpindist[i + q * ng] + D.alpha[q], 1.0, R, &gerr);
+                }
+            }
+            double sx = 0.0;
+            for (int q = 0; q < nm; ++q) {
+                double v = __shfl_sync(0xffffffffu, x, min(first + q, 31));
+                const double w = __shfl_sync(0xffffffffu, redo && j == 0 ? y[q] : 0.0, min(first, 31));
+                if (redo) v = w;
+                if (j == q) x = v;
+                sx = sx + v;
+            }
+            if (in) S->p[i + j * ng] = x / sx;
+            err |= gerr;
         }
     }
     if (err) flag_err(D, 1);
@@ -1118,11 +1148,13 @@ __device__ __forceinline__ void post_body(const Dev &D, const VB &vb)
     const int c = vb.y, rep = cur_rep(D);
     const ChainScal *S = &D.scal[c];
     const int t0 = vb.x * blockDim.x + threadIdx.x, stride = vb.nx * blockDim.x;
-    const double sd = sqrt(S->vare);
-    // FP64 draws: one row of every CTA's share after the other, so that the narrow FP64 pipes of all SMs
-    // take part (with CTA-contiguous rows the first CTAs of a chain did all of them: 26 us for 16 x 2000
-    // rows, 23 us like this)
-    for (int i = threadIdx.x * vb.nx + vb.x; i < D.naind; i += stride) {
+    // FP64 draws, spread over the FP64 pipes, of which each SM has one per four warps: every CTA takes an equal share of
+    // the rows, and CTAs that follow one another on an SM take theirs in different warps.  16 x 2000 rows: 18.6 us (26 us
+    // when the first CTAs of a chain did all of them, 23 us when the first warp of every CTA did)
+    const int turn = vb.x + vb.y * vb.nx, lin = (threadIdx.x + 32 * (turn + turn / 152)) & 255;
+    double sd = 0.0;
+    for (int i = lin * vb.nx + vb.x; i < D.naind; i += stride) {
+        if (sd == 0.0) sd = sqrt(S->vare);
         CRng R;
         crng_site(R, D, c, rep, i, P_RA);
         store_ra(D, c, i, d_rnorm(0.0, sd, R));

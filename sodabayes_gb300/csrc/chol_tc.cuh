@@ -20,7 +20,7 @@
 // The factorisation fails (status) on a pivot that is not positive, or, the same thing noticed earlier, when a
 // column's squares exceed M_jj.
 //
-// Measured, 10 subsets of 2000 SNPs: updates 3.1 ms, diagonal blocks 3.9, substitution 5.0 (the last two bound by the
+// Measured, 10 subsets of 2000 SNPs: updates 3.2 ms, diagonal blocks 2.9, substitution 2.6 (the last two bound by the
 // FP64 pipe, which takes any warp's instruction 64 cycles), against 31.9 ms of FP64 kernels (rank-32 updates 25.6,
 // panels 6.3).  U'U + A - d I is 2.2e-17 d at N = 301 and 1.3e-17 d at N = 1000 (rms), as before.
 #pragma once
@@ -221,8 +221,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     }
 }
 
-// 1 / sqrt(p) and sqrt(p) from an FP32 seed and Newton steps (FP64's own square root and division are some sixty
-// dependent instructions on the critical path of every pivot); each result is off by at most a unit in the last place.
+// 1 / sqrt(p) and sqrt(p) from an FP32 seed and one third-order step (FP64's own square root and division are twenty
+// dependent instructions on the critical path of every pivot, 64 cycles each); each result is off by at most a unit in
+// the last place.
 __device__ __forceinline__ void ch_rsqrt(double p, double &inv, double &root)
 {
     if (!(p > 1e-30 && p < 1e30)) {
@@ -230,12 +231,11 @@ __device__ __forceinline__ void ch_rsqrt(double p, double &inv, double &root)
         inv = 1.0 / root;
         return;
     }
-    double y = (double)rsqrtf((float)p);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) y = fma(y * 0.5, fma(-p * y, y, 1.0), y);
-    const double r = p * y;
-    root = fma(0.5 * y, fma(-r, r, p), r);
-    inv = fma(y, fma(-root, y, 1.0), y);
+    const double y = (double)rsqrtf((float)p);
+    const double e = fma(-(p * y), y, 1.0);                   // |e| < 2^-21
+    inv = fma(y * e, fma(e, 0.375, 0.5), y);                  // y (1 + e/2 + 3 e^2 / 8), error e^3
+    const double r = p * inv;
+    root = fma(0.5 * inv, fma(-r, r, p), r);
 }
 // c / root with inv = 1 / root
 __device__ __forceinline__ double ch_div(double c, double root, double inv)
@@ -244,8 +244,12 @@ __device__ __forceinline__ double ch_div(double c, double root, double inv)
     return fma(fma(-x, root, c), inv, x);
 }
 
-// The panel's diagonal block, in steps of 16: a warp factors 16 x 16 with a column a lane, a thread a column solves
-// the rest of its rows, and all threads take the rank-16 update.  piv: the pivots and their reciprocals, for k_ch_trsm.
+// The panel's diagonal block, in steps of 8: a warp factors 8 x 8 with a column a lane, a thread a column solves the
+// rest of its rows, and the warps take the rank-8 update's rows.  Bound by the chain of FP64 instructions: about 17 a
+// pivot in the factoring warp, 52 a step in the solving ones; 92 us a panel (121 us in steps of 16).  inv: the pivots'
+// reciprocals, for k_ch_trsm.
+constexpr int CH_D = 8;
+
 __global__ void __launch_bounds__(256) k_ch_diag(double *W, const int64_t *wofs, const int32_t *blk_ls,
                                                  const int32_t *batch_blocks, int32_t *status, int i0, double *piv)
 {
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(256) k_ch_diag(double *W, const int64_t *wofs,
     if (i0 >= N || status[b] != 0) return;
     const int nb = min(CH_P, N - i0);
     double *A = W + wofs[b] + (size_t)i0 * N + i0;
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int t = tid; t < CH_P * CH_P; t += 256) {
         const int r = t % CH_P, c = t / CH_P;
         // rows and columns past the subset: the identity, which changes nothing
@@ -267,53 +271,55 @@ __global__ void __launch_bounds__(256) k_ch_diag(double *W, const int64_t *wofs,
     }
     if (tid == 0) s_fail = 0;
     __syncthreads();
-    for (int kb = 0; kb < CH_P; kb += 16) {
-        if (tid < 32) {
-            const int c = kb + (lane & 15);
-            double x[16];
+    for (int kb = 0; kb < CH_P; kb += CH_D) {
+        if (warp == 0) {
+            const int l = lane & (CH_D - 1), c = kb + l;
+            double x[CH_D];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) x[r] = T[kb + r][c];
+            for (int r = 0; r < CH_D; ++r) x[r] = T[kb + r][c];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
+            for (int r = 0; r < CH_D; ++r) {
                 const double p = __shfl_sync(0xffffffffu, x[r], r);
                 if (!(p > 0.0) && lane == 0 && !s_fail) s_fail = i0 + kb + r + 1;
                 double inv, root;
                 ch_rsqrt(p, inv, root);
                 if (lane == r) s_inv[kb + r] = inv;
-                x[r] = (lane & 15) == r ? root : ch_div(x[r], root, inv);
+                x[r] = l == r ? root : ch_div(x[r], root, inv);
 #pragma unroll
-                for (int q = r + 1; q < 16; ++q) x[q] = fma(-__shfl_sync(0xffffffffu, x[r], q), x[r], x[q]);
+                for (int q = r + 1; q < CH_D; ++q) x[q] = fma(-__shfl_sync(0xffffffffu, x[r], q), x[r], x[q]);
             }
-            if (lane < 16)
+            if (lane < CH_D)
 #pragma unroll
-                for (int r = 0; r < 16; ++r)
+                for (int r = 0; r < CH_D; ++r)
                     if (r <= lane) T[kb + r][c] = x[r];
         }
         __syncthreads();
         if (s_fail) break;
-        const int c = kb + 16 + tid;
+        const int c = kb + CH_D + tid;
         if (c < CH_P) {
-            double x[16];
+            double x[CH_D];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) x[r] = T[kb + r][c];
+            for (int r = 0; r < CH_D; ++r) x[r] = T[kb + r][c];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
+            for (int r = 0; r < CH_D; ++r) {
                 x[r] = ch_div(x[r], T[kb + r][kb + r], s_inv[kb + r]);
 #pragma unroll
-                for (int q = r + 1; q < 16; ++q) x[q] = fma(-T[kb + r][kb + q], x[r], x[q]);
+                for (int q = r + 1; q < CH_D; ++q) x[q] = fma(-T[kb + r][kb + q], x[r], x[q]);
             }
 #pragma unroll
-            for (int r = 0; r < 16; ++r) T[kb + r][c] = x[r];
+            for (int r = 0; r < CH_D; ++r) T[kb + r][c] = x[r];
         }
         __syncthreads();
-        const int m = CH_P - kb - 16;
-        for (int t = tid; t < m * m; t += 256) {
-            const int r = kb + 16 + t % m, cc = kb + 16 + t / m;
-            if (r > cc) continue;
-            double s = T[r][cc];
+        for (int r = kb + CH_D + warp; r < CH_P; r += 8) {
+            double m[CH_D];
 #pragma unroll
-            for (int q = 0; q < 16; ++q) s = fma(-T[kb + q][r], T[kb + q][cc], s);
-            T[r][cc] = s;
+            for (int q = 0; q < CH_D; ++q) m[q] = -T[kb + q][r];
+            for (int cc = (r & ~31) + lane; cc < CH_P; cc += 32) {
+                double s = T[r][cc];
+#pragma unroll
+                for (int q = 0; q < CH_D; ++q) s = fma(m[q], T[kb + q][cc], s);
+                if (cc >= r) T[r][cc] = s;
+            }
         }
         __syncthreads();
     }
@@ -328,58 +334,89 @@ __global__ void __launch_bounds__(256) k_ch_diag(double *W, const int64_t *wofs,
     if (tid < CH_P) piv[(size_t)blockIdx.x * CH_P + tid] = s_inv[tid];
 }
 
-// The panel's rows for the columns right of it, one column a thread: substitution (the FP64 pipe bounds it: CH_P^2 / 2
-// multiply-adds a column, a warp a CTA so that every SM's pipe takes part), the columns' squares, and the digits of the
-// new rows, [digit][column][row], eight rows a 16-byte store.
-__global__ void __launch_bounds__(32)
+// The panel's rows for 32 columns right of it: substitution in blocks of 16 rows, the columns' squares, and the digits
+// of the new rows, [digit][column][row], eight rows a 16-byte store.  A block is solved by one warp, a column a lane
+// (the warp changes with the block and the CTA, so that all of an SM's FP64 pipes are used), and four warps take its
+// products out of the rows below: 1120 instructions in a chain, 64 cycles each, in place of 2400 for a column a thread: 85 us a
+// panel of 10 subsets of 2000 SNPs, 161 us before.
+constexpr int CH_S = 16;
+constexpr size_t CH_TRSM_SMEM = sizeof(double) * (CH_P * CH_P + CH_P * 32 + CH_P);
+
+__global__ void __launch_bounds__(128)
     k_ch_trsm(double *W, const int64_t *wofs, const int32_t *blk_ls, const int32_t *batch_blocks, const double *xxd,
               const double *sc, double *nrm, int np, int32_t *status, int i0, const double *piv, uint16_t *dig, int ldt)
 {
-    __shared__ double T[CH_P][CH_P];      // row r of the diagonal block's factor
-    __shared__ double s_inv[CH_P];
+    extern __shared__ __align__(16) double ch_smem[];
+    __shared__ double s_ss[CH_P / CH_S][32];
+    double (*T)[CH_P] = reinterpret_cast<double (*)[CH_P]>(ch_smem);                   // row r of the block's factor
+    double (*C)[32] = reinterpret_cast<double (*)[32]>(ch_smem + CH_P * CH_P);         // the columns
+    double *s_inv = ch_smem + CH_P * CH_P + CH_P * 32;
     tc::pdl_trigger();
     tc::pdl_wait();
     const int b = batch_blocks[blockIdx.y];
     const int N = blk_ls[b + 1] - blk_ls[b], c0 = i0 + CH_P + 32 * blockIdx.x;
-    const int lane = threadIdx.x, j = c0 + lane;
-    // (columns of other CTAs may fail meanwhile: one lane reads)
-    if (c0 >= N || __shfl_sync(0xffffffffu, status[b], 0) != 0) return;
+    if (__syncthreads_or(c0 >= N || status[b] != 0)) return;   // (columns of other CTAs may fail meanwhile)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, j = c0 + lane;
     double *A = W + wofs[b];
-    for (int c = 0; c < CH_P; ++c)
-        for (int r = lane; r <= c; r += 32) T[r][c] = A[(size_t)(i0 + r) + (size_t)(i0 + c) * N];
-    for (int r = lane; r < CH_P; r += 32) s_inv[r] = piv[(size_t)blockIdx.y * CH_P + r];
-    __syncwarp();
-    if (j >= N) return;
-    double x[CH_P];
-    double *col = A + (size_t)j * N + i0;
-#pragma unroll
-    for (int r = 0; r < CH_P; ++r) x[r] = col[r];
-    double ss = 0.0;
-#pragma unroll
-    for (int r = 0; r < CH_P; ++r) {
-        x[r] = ch_div(x[r], T[r][r], s_inv[r]);
-        ss = fma(x[r], x[r], ss);
-#pragma unroll
-        for (int q = r + 1; q < CH_P; ++q) x[q] = fma(-T[r][q], x[r], x[q]);
+    for (int t = tid; t < CH_P * CH_P; t += 128) {
+        const int r = t % CH_P, c = t / CH_P;
+        if (r <= c) T[r][c] = A[(size_t)(i0 + r) + (size_t)(i0 + c) * N];
     }
+    for (int t = tid; t < CH_P * 32; t += 128) {
+        const int r = t % CH_P, c = t / CH_P;
+        C[r][c] = c0 + c < N ? A[(size_t)(i0 + r) + (size_t)(c0 + c) * N] : 0.0;
+    }
+    if (tid < CH_P) s_inv[tid] = piv[(size_t)blockIdx.y * CH_P + tid];
+    __syncthreads();
+    for (int kb = 0; kb < CH_P; kb += CH_S) {
+        if (warp == ((kb / CH_S + blockIdx.x) & 3)) {
+            double x[CH_S], ss = 0.0;
 #pragma unroll
-    for (int r = 0; r < CH_P; ++r) col[r] = x[r];
-    // the squares of a column never exceed M_jj (its diagonal entry is still A's) when M is positive definite
+            for (int r = 0; r < CH_S; ++r) x[r] = C[kb + r][lane];
+#pragma unroll
+            for (int r = 0; r < CH_S; ++r) {
+                x[r] = ch_div(x[r], T[kb + r][kb + r], s_inv[kb + r]);
+                ss = fma(x[r], x[r], ss);
+#pragma unroll
+                for (int q = r + 1; q < CH_S; ++q) x[q] = fma(-T[kb + r][kb + q], x[r], x[q]);
+            }
+#pragma unroll
+            for (int r = 0; r < CH_S; ++r) C[kb + r][lane] = x[r];
+            s_ss[kb / CH_S][lane] = ss;
+        }
+        __syncthreads();
+        if (kb + CH_S < CH_P) {
+            double x[CH_S];
+#pragma unroll
+            for (int q = 0; q < CH_S; ++q) x[q] = -C[kb + q][lane];
+            for (int r = kb + CH_S + warp; r < CH_P; r += 4) {
+                double s = C[r][lane];
+#pragma unroll
+                for (int q = 0; q < CH_S; ++q) s = fma(T[kb + q][r], x[q], s);
+                C[r][lane] = s;
+            }
+            __syncthreads();
+        }
+    }
+    for (int t = tid; t < CH_P * 32; t += 128) {
+        const int r = t % CH_P, c = t / CH_P;
+        if (c0 + c < N) A[(size_t)(i0 + r) + (size_t)(c0 + c) * N] = C[r][c];
+    }
+    if (j >= N) return;
     const size_t o = (size_t)blockIdx.y * np + j;
-    ss += nrm[o];
-    nrm[o] = ss;
-    if (!(ss <= (xxd[b] - A[(size_t)j + (size_t)j * N]) * (1.0 + 1e-9))) {
-        status[b] = i0 + CH_P + 1;
-        return;
+    if (warp == 0) {
+        // the squares of a column never exceed M_jj (its diagonal entry is still A's) when M is positive definite
+        const double ss = nrm[o] + ((s_ss[0][lane] + s_ss[1][lane]) + (s_ss[2][lane] + s_ss[3][lane]));
+        nrm[o] = ss;
+        if (!(ss <= (xxd[b] - A[(size_t)j + (size_t)j * N]) * (1.0 + 1e-9))) status[b] = i0 + CH_P + 1;
     }
     const double q55 = 36028797018963968.0 / sc[o];   // 2^55 / 2^e_j: one unit is 2^-55 of the bound
     uint16_t *dst = dig + ((size_t)blockIdx.y * CH_DIG * np + j) * ldt + i0;
-#pragma unroll
-    for (int r0 = 0; r0 < CH_P; r0 += 8) {
+    for (int r0 = CH_S * warp; r0 < CH_S * (warp + 1); r0 += 8) {
         uint32_t w[CH_DIG][4];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            long long v = __double2ll_rn(x[r0 + e] * q55);
+            long long v = __double2ll_rn(C[r0 + e][lane] * q55);
 #pragma unroll
             for (int s = CH_DIG - 1; s >= 0; --s) {
                 const int dgt = s > 0 ? (int)(signed char)(v & 0xFF) : (int)v;

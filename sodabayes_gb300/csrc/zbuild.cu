@@ -596,6 +596,8 @@ cudaError_t zb_cholesky(const CUtensorMap *tm_a, const CUtensorMap *tm_b, double
     double *sc = work, *nrm = sc + (size_t)nbatch * np, *piv = nrm + (size_t)nbatch * np;
     cudaError_t e = cudaFuncSetAttribute(k_ch_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM);
     if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_ch_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_TRSM_SMEM);
+    if (e != cudaSuccess) return e;
     k_ch_init<<<nbatch, 256, 0, st>>>(W, wofs, blk_ls, batch_blocks, xxd, sc, nrm, np, status);
     e = cudaGetLastError();
     for (int i0 = 0; i0 < maxN && e == cudaSuccess; i0 += CH_P) {
@@ -604,7 +606,7 @@ cudaError_t zb_cholesky(const CUtensorMap *tm_a, const CUtensorMap *tm_b, double
         if (e == cudaSuccess)
             e = launch_after(k_ch_diag, dim3(nbatch), dim3(256), 0, st, W, wofs, blk_ls, batch_blocks, status, i0, piv);
         if (e == cudaSuccess && maxN - i0 > CH_P)
-            e = launch_after(k_ch_trsm, dim3((maxN - i0 - CH_P + 31) / 32, nbatch), dim3(32), 0, st, W, wofs, blk_ls,
+            e = launch_after(k_ch_trsm, dim3((maxN - i0 - CH_P + 31) / 32, nbatch), dim3(128), CH_TRSM_SMEM, st, W, wofs, blk_ls,
                              batch_blocks, xxd, (const double *)sc, nrm, np, status, i0, (const double *)piv, dig, ldt);
     }
     return e;

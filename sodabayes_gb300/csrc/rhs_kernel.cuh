@@ -194,7 +194,7 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
     }
     __syncthreads();
     DrawSnp<T> ahead;
-    if (snp >= 0 && !D.rhs_out) draw_ahead(D, s_sub[c], (T)zz, vs, R, ahead);
+    if (snp >= 0 && !D.rhs_out) draw_ahead(D, &D.scal[c], s_sub[c], (T)zz, vs, sg, R, ahead);
     // tensor-core path: the rhs is assembled in FP32 (its split sums are FP32; the FP64 pipe of
     // GB300 is narrow and also runs every double <-> float conversion)
     const float x0f = (float)x0, rsf = TC ? (float)s_rs[c] : 0.0f;

@@ -135,6 +135,8 @@ struct DrawSub {
     // class k: log pi of group 1, log(gamma_k sigma2_g zz / sigma2_e + 1), the denominators of the score and
     // of the conditional mean, the conditional standard deviation
     T logp[DRAW_PRE], ld[DRAW_PRE], den[DRAW_PRE], v1[DRAW_PRE], sd[DRAW_PRE];
+    // FP64: class k's score is b_k + c_k rhs^2 (b_k: DrawSnp), the quotient rhs^2 / (den sigma2_e) / 2 as one factor
+    T c[DRAW_PRE];
 };
 
 // Class k of chain S in a subset with d = zz (k = 0 also fills what all classes share).
@@ -155,6 +157,7 @@ __device__ __forceinline__ void draw_sub(const Dev &D, const ChainScal *S, int k
     q.den[k] = zt + (in ? (T)S->vare_gp[k] : (T)0.0);
     q.v1[k] = zt + vare / gp;
     q.sd[k] = t_sqrt(vare / q.v1[k]);
+    if constexpr (sizeof(T) == 8) q.c[k] = k > 0 ? 0.5 / (q.den[k] * vare) : 0.0;
 }
 
 template <typename T>
@@ -163,13 +166,15 @@ struct DrawSnp {
     NormalPre<T> z;
     GammaPre<T> gam;       // BayesA/B
     T ld, den, sd, sdv;    // BayesA/B: from the locus variance
+    T b[DRAW_PRE], c;      // FP64 scores: what does not depend on the right-hand side (c: BayesB's factor)
     bool plain;            // a standard deviation is 0: the draws follow the plain order at their use
     int err;
 };
 
 // Advances R past the uniforms that the SNP's draw takes (up to the class uniform when `plain`).
 template <typename T>
-__device__ __forceinline__ void draw_ahead(const Dev &D, const DrawSub<T> &q, T zz, T vs, CRng &R, DrawSnp<T> &a)
+__device__ __forceinline__ void draw_ahead(const Dev &D, const ChainScal *S, const DrawSub<T> &q, T zz, T vs, int sg,
+                                           CRng &R, DrawSnp<T> &a)
 {
     const int m = D.method;
     a.plain = false;
@@ -183,6 +188,11 @@ __device__ __forceinline__ void draw_ahead(const Dev &D, const DrawSub<T> &q, T 
             a.sdv = t_sqrt(vs);
             a.plain = a.plain || a.sdv <= (T)0.0;
             a.u = crng_unit_t<T>(R);
+            if constexpr (sizeof(T) == 8) {
+                a.c = 0.5 / (a.den * q.vare);
+                a.b[0] = S->log_p[0];
+                a.b[1] = S->log_p[D.ngroup] - 0.5 * a.ld;
+            }
         }
         if (a.plain) return;
         a.z = normal_pre<T>(R);
@@ -191,6 +201,52 @@ __device__ __forceinline__ void draw_ahead(const Dev &D, const DrawSub<T> &q, T 
     }
     a.u = crng_unit_t<T>(R);
     a.z = normal_pre<T>(R);
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int k = 0; k < DRAW_PRE; ++k)
+            if (k < D.nmix) a.b[k] = S->log_p[sg + k * D.ngroup] - (k > 0 ? 0.5 * q.ld[k] : 0.0);
+    }
+}
+
+// The class (1-based) for the FP64 scores b_k + c_k r2 of up to DRAW_PRE classes: the first whose cumulative weight
+// exceeds u times their sum, weights exp(s_k - s_0), or relative to the largest score where that could overflow.  (The
+// probabilities of models.f90:366-379 one by one take up to twelve exponentials and four divisions, 16 and 10 FP64
+// instructions of 64 cycles each, in every warp with a SNP outside the first class.)
+__device__ __forceinline__ int draw_class64(double r2, const double (&b)[DRAW_PRE], const double (&c)[DRAW_PRE],
+                                            int nm, double u)
+{
+    double w[DRAW_PRE], ref = b[0];
+    bool big = false;
+#pragma unroll
+    for (int k = 0; k < DRAW_PRE; ++k) {
+        w[k] = k == 0 ? b[0] : (k < nm ? fma(r2, c[k], b[k]) : -1e308);
+        big = big || w[k] - b[0] > 700.0;
+    }
+    if (big) {
+#pragma unroll
+        for (int k = 1; k < DRAW_PRE; ++k) ref = fmax(ref, w[k]);
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < DRAW_PRE; ++k)
+        if (k < nm) {
+            w[k] = k == 0 && !big ? 1.0 : exp(w[k] - ref);
+            sum = sum + w[k];
+        }
+    const double us = u * sum;
+    double cum = 0.0;
+    int flag = 1;
+    bool done = false;
+#pragma unroll
+    for (int k = 0; k < DRAW_PRE; ++k)
+        if (k < nm && !done) {
+            cum = cum + w[k];
+            if (us < cum) {
+                flag = k + 1;
+                done = true;
+            }
+        }
+    return flag;
 }
 
 // Returns delta = g_old - g_new; gold = g and cl = class of the SNP in this chain, sg = its group - 1.
@@ -206,7 +262,11 @@ __device__ __forceinline__ double draw_snp(const Dev &D, const ChainScal *S, int
         const T df_va = (T)D.df_va;
         int flag = 2;
         if (m == SODAGPU_BAYES_A || cl > 1) rhs = rhs + zz * gk;
-        if (m == SODAGPU_BAYES_B) {
+        if (m == SODAGPU_BAYES_B && sizeof(T) == 8) {
+            // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2))
+            const T d = a.b[0] - (a.b[1] + a.c * (rhs * rhs));
+            flag = a.u * ((T)1.0 + t_exp(d)) < (T)1.0 ? 2 : 1;
+        } else if (m == SODAGPU_BAYES_B) {
             const T s1 = q.logp[0];
             const T uhat = rhs / a.den;
             const T s2 = (T)-0.5 * (a.ld - (rhs * uhat / vare)) + q.logp[1];
@@ -237,36 +297,40 @@ __device__ __forceinline__ double draw_snp(const Dev &D, const ChainScal *S, int
     int flag = 1;
     T v1, sd;
     if (nm <= DRAW_PRE) {
-        // every loop unrolled: the scores stay in registers
-        T sv[DRAW_PRE];
+        if constexpr (sizeof(T) == 8) {
+            flag = draw_class64(rhs * rhs, a.b, q.c, nm, a.u);
+        } else {
+            // every loop unrolled: the scores stay in registers
+            T sv[DRAW_PRE];
 #pragma unroll
-        for (int kk = 0; kk < DRAW_PRE; ++kk) {
-            const T lp = ng > 1 && kk < nm ? (T)S->log_p[sg + kk * ng] : q.logp[kk];
-            sv[kk] = lp;
-            if (kk > 0 && kk < nm) {
-                const T uhat = rhs / q.den[kk];
-                sv[kk] = (T)-0.5 * (q.ld[kk] - (rhs * uhat / vare)) + lp;
-            }
-        }
-        T ssculm = (T)0.0;
-        bool done = false;
-#pragma unroll
-        for (int kk = 0; kk < DRAW_PRE; ++kk) {
-            if (kk < nm && !done) {
-                T sk = (T)0.0;
-                bool overflow = false;
-#pragma unroll
-                for (int j = 0; j < DRAW_PRE; ++j) {
-                    if (j < nm && j != kk && !overflow) {
-                        const T clike = sv[j] - sv[kk];
-                        if (clike > (T)700.0) overflow = true;
-                        else if (clike >= (T)-700.0) sk = sk + t_exp(clike);
-                    }
+            for (int kk = 0; kk < DRAW_PRE; ++kk) {
+                const T lp = ng > 1 && kk < nm ? (T)S->log_p[sg + kk * ng] : q.logp[kk];
+                sv[kk] = lp;
+                if (kk > 0 && kk < nm) {
+                    const T uhat = rhs / q.den[kk];
+                    sv[kk] = (T)-0.5 * (q.ld[kk] - (rhs * uhat / vare)) + lp;
                 }
-                ssculm = ssculm + (overflow ? (T)0.0 : (T)1.0 / ((T)1.0 + sk));
-                if (a.u < ssculm) {
-                    flag = kk + 1;
-                    done = true;
+            }
+            T ssculm = (T)0.0;
+            bool done = false;
+#pragma unroll
+            for (int kk = 0; kk < DRAW_PRE; ++kk) {
+                if (kk < nm && !done) {
+                    T sk = (T)0.0;
+                    bool overflow = false;
+#pragma unroll
+                    for (int j = 0; j < DRAW_PRE; ++j) {
+                        if (j < nm && j != kk && !overflow) {
+                            const T clike = sv[j] - sv[kk];
+                            if (clike > (T)700.0) overflow = true;
+                            else if (clike >= (T)-700.0) sk = sk + t_exp(clike);
+                        }
+                    }
+                    ssculm = ssculm + (overflow ? (T)0.0 : (T)1.0 / ((T)1.0 + sk));
+                    if (a.u < ssculm) {
+                        flag = kk + 1;
+                        done = true;
+                    }
                 }
             }
         }
@@ -510,7 +574,7 @@ __device__ __forceinline__ void skipped_pre_body(const Dev &D, const VB &vb, int
         sub.zz_vare = zz_vare;
         DrawSnp<double> a;
         a.u = a.ld = a.sdv = 0.0;
-        draw_ahead(D, sub, zz, vs, R, a);
+        draw_ahead(D, S, sub, zz, vs, 0, R, a);
         q[SS_U] = a.u;
         q[SS_DEN] = a.den;
         q[SS_SD] = a.sd;

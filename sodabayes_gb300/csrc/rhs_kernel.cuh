@@ -95,10 +95,11 @@ __device__ __forceinline__ float code_to_f32(uint32_t w, int k)
 }
 
 // Threads of a draw CTA.  With the CUDA-core rhs a subset has N * CT draws, few for one or two chains, and in the
-// FP64 mode each is some hundred instructions of the FP64 pipe, which takes a warp's instruction 16 cycles: the draws
+// FP64 mode each is some hundred instructions of the FP64 pipe, which takes a warp's instruction 64 cycles: the draws
 // are spread over the SMs, a warp each (two for 4 chains and more, whose CTAs need at least CT threads).  N = 935, one
 // FP64 chain, the kernel by itself: 34 us, against 42 us in four CTAs of 256 threads (most of it now lies before the
-// dependency wait: an iteration of 10 subsets takes 527 us, 636 us without draw_ahead, 745 us with neither).
+// dependency wait: an iteration of 10 subsets took 527 us with both, 636 us without draw_ahead and 745 us with neither;
+// with the cheaper class draws and the later rhs and update it takes 341 us).
 // The tensor-core path has C >= 4 and FP32 draws: 256 threads fill the SMs.
 template <int CT, bool TC>
 struct DrawThreads { static constexpr int v = TC ? 256 : (CT <= 2 ? 32 : 64); };

@@ -953,8 +953,8 @@ int sodagpu_init_chains(sodagpu_ctx *c)
             TRY(c->alloc(&c->ssrec, sweep_skip_records(c->nskipped, C, nm), false));
             TRY(c->alloc(&c->ssdense, C));
         }
-        TRY(c->alloc(&c->rpx, (size_t)RHS_KSPLIT_MAX * C * c->bs));
-        TRY(c->alloc(&c->rpu, (size_t)RHS_KSPLIT_MAX * C * c->bs));
+        TRY(c->alloc(&c->rpx, (size_t)RHS_KSPLIT_MAX_CC * C * c->bs));
+        TRY(c->alloc(&c->rpu, (size_t)RHS_KSPLIT_MAX_CC * C * c->bs));
         c->tc = !c->regular && c->cfg.kernels == SODAGPU_KERNELS_AUTO &&
                 sweep_tc_supported(c->cfg.precision, C, c->bs);
         if (c->tc) {

@@ -23,9 +23,14 @@
 // individuals so that every SM has a share, and a warp's sums are reduced eight at a time (nine exchanges in
 // place of forty; in FP64 the forty took longer than the products).  Measured by
 // itself, its loads not early: FP64, N = 935, n = 2,326: 15.5 us (26.7 with stages
-// of 512 and two reductions); an FP32 iteration of 50 subsets of N = 1000, n =
-// 5,000: 0.90 ms (1.21 with FP32 columns of four times the bytes, one CTA an SM and
-// no early loads); a step of eight FP8 analyses: 31.5 us (36.5).
+// of 512 and two reductions); a step of eight FP8 analyses: 31.5 us (36.5).
+// With more individuals the FP32 mode is bound by the instructions that turn a
+// code into its x value: a test of one bit of the word for each of two
+// selections, not a shift, a mask and two comparisons (FP64 reads a byte a code).  With that, and up to 24 K
+// splits in place of 16 (the last stage of an uneven share is the whole kernel's),
+// a subset of one FP32 chain takes, draws and update included: N = 2000, n = 20,000:
+// 32.1 us (49.6); N = 500, n = 20,000: 17.9 us (29.6); N = 1000, n = 10,000: 19.8 us
+// (26.2).  FP32 columns of four times the bytes, one CTA an SM: 51.2, 26.9, 29.7 us.
 #pragma once
 #include <cuda_pipeline_primitives.h>
 
@@ -219,9 +224,9 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
         // columns with sd = 0 (zero codes) carry U unscaled
         xf = __fmaf_rn(x0f, rsf, __fmul_rn(xs, inv32 != 0.0f ? inv32 : 1.0f));
     } else {
-        double px[RHS_KSPLIT_MAX], pu[RHS_KSPLIT_MAX];
+        double px[RHS_KSPLIT_MAX_CC], pu[RHS_KSPLIT_MAX_CC];
 #pragma unroll
-        for (int sp = 0; sp < RHS_KSPLIT_MAX; ++sp) {
+        for (int sp = 0; sp < RHS_KSPLIT_MAX_CC; ++sp) {
             px[sp] = pu[sp] = 0.0;
             if (act && sp < ksplit) {
                 const size_t o = ((size_t)sp * CT + c) * D.bs + jl;
@@ -230,7 +235,7 @@ __device__ __forceinline__ void draw_body(const Dev &D, const VB &vb, int b, int
             }
         }
 #pragma unroll
-        for (int sp = 0; sp < RHS_KSPLIT_MAX; ++sp) {
+        for (int sp = 0; sp < RHS_KSPLIT_MAX_CC; ++sp) {
             if (sp < ksplit) {
                 xr += px[sp];
                 if (MODE == SODAGPU_FP8) ur += pu[sp];
@@ -460,8 +465,8 @@ __device__ __forceinline__ void rhs_body(const Dev &D, const VB &vb, int b, int 
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         if constexpr (MODE == SODAGPU_FP32) {
-                            const uint32_t g = w >> (8 * e) & 3u;
-                            x[s][e] = g == 0u ? xl[s][0] : (g == 1u ? xl[s][1] : xl[s][2]);
+                            // one instruction tests a bit: the shift and mask of a comparison would be two more
+                            x[s][e] = w & (2u << (8 * e)) ? xl[s][2] : (w & (1u << (8 * e)) ? xl[s][1] : xl[s][0]);
                         } else {
                             x[s][e] = code_to_f32(w, e);
                         }

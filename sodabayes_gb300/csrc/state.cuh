@@ -109,7 +109,7 @@ struct Dev {
     double *recal_part;        // [C][RECAL_SPLIT][ldr]
     double *ssrec;             // [C][min(nskipped, SS_CHUNK)][SS_HEAD + 2 nmix] single-site draws' constants
     int32_t *ssdense;          // [C] SNPs of the current chunk that are in the model
-    double *rpx, *rpu;         // [RHS_KSPLIT_MAX][C][bs] rhs partial sums (genotype / augmented part)
+    double *rpx, *rpu;         // [RHS_KSPLIT_MAX_CC][C][bs] rhs partial sums (genotype / augmented part)
     // tensor-core sweep (FP8 mode, 4/8/16 chains)
     int tc;                    // 1 when the tensor-core kernels run
     int ldd;                   // row stride of dsplit (bs rounded up to 128)
@@ -183,7 +183,8 @@ __device__ __forceinline__ int jg_locate(const JobGrid &G, VB &vb)
     return lo;
 }
 
-constexpr int RHS_KSPLIT_MAX = 16;
+constexpr int RHS_KSPLIT_MAX = 16;     // K splits of the tensor-core rhs
+constexpr int RHS_KSPLIT_MAX_CC = 24;  // of the CUDA-core rhs, whose draws have registers for more loads at once
 
 constexpr int NSTAT = 64;          // CTAs of the per-iteration SNP statistics
 constexpr int ROW_THREADS = 128;   // threads of the row kernels

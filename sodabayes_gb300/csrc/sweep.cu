@@ -1489,7 +1489,7 @@ static cudaError_t launch_block_tc(const Dev &D, int b, int nblk_snps, int sm_co
 // genotype stages (a split with one stage fewer only waits for the others).
 static int rhs_splits(int ctas, int mtiles, int nst)
 {
-    int ks = std::max(1, std::min({ctas / std::max(1, mtiles), RHS_KSPLIT_MAX, nst}));
+    int ks = std::max(1, std::min({ctas / std::max(1, mtiles), RHS_KSPLIT_MAX_CC, nst}));
     const int per = (nst + ks - 1) / ks;
     return (nst + per - 1) / per;
 }

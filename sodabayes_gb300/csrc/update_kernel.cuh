@@ -126,8 +126,7 @@ __device__ __forceinline__ void update_body(const Dev &D, const VB &vb, int b)
                     }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const uint32_t code = (wv >> (8 * e)) & 3u;
-                        x[u][e] = code == 0u ? x0 : (code == 1u ? x1 : x2);
+                        x[u][e] = wv & (2u << (8 * e)) ? x2 : (wv & (1u << (8 * e)) ? x1 : x0);
                     }
                 }
             } else if (i0 + 4 <= npad) {

@@ -1147,6 +1147,8 @@ int sodagpu_get_state(sodagpu_ctx *c, int32_t chain, double *g, int32_t *cls, do
     if (chain < 0 || chain >= c->C) return fail(SODAGPU_E_ARG, "chain out of range");
     const int p = c->p;
     const size_t off = (size_t)chain * p;
+    // the caller's yaadj holds blocksize entries, in the regular sampler (bs = 8) perhaps fewer than bs
+    const size_t nra = (size_t)std::max(0, std::min(c->bs, c->cfg.blocksize));
     unsigned want = (g ? STATE_G : 0) | (vara_s ? STATE_VARA_S : 0) | (yadj ? STATE_R : 0) | (yaadj ? STATE_RA : 0) |
                     (cls ? STATE_CLS : 0);
     StateLayout L = sweep_state_layout(c->D, want);
@@ -1162,13 +1164,13 @@ int sodagpu_get_state(sodagpu_ctx *c, int32_t chain, double *g, int32_t *cls, do
         if (yadj)
             CUDA_TRY(cudaMemcpy(yadj, c->r + (size_t)chain * c->ldr, sizeof(double) * c->n, cudaMemcpyDeviceToHost));
         if (yaadj)
-            CUDA_TRY(cudaMemcpy(yaadj, c->ra + (size_t)chain * c->ldra, sizeof(double) * c->bs, cudaMemcpyDeviceToHost));
+            CUDA_TRY(cudaMemcpy(yaadj, c->ra + (size_t)chain * c->ldra, sizeof(double) * nra, cudaMemcpyDeviceToHost));
     } else {
         if (g) memcpy(g, c->pinned + L.g, sizeof(double) * p);
         if (cls) memcpy(cls, c->pinned + L.cls, sizeof(int32_t) * p);
         if (vara_s) memcpy(vara_s, c->pinned + L.vara_s, sizeof(double) * p);
         if (yadj) memcpy(yadj, c->pinned + L.r, sizeof(double) * c->n);
-        if (yaadj) memcpy(yaadj, c->pinned + L.ra, sizeof(double) * c->bs);
+        if (yaadj) memcpy(yaadj, c->pinned + L.ra, sizeof(double) * nra);
     }
     if (scalars) memcpy(scalars, c->pinned + L.scalars, 4 * sizeof(double));
     return 0;
@@ -1200,7 +1202,9 @@ int sodagpu_set_state(sodagpu_ctx *c, int32_t chain, const double *g, const int3
     CUDA_TRY(cudaMemcpyAsync(c->st_cls, cls, sizeof(int32_t) * p, cudaMemcpyHostToDevice, c->st));
     CUDA_TRY(cudaMemcpyAsync(c->st_vs, vara_s, sizeof(double) * p, cudaMemcpyHostToDevice, c->st));
     CUDA_TRY(cudaMemcpyAsync(c->st_r, yadj, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->st));
-    CUDA_TRY(cudaMemcpyAsync(c->st_ra, yaadj, sizeof(double) * c->bs, cudaMemcpyHostToDevice, c->st));
+    const size_t nra = (size_t)std::max(0, std::min(c->bs, c->cfg.blocksize));   // the caller's array (sodagpu_get_state)
+    CUDA_TRY(cudaMemsetAsync(c->st_ra, 0, sizeof(double) * c->bs, c->st));
+    CUDA_TRY(cudaMemcpyAsync(c->st_ra, yaadj, sizeof(double) * nra, cudaMemcpyHostToDevice, c->st));
     if (pi) CUDA_TRY(cudaMemcpyAsync(c->st_pi, pi, sizeof(double) * ngm, cudaMemcpyHostToDevice, c->st));
     CUDA_TRY(sweep_set_state(c->D, chain, c->st_g, c->st_cls, c->st_vs, c->st_r, c->st_ra, pi ? c->st_pi : nullptr,
                              scalars[0], scalars[1], scalars[2], (int)scalars[3], c->st));

@@ -301,10 +301,11 @@ int sodagpu_profile_kernels(sodagpu_ctx *ctx, int32_t iters, double *ms, int32_t
  * looked up for that device: after a reset, do not call this again on that
  * device in the same process.  The columns are summed in sodagpu_predict's
  * splits while nind times their number fits the scratch, in fewer above that
- * (the last bits may differ then).  Codes outside 0..2 count as 1 (a missing call, utilities.f90:446-449), where
- * sodagpu_predict returns SODAGPU_E_ARG.  Errors are reported by the return
- * code only (sodagpu_last_error is not updated); a launch error the caller
- * left pending is neither reported nor cleared. */
+ * (the last bits may differ then).  Codes outside 0..2 count as 1 (a missing
+ * call, utilities.f90:446-449), where sodagpu_predict returns SODAGPU_E_ARG.
+ * Errors are reported by the return code only (sodagpu_last_error is not
+ * updated); a launch error the caller left pending is neither reported nor
+ * cleared. */
 #define SODAGPU_NOALLOC_SCRATCH (2 * 1024 * 1024)
 int sodagpu_compute_dgv_noalloc(int32_t nind, int32_t nloci, const int8_t *codes, int32_t ldg,
                                 const double *freq, double mu, const double *effects, double *pred,

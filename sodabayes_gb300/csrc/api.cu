@@ -697,7 +697,10 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
                 CUDA_TRY(cudaMemcpyAsync(&h_rank, rank, sizeof(int32_t), cudaMemcpyDeviceToHost, c->st));
                 CUDA_TRY(cudaMemcpyAsync(&h_pst, pst, sizeof(int32_t), cudaMemcpyDeviceToHost, c->st));
                 CUDA_TRY(cudaMemcpyAsync(hpiv.data(), piv, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, c->st));
+                CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
                 CUDA_TRY(cudaStreamSynchronize(c->st));
+                // first: the rank and the status of a Gram that gave up mean nothing
+                if (h_err) return fail(SODAGPU_E_TIMEOUT, "a bounded device wait of the pivoted fallback gave up");
                 if (h_pst != 0) return fail(SODAGPU_E_NOTPSD, "subset %d: d*I - X'X is not positive semidefinite", b + 1);
                 for (int j = h_rank; j < N; ++j) {
                     const int jj = hpiv[j] - 1;

@@ -29,7 +29,8 @@ namespace {   // each translation unit that includes this has kernels of its own
 
 enum { DGV_PADDED = 0, DGV_RAW = 1, DGV_BED = 2 };
 
-constexpr int DGV_GROUP = 5, DGV_TAB = 243;     // SNPs per table, its entries
+constexpr int DGV_GROUP = 5;                    // SNPs per table of 3^5 = 243 sums
+constexpr int DGV_TAB = 256;                    // its entries: codes that the caller is about to refuse index up to 255
 constexpr int DGV_CHUNK = 8;                    // tables built at a time
 constexpr int DGV_SUB = 24 * DGV_CHUNK * DGV_GROUP;   // SNPs that share a fixed-point unit
 
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
               const double *eff, int n, int p, int per, double *part, size_t ldp)
 {
     __shared__ double s_w[DGV_SUB];                         // w, then the same slot in fixed point
-    __shared__ long long s_t[DGV_CHUNK][DGV_TAB + 1];
+    __shared__ long long s_t[DGV_CHUNK][DGV_TAB];
     __shared__ double sh[NT / 32][2], s_c[3];
     long long *s_f = reinterpret_cast<long long *>(s_w);
     constexpr int PF = SRC == DGV_BED ? 2 : (W == 1 ? 4 : 1);

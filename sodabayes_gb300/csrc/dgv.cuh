@@ -149,7 +149,10 @@ __device__ __forceinline__ void dgv_coef(const double *xv, const double *freq, c
         return;
     }
     const double f = freq[k], eps = 2.220446049250313e-16;
-    if (f < eps || (1.0 - f) < eps) return;
+    if (f < eps || (1.0 - f) < eps) {
+        w = x0e = 0.0 * e;   // NaN for an effect that is not finite, which takes the sub-range to the plain sum
+        return;
+    }
     const double twop = __dmul_rn(2.0, f);
     w = e / sqrt(__dmul_rn(twop, __dsub_rn(1.0, f)));
     x0e = -(twop * w);

@@ -1,0 +1,67 @@
+"""Genomic values where the centring matters (dgv.cuh): effects that are not finite
+at SNPs that are monomorphic in the frequencies given, through the three entry
+points that centre by frequencies and the one that has its own table."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import sodabayes_gb300 as sg
+from sodabayes_gb300 import JobOptions, SodaJob, make_config
+
+pytestmark = pytest.mark.gpu
+
+
+def _bed(codes):
+    n, p = codes.shape
+    c = np.zeros((p, (n + 3) // 4 * 4), dtype=np.uint8)
+    c[:, :n] = np.array([0, 2, 3], dtype=np.uint8)[codes.T]
+    c = c.reshape(p, -1, 4)
+    return c[..., 0] | c[..., 1] << 2 | c[..., 2] << 4 | c[..., 3] << 6
+
+
+def _noalloc(lib, codes, freq, eff, mu):
+    import torch
+    n, p = codes.shape
+    d = torch.from_numpy(np.ascontiguousarray(codes.T)).cuda()
+    f, e = torch.from_numpy(freq).cuda(), torch.from_numpy(eff).cuda()
+    out = torch.full((n,), 7.0, dtype=torch.float64, device="cuda")
+    rc = lib.sodagpu_compute_dgv_noalloc(n, p, C.c_void_p(d.data_ptr()), n, C.c_void_p(f.data_ptr()), float(mu),
+                                         C.c_void_p(e.data_ptr()), C.c_void_p(out.data_ptr()), None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _all(lib, codes, freq, eff, mu):
+    """The three entry points that centre by allele frequencies."""
+    yield sg.predict(codes=codes, freq=freq, mu=mu, effects=eff)
+    yield sg.predict(bed=_bed(codes), nind=codes.shape[0], freq=freq, mu=mu, effects=eff)
+    yield _noalloc(lib, codes, freq, eff, mu)
+
+
+def _job(codes):
+    n, p = codes.shape
+    job = SodaJob(make_config(n, p, JobOptions(method="BayesC", pi=0.9, blocksize=max(2, p // 3), seed=1)))
+    job.load_genotypes(codes)
+    job.build_z()
+    return job
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("f", [0.0, 1.0])
+def test_non_finite_effect_of_a_monomorphic_snp(gpu_lib, value, f):
+    """x = 0 there, and 0 times such an effect is not a number: everyone's value is NaN."""
+    rng = np.random.default_rng(4)
+    codes = np.asfortranarray(rng.binomial(2, 0.4, size=(50, 30)).astype(np.int8))
+    codes[:, 11] = int(2 * f)
+    freq = codes.mean(axis=0) / 2.0
+    eff = rng.standard_normal(30)
+    eff[11] = value
+    for got in _all(gpu_lib, codes, freq, eff, 1.0):
+        assert np.all(np.isnan(got))
+    with _job(codes) as job:
+        assert np.all(np.isnan(job.compute_dgv(1.0, eff)))
+    eff[11] = 1e300     # a finite one adds nothing
+    for got in _all(gpu_lib, codes, freq, eff, 1.0):
+        assert np.all(np.isfinite(got))

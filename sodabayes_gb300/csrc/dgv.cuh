@@ -5,17 +5,23 @@
 // are 1.6 ms of additions alone, and byte-wide loads with a dependent table lookup each took 4.1 ms).  So the
 // additions are integer, and there is one for every five SNPs:
 //   * w_k = effect_k / sd_k becomes a 64-bit fixed-point number.  The unit of a sub-range of at most DGV_SUB SNPs
-//     is 2^(E-62) with 4 * sum |w| < 2^E, so no sum overflows and all of them are exact; the rounding of each w is
-//     at most 2^-63 of that sum, below the 2^-53 of the running FP64 sum that a chain of additions makes at every
-//     term.  The constant sum_k x0_k effect_k of a sub-range is added in FP64 by a tree.
+//     is 2^(E-62) with 4 * sum |w| < 2^E <= 8 * sum |w|, so no sum overflows and all of them are exact; the rounding
+//     of each w is at most 2^-60 of that sum, below the 2^-53 of the running FP64 sum that a chain of additions makes
+//     at every term.
+//   * the value of a code is (code - 2 f) / sd.  With m the code nearest to 2 f it is split into (code - m) w, summed in
+//     integers (the constant sum m_k w_k is one more of them, subtracted at the end), and (m - 2 f) w, which is the
+//     same for everyone: their sum over a sub-range is added in FP64 by a tree.  Where one allele is common, code - 2 f
+//     is near 0 for nearly everyone, and with 2 f w in place of (m - 2 f) w the two sums would cancel (n = 20,000,
+//     f = 1 - 1 / (2 n): 1e-12 of the value).
 //   * five SNPs' codes (0..2) make a base-3 index below 243, computed for four individuals at once in the bytes of
 //     a word (w0 + 3 w1 + 9 w2 + 27 w3 + 81 w4, no carries), into a table of the group's 243 sums in shared
 //     memory.  Per five SNPs and individual: one 8-byte shared load and one 64-bit integer addition.
 // The kernel is then bound by the codes' bandwidth and the shared-memory lookups (4.6 wavefronts a warp, bank
 // conflicts included) together.  Measured: n = 20,000, p = 50,000, a job's int8 codes 189 us, 5.3 TB/s (4055 us
 // before); a .bed payload, n = 4,999, p = 50,000, 143 us (1216 us after its expansion to bytes); the caller's codes
-// at n = 1,001, p = 5,003 in 14 us (36 us).  Against 64-bit arithmetic elsewhere the relative error is 2.5e-16 to
-// 5e-16 (3.8e-16 to 1.4e-15 before).
+// at n = 1,001, p = 5,003 in 14 us (36 us).  Against 113-bit arithmetic (n = 300 to 1,001, p = 4,000 to 20,000) the
+// relative error is 2.5e-16 (rms; 3.2e-16 by frequencies and 4.3e-16 by the table with 2 f w, 6.2e-16 as a chain of
+// FP64 additions).
 //
 // Sub-ranges whose effects are not finite, or whose sum of |w| lies outside 1e-280..1e280, take one FP64 addition
 // a genotype, as every sub-range did: an infinite or NaN effect gives what the plain sum gives.
@@ -133,29 +139,37 @@ __device__ __forceinline__ uint32_t dgv_codes(const DgvLoad<SRC, W> &r, int j, u
     }
 }
 
-// Effect of SNP k, w = effect / sd (0 for monomorphic SNPs) and 2 f: the value of a code is (code - 2 f) / sd
-// (xscale, utilities.f90:525-534, 545-552).  From a centring table, or from the allele frequency.
+// SNP k: w = effect / sd (0 for monomorphic SNPs), the code m nearest to 2 f, and xme, the value of that code times the
+// effect: the value of a code is (code - 2 f) / sd (xscale, utilities.f90:525-534, 545-552).  From a centring table, or
+// from the allele frequency.
 __device__ __forceinline__ void dgv_coef(const double *xv, const double *freq, const int32_t *perm,
-                                         const double *eff, int k, double &w, double &x0e)
+                                         const double *eff, int k, double &w, double &xme, unsigned &m)
 {
     const double e = eff[perm ? perm[k] : k];
-    w = x0e = 0.0;
+    w = xme = 0.0;
+    m = 0;
     if (e == 0.0) return;
     if (xv) {
         const double2 lo = *reinterpret_cast<const double2 *>(xv + (size_t)k * 4);
         const double2 hi = *reinterpret_cast<const double2 *>(xv + (size_t)k * 4 + 2);
         w = hi.y * e;
-        x0e = lo.x * e;
+        // the value of least magnitude, by the upper words: an FP64 comparison takes the narrow pipe 64 cycles a warp
+        const int h0 = __double2hiint(lo.x) & 0x7FFFFFFF, h1 = __double2hiint(lo.y) & 0x7FFFFFFF;
+        const int h2 = __double2hiint(hi.x) & 0x7FFFFFFF;
+        m = h0 < h1 ? 0 : (h2 < h1 ? 2 : 1);
+        xme = (m == 0 ? lo.x : (m == 1 ? lo.y : hi.x)) * e;
         return;
     }
     const double f = freq[k], eps = 2.220446049250313e-16;
     if (f < eps || (1.0 - f) < eps) {
-        w = x0e = 0.0 * e;   // NaN for an effect that is not finite, which takes the sub-range to the plain sum
+        w = xme = 0.0 * e;   // NaN for an effect that is not finite, which takes the sub-range to the plain sum
         return;
     }
     const double twop = __dmul_rn(2.0, f);
     w = e / sqrt(__dmul_rn(twop, __dsub_rn(1.0, f)));
-    x0e = -(twop * w);
+    const int h = __double2hiint(twop);   // 1/2 and 3/2: the upper words 0x3FE00000 and 0x3FF80000
+    m = h < 0x3FE00000 ? 0 : (h < 0x3FF80000 ? 1 : 2);
+    xme = __dsub_rn(m == 0 ? 0.0 : (m == 1 ? 1.0 : 2.0), twop) * w;
 }
 
 // A sub-range outside the fixed-point range: the plain sum of one individual, one FP64 addition a genotype.
@@ -198,6 +212,8 @@ __global__ void __launch_bounds__(NT, 512 / NT)
     __shared__ double s_w[DGV_SUB];                         // w, then the same slot in fixed point
     __shared__ long long s_t[DGV_CHUNK][DGV_TAB];
     __shared__ double sh[NT / 32][2], s_c[3];
+    __shared__ uint8_t s_near[DGV_SUB];                     // m
+    __shared__ long long s_m[NT / 32];                      // the warps' sums of m w
     long long *s_f = reinterpret_cast<long long *>(s_w);
     constexpr int PF = SRC == DGV_BED ? 2 : (W == 1 ? 4 : 1);
     static_assert(DGV_CHUNK % PF == 0, "a chunk's tables serve whole rounds of the ring");
@@ -225,15 +241,17 @@ __global__ void __launch_bounds__(NT, 512 / NT)
         };
 #pragma unroll
         for (int q = 0; q < PF; ++q) fetch(ring[q], q);
-        // the sums of w's magnitude and of x0 e over the warps that hold SNPs, then one thread: every FP64
+        // the sums of w's magnitude and of xme over the warps that hold SNPs, then one thread: every FP64
         // instruction of a warp takes the pipe 16 cycles
         __syncthreads();
         const int warps = min(NT, padded + 31) / 32;
         for (int q = tid; q < padded; q += NT) {
-            double w = 0.0, x0e = 0.0;
-            if (q < cnt) dgv_coef(xv, freq, perm, eff, k0 + q, w, x0e);
+            double w = 0.0, xme = 0.0;
+            unsigned m = 0;
+            if (q < cnt) dgv_coef(xv, freq, perm, eff, k0 + q, w, xme, m);
             s_w[q] = w;
-            base += x0e;
+            s_near[q] = (uint8_t)m;
+            base += xme;
             mag += fabs(w);
         }
         if ((tid >> 5) < warps) {
@@ -272,14 +290,30 @@ __global__ void __launch_bounds__(NT, 512 / NT)
             }
             continue;
         }
-        for (int q = tid; q < padded; q += NT) s_f[q] = __double2ll_rn(s_w[q] * scale);
+        long long msum = 0;
+        for (int q = tid; q < padded; q += NT) {
+            const long long f = __double2ll_rn(s_w[q] * scale);
+            const unsigned m = s_near[q];
+            s_f[q] = f;
+            msum += (m & 1u ? f : 0) + (m & 2u ? f << 1 : 0);
+        }
+        if ((tid >> 5) < warps) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) msum += __shfl_xor_sync(0xffffffffu, msum, o);
+            if (lane == 0) s_m[tid >> 5] = msum;
+        }
+        __syncthreads();   // s_f and s_m are complete
+        // the sums start at the constant: subtracted at the end, in registers that live through the loop, it cost the
+        // 256-thread kernel a tenth
+        long long centre = 0;
+        for (int w = 0; w < warps; ++w) centre += s_m[w];
         long long acc[4 * W];
 #pragma unroll
-        for (int j = 0; j < 4 * W; ++j) acc[j] = 0;
+        for (int j = 0; j < 4 * W; ++j) acc[j] = -centre;
 #pragma unroll 1
         for (int g0 = 0; g0 < groups; g0 += PF) {
             if (g0 % DGV_CHUNK == 0) {
-                __syncthreads();   // s_f is complete, and every lookup in the previous chunk's tables is done
+                if (g0 > 0) __syncthreads();   // every lookup in the previous chunk's tables is done
 #pragma unroll 1
                 for (int h = tid >> 5; h < DGV_CHUNK; h += NT / 32) {
                     const long long *f = s_f + DGV_GROUP * (g0 + h);

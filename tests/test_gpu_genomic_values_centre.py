@@ -1,6 +1,14 @@
-"""Genomic values where the centring matters (dgv.cuh): effects that are not finite
-at SNPs that are monomorphic in the frequencies given, through the three entry
-points that centre by frequencies and the one that has its own table."""
+"""Genomic values where the centring matters (dgv.cuh): SNPs whose counted allele
+is common, so that code - 2 f is near 0 for nearly everyone, and effects that
+are not finite at SNPs that are monomorphic in the frequencies given, through
+the three entry points that centre by frequencies and the one that has its own
+table.
+
+Reference: mu + sum x_k e_k in numpy FP64 with x = (code - 2 f) / sd.  Each side
+rounds every x_k e_k a few times and adds p terms, so for each individual they
+agree to 4 (p + 16) eps times the sum of its |x_k e_k| (Higham, Accuracy and
+Stability of Numerical Algorithms, section 4.2), and the fixed-point weights
+add 2^-60 of the sum of the |e_k / sd_k|."""
 import ctypes as C
 
 import numpy as np
@@ -10,6 +18,8 @@ import sodabayes_gb300 as sg
 from sodabayes_gb300 import JobOptions, SodaJob, make_config
 
 pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(float).eps
 
 
 def _bed(codes):
@@ -46,6 +56,26 @@ def _job(codes):
     job.load_genotypes(codes)
     job.build_z()
     return job
+
+
+@pytest.mark.parametrize("n,p", [(300, 7), (1500, 41), (20000, 1000)])
+def test_a_common_allele_does_not_cost_precision(gpu_lib, n, p):
+    rng = np.random.default_rng(n + p)
+    codes = np.full((n, p), 2, dtype=np.int8, order="F")
+    for j in range(p):      # one to three other calls in n; every third SNP has the other allele common instead
+        codes[rng.choice(n, size=1 + j % 3, replace=False), j] = 1
+        if j % 3 == 2:
+            codes[:, j] = 2 - codes[:, j]
+    freq = codes.mean(axis=0) / 2.0
+    eff = rng.standard_normal(p)
+    sd = np.sqrt(2.0 * freq * (1.0 - freq))
+    terms = (codes - 2.0 * freq) / sd * eff
+    want = terms.sum(axis=1)
+    tol = 4.0 * (p + 16) * EPS * np.abs(terms).sum(axis=1) + 2.0 ** -60 * np.abs(eff / sd).sum()
+    for got in _all(gpu_lib, codes, freq, eff, 0.0):
+        assert np.all(np.abs(got - want) <= tol)
+    with _job(codes) as job:
+        assert np.all(np.abs(job.compute_dgv(0.0, eff) - want) <= tol)
 
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])

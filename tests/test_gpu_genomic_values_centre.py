@@ -95,3 +95,32 @@ def test_non_finite_effect_of_a_monomorphic_snp(gpu_lib, value, f):
     eff[11] = 1e300     # a finite one adds nothing
     for got in _all(gpu_lib, codes, freq, eff, 1.0):
         assert np.all(np.isfinite(got))
+
+
+@pytest.mark.parametrize("where", [0, 500, 959, 960, 1009])
+@pytest.mark.parametrize("value", [1e290, np.inf])
+def test_sub_ranges_of_both_kinds_in_one_split(gpu_lib, where, value):
+    """More individuals than the scratch has room for two splits of: one split of a sub-range of 960 SNPs and one of 50,
+    of which the one with the large effect is summed in FP64."""
+    import torch
+    n, p = 1100000, 1010
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    g = torch.randint(0, 3, (p, n), dtype=torch.int8, device="cuda", generator=gen)
+    freq = np.full(p, 0.45)
+    eff = np.random.default_rng(6).standard_normal(p)
+    eff[where] = value
+    f, e = torch.from_numpy(freq).cuda(), torch.from_numpy(eff).cuda()
+    out = torch.full((n,), 7.0, dtype=torch.float64, device="cuda")
+    rc = gpu_lib.sodagpu_compute_dgv_noalloc(n, p, C.c_void_p(g.data_ptr()), n, C.c_void_p(f.data_ptr()), 0.0,
+                                             C.c_void_p(e.data_ptr()), C.c_void_p(out.data_ptr()), None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    rows = np.concatenate([np.arange(0, 200), np.arange(4000, 4200), np.arange(n - 300, n)])
+    codes = g[:, torch.from_numpy(rows).cuda()].cpu().numpy().T
+    got = out.cpu().numpy()[rows]
+    terms = (codes - 2.0 * freq) / np.sqrt(2.0 * freq * (1.0 - freq)) * eff
+    want = terms.sum(axis=1)
+    if np.isinf(value):
+        assert np.array_equal(got, want)
+    else:
+        assert np.all(np.abs(got - want) <= 4.0 * (p + 16) * EPS * np.abs(terms).sum(axis=1))

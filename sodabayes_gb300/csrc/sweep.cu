@@ -1108,8 +1108,10 @@ __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
     } else if (warp >= 2 && (m == SODAGPU_BAYES_CPI || m == SODAGPU_BAYES_R || m == SODAGPU_BAYES_RC)) {
         // pi ~ Dirichlet(counts + alpha) of each group (models.f90:517-522).  The nm gamma variates of a group come from
         // one stream, one after another, 5 us each; nearly always each takes exactly three uniforms, so nm lanes draw
-        // them at once from those places, and where one but the last took more, its group's first lane draws them in turn
+        // them at once from those places, and where one but the last took more, its group's first lane draws them in
+        // turn.  From an injected-draw tape always in turn: a guessed place could run past a record that is long enough
         const int per = 32 / nm, sub = lane / nm, j = lane - sub * nm, first = sub * nm;
+        const bool guess = D.tape == nullptr;
         for (int i0 = (warp - 2) * per; i0 < ng; i0 += (NW - 2) * per) {
             const int i = i0 + sub;
             const bool in = sub < per && i < ng;
@@ -1118,13 +1120,13 @@ __device__ __forceinline__ void hyper_body(const Dev &D, const VB &vb)
             gam.taken = 3;
             double x = 0.0;
             int gerr = 0;
-            if (in) {
+            if (in && guess) {
                 crng_site(R, D, c, rep, i, P_PI);
                 crng_skip(R, 3 * j);
                 gam = gamma_pre<double>((double)S->snpindist[i + j * ng] + D.alpha[j], R, &gerr);
                 x = gamma_from(1.0, gam);
             }
-            const unsigned odd = __ballot_sync(0xffffffffu, in && j < nm - 1 && gam.taken != 3);
+            const unsigned odd = __ballot_sync(0xffffffffu, in && (!guess || (j < nm - 1 && gam.taken != 3)));
             const bool redo = in && (odd >> first & ((1u << nm) - 1u)) != 0;
             double y[MAXDIST];
             if (redo) {

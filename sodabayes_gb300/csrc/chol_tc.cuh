@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
             int issued = 0;
             for (int s = 0; s < ns; ++s) {
                 const int sl = s % CH_NS;
-                if (s >= CH_NS && !tc::mbar_wait(&s_free[sl], ((s / CH_NS) - 1) & 1)) {
+                if (s >= CH_NS && !tc::mbar_wait(&s_free[sl], ((s / CH_NS) - 1) & 1, tc::BUILD_WAIT_NS)) {
                     s_err = 1;
                     break;
                 }
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
             }
             // no copy may still be in flight into this CTA's shared memory when it exits
             for (int s = max(0, issued - CH_NS); s < issued; ++s)
-                if (!tc::mbar_wait(&s_full[s % CH_NS], (s / CH_NS) & 1)) s_err = 1;
+                if (!tc::mbar_wait(&s_full[s % CH_NS], (s / CH_NS) & 1, tc::BUILD_WAIT_NS)) s_err = 1;
         }
     } else if (warp == 9) {
         const bool leader = tc::elect_one();
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         for (int s = 0; s < ns && ok; ++s) {
             const int sl = s % CH_NS;
             const bool first = s % CH_GROUP == 0;
-            if (first && s > 0) ok = tc::mbar_wait(&s_read, (s / CH_GROUP - 1) & 1);   // the last group is drained
-            ok = ok && tc::mbar_wait(&s_full[sl], (s / CH_NS) & 1);
+            if (first && s > 0) ok = tc::mbar_wait(&s_read, (s / CH_GROUP - 1) & 1, tc::BUILD_WAIT_NS);   // the last group is drained
+            ok = ok && tc::mbar_wait(&s_full[sl], (s / CH_NS) & 1, tc::BUILD_WAIT_NS);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 s_err = 1;
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         for (int c = 0; c < CH_P / 2; ++c) acc[c] = 0;
         const uint32_t ta = tm + ((uint32_t)(32 * qd) << 16) + h * (CH_P / 2);
         for (int g = 0; g < ngr; ++g) {
-            bool ok = tc::mbar_wait(&s_done, g & 1);
+            bool ok = tc::mbar_wait(&s_done, g & 1, tc::BUILD_WAIT_NS);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 s_err = 1;

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
             int issued = 0;
             for (int s = 0; s < ns; ++s) {
                 const int sl = s % GR_NS;
-                if (s >= GR_NS && !tc::mbar_wait(&s_free[sl], ((s / GR_NS) - 1) & 1)) {
+                if (s >= GR_NS && !tc::mbar_wait(&s_free[sl], ((s / GR_NS) - 1) & 1, tc::BUILD_WAIT_NS)) {
                     s_err = 1;
                     break;
                 }
@@ -96,14 +96,14 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
             }
             // no copy may still be in flight into this CTA's shared memory when it exits
             for (int s = max(0, issued - GR_NS); s < issued; ++s)
-                if (!tc::mbar_wait(&s_full[s % GR_NS], (s / GR_NS) & 1)) s_err = 1;
+                if (!tc::mbar_wait(&s_full[s % GR_NS], (s / GR_NS) & 1, tc::BUILD_WAIT_NS)) s_err = 1;
         }
     } else if (warp == 5) {
         const bool leader = tc::elect_one();
         const uint32_t idesc = tc::idesc_e4m3(GR_T, GR_T);
         for (int s = 0; s < ns; ++s) {
             const int sl = s % GR_NS;
-            if (!__all_sync(0xffffffffu, tc::mbar_wait(&s_full[sl], (s / GR_NS) & 1))) {
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(&s_full[sl], (s / GR_NS) & 1, tc::BUILD_WAIT_NS))) {
                 s_err = 1;
                 break;
             }
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
             s_inv[tid] = c.inv;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (!tc::mbar_wait(&s_done, 0, 1000000000ull)) s_err = 1;   // every stage: up to 32,768
+        if (!tc::mbar_wait(&s_done, 0, tc::BUILD_WAIT_NS)) s_err = 1;   // every stage: up to 32,768
         tc::fence_after_sync();
         double *Wb = W + wofs[b];
         float *Fb = W32 ? W32 + blockIdx.y * stride32 : nullptr;

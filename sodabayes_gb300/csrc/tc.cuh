@@ -113,6 +113,10 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
     return t;
 }
 
+// The limit of the Z build's waits: a process that the GPU takes away for the time slices of others in the middle of one
+// must not lose its set-up (20 ms is a few slices), and nothing else waits for these kernels.
+constexpr uint64_t BUILD_WAIT_NS = 1000000000ull;
+
 // Bounded wait for the phase with the given parity: false once `limit_ns`
 // (default 20 ms; phases complete within microseconds) has passed.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns = 20000000ull)

@@ -221,9 +221,11 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     }
 }
 
-// 1 / sqrt(p) and sqrt(p) from an FP32 seed and one third-order step (FP64's own square root and division are twenty
-// dependent instructions on the critical path of every pivot, 64 cycles each); each result is off by at most a unit in
-// the last place.
+// 1 / sqrt(p) and sqrt(p) from an FP32 seed, one third-order step of Householder's method (The Numerical Treatment of a
+// Single Nonlinear Equation, 1970: the binomial series of (1 - e)^-1/2 to e^2) and, for the root, a correction by its
+// exact remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990).  FP64's own square root and division lie on the critical path of every pivot, where a dependent
+// instruction takes 64 cycles.  The root is off by at most a unit in the last place, 1 / sqrt(p) by at most two.
 __device__ __forceinline__ void ch_rsqrt(double p, double &inv, double &root)
 {
     if (!(p > 1e-30 && p < 1e30)) {
@@ -237,7 +239,7 @@ __device__ __forceinline__ void ch_rsqrt(double p, double &inv, double &root)
     const double r = p * inv;
     root = fma(0.5 * inv, fma(-r, r, p), r);
 }
-// c / root with inv = 1 / root
+// c / root with inv = 1 / root, corrected by its exact remainder (Markstein): at most a unit in the last place off.
 __device__ __forceinline__ double ch_div(double c, double root, double inv)
 {
     const double x = c * inv;

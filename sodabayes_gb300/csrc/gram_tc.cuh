@@ -27,7 +27,8 @@ constexpr int GR_NMAX = 1 << 22;             // individuals: 4 n <= 2^24
 
 // res = (S - n pa pb) / sqrt(pa qa pb qb) for the SNP pair (a, b), a the later position, 0 where one is
 // monomorphic; p = 2 f, q = 1 - f.  The quotient by the product of the two standard deviations is formed from their
-// reciprocals with one correction step (a division is twenty FP64 instructions).
+// reciprocals with one correction by its exact remainder (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): a division an element would take longer than everything else.
 struct GramCol {
     double p, np, sd, inv;
 };
@@ -41,6 +42,13 @@ __device__ __forceinline__ GramCol gram_col(double f, int n)
     c.sd = mono ? 0.0 : sqrt(__dmul_rn(c.p, q));
     c.inv = mono ? 0.0 : 1.0 / c.sd;
     return c;
+}
+
+// num / (sda sdb) from inva = 1 / sda and invb = 1 / sdb, 0 where these are 0; off by at most a unit in the last place.
+__device__ __forceinline__ double gram_quot(double num, double sda, double sdb, double inva, double invb)
+{
+    const double r = inva * invb, den = sda * sdb, q = num * r;
+    return fma(fma(-q, den, num), r, q);
 }
 
 __global__ void __launch_bounds__(GR_THREADS, 2)
@@ -146,9 +154,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
                 const int k = k0 + e;
                 if (j >= N || k >= N || k < j) continue;
                 const double num = __dsub_rn((double)(v[e] * 262144.0f), __dmul_rn(s_np[8 * g + e], row.p));
-                const double r = row.inv * s_inv[8 * g + e], den = row.sd * s_sd[8 * g + e];
-                double res = num * r;
-                res = fma(fma(-res, den, num), r, res);
+                const double res = gram_quot(num, row.sd, s_sd[8 * g + e], row.inv, s_inv[8 * g + e]);
                 Wb[(size_t)j + (size_t)k * N] = res;
                 Wb[(size_t)k + (size_t)j * N] = res;
                 if (Fb) {

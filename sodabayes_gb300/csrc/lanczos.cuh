@@ -10,7 +10,7 @@
 // exchange their partial dot products through distributed shared memory; on one SM the dot products alone were 110 us
 // of its FP64 pipe).  Measured, 10 subsets of 2000 SNPs (n = 20,000, LD blocks): 128 FP32 steps of 32 +
 // 21 us and 40 FP64 steps of 84 + 27 us, 11.4 ms, against 46.7 ms for 112 FP64 steps of 279 + 139 us.  The eigenvalue
-// is off by 1.8e-16 (relative rms over 64 subsets; 1.3e-16 from a random start: both below one unit in the last place).
+// is off by 1.25e-16 (relative rms, 44 subsets of 96 to 1000 SNPs; 1.33e-16 from a random start).
 #pragma once
 #include <cooperative_groups.h>
 #include "rng.cuh"
@@ -140,11 +140,39 @@ __global__ void __launch_bounds__(LZ_THREADS)
     }
 }
 
+// Sums in twice the working precision (Dekker, "A floating-point technique for extending the available precision",
+// Numer. Math. 18, 1971; Ogita, Rump and Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput. 26, 2005).
+struct LzSum {
+    double hi, lo;
+};
+__device__ __forceinline__ LzSum lz_plus(LzSum a, double hi, double lo)
+{
+    const double s = __dadd_rn(a.hi, hi), t = __dsub_rn(s, a.hi);
+    const double e = __dadd_rn(__dsub_rn(a.hi, __dsub_rn(s, t)), __dsub_rn(hi, t));
+    return {s, a.lo + lo + e};
+}
+__device__ __forceinline__ LzSum lz_plus_product(LzSum a, double x, double y)
+{
+    const double q = __dmul_rn(x, y);
+    return lz_plus(a, q, fma(x, y, -q));
+}
+__device__ __forceinline__ LzSum lz_warp_sum(LzSum a)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        a = lz_plus(a, __shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o));
+    return a;
+}
+
 // Two classical Gram-Schmidt passes of w = A v_j against v_0 .. v_j (the first pass's coefficient of v_j is
 // alpha_j; a single pass is not stable: in FP32 the vectors lose their orthogonality within 40 steps), beta_j = |w|
 // and v_{j+1} = w / beta_j.  CTA r of the cluster holds elements r * sl .. of the vectors; sums
 // over the cluster are added in rank order.  Bound by the exchanges (a cluster barrier and a remote read, about 2 us
 // together): one a pass, one for the norm.
+//
+// v_0 of the FP64 run holds nearly all of the eigenvector, and alpha_0 = v_0'A v_0 nearly all of the eigenvalue: the
+// rounding of that one sum, and of |v_0|^2 which is 1 only to rounding, would be the eigenvalue's.  So alpha_0 is the
+// quotient of both, summed in twice the precision.
 template <typename T>
 __global__ void __cluster_dims__(LZ_CTAS, 1, 1) __launch_bounds__(LZ_THREADS)
     k_lz_orth(const int32_t *blk_ls, const int32_t *batch_blocks, size_t vstride, T *V, const T *wpart, int nsp, int ldw,
@@ -155,6 +183,8 @@ __global__ void __cluster_dims__(LZ_CTAS, 1, 1) __launch_bounds__(LZ_THREADS)
     constexpr int NW = LZ_THREADS / 32, PASSES = 2;
     extern __shared__ __align__(16) unsigned char lz_smem[];
     __shared__ T s_nrm[NW];
+    __shared__ LzSum s_q[2];                        // this CTA's parts of v_0'w and v_0'v_0
+    const bool quotient = sizeof(T) == 8 && j == 0;
     const int bi = blockIdx.x / LZ_CTAS, rank = (int)cl.block_rank();
     const int b = batch_blocks[bi];
     const int N = blk_ls[b + 1] - blk_ls[b], sl = (N + LZ_CTAS - 1) / LZ_CTAS;
@@ -192,11 +222,28 @@ __global__ void __cluster_dims__(LZ_CTAS, 1, 1) __launch_bounds__(LZ_THREADS)
             for (int q = 0; q < 4; ++q) s[q] = lz_warp_sum(s[q]);
             if (lane < 4 && t + lane <= j) h[t + lane] = lane == 0 ? s[0] : (lane == 1 ? s[1] : (lane == 2 ? s[2] : s[3]));
         }
+        if (quotient && pass == 0 && warp < 2) {
+            LzSum s = {0.0, 0.0};
+            for (int i = lane; i < cnt; i += 32) s = lz_plus_product(s, (double)Vb[i], warp == 0 ? (double)w[i] : (double)Vb[i]);
+            s = lz_warp_sum(s);
+            if (lane == 0) s_q[warp] = s;
+        }
         cl.sync();
         for (int t = tid; t <= j; t += LZ_THREADS) {
             T s = (T)0.0;
 #pragma unroll
             for (int q = 0; q < LZ_CTAS; ++q) s += cl.map_shared_rank(h, q)[t];
+            if (quotient && pass == 0) {
+                LzSum x[2] = {{0.0, 0.0}, {0.0, 0.0}};
+                for (int q = 0; q < LZ_CTAS; ++q)
+                    for (int k = 0; k < 2; ++k) {
+                        const LzSum r = cl.map_shared_rank(s_q, q)[k];
+                        x[k] = lz_plus(x[k], r.hi, r.lo);
+                    }
+                // (hi + lo) / (hi' + lo') with hi' near 1
+                const double n = x[1].hi + x[1].lo, a0 = x[0].hi / n;
+                s = (T)(a0 + ((fma(-a0, n, x[0].hi) + x[0].lo) - a0 * (x[1].hi - n + x[1].lo)) / n);
+            }
             s_ht[t] = s;
         }
         __syncthreads();
@@ -315,15 +362,8 @@ __global__ void __launch_bounds__(1024)
         }
         nn = lz_block_sum(nn, sh);
     }
-    double inv = 1.0 / sqrt(nn);
+    const double inv = 1.0 / sqrt(nn);   // (what rounding leaves of |v_0|^2 - 1 is no matter: alpha_0 is a quotient)
     for (int i = tid; i < N; i += 1024) v[i] *= inv;
-    // v_0 holds nearly all of the result, alpha_0 = v_0'A v_0: what the first scaling left of |v_0|^2 - 1 (the rounding
-    // of 1 / |v_0|, the same for every element) would be a relative error of lambda_max
-    nn = 0.0;
-    for (int i = tid; i < N; i += 1024) nn += v[i] * v[i];
-    nn = lz_block_sum(nn, sh);
-    inv = 0.5 * (nn - 1.0);
-    for (int i = tid; i < N; i += 1024) v[i] -= inv * v[i];
 }
 
 }  // namespace soda

@@ -1246,27 +1246,57 @@ __global__ void __launch_bounds__(256) k_post(Dev D)
 // iteration (the iteration is a captured graph) and return at once on the others, so their grids hold
 // RECAL_CTAS CTAs that walk the (rows, column split, chain) tiles: one CTA a tile cost 302 us an iteration in
 // CTA launches alone at n = 50,000 and 16 chains.
+//
+// A tile's SNPs with an effect are gathered in shared memory, 256 at a time and in order, so that the loads of their
+// codes do not wait for one another: with the effect and the centring table looked up for each SNP by each thread, the
+// loop was a chain of three loads, whose rate was the number of resident CTAs (and these are half of what
+// an SM holds).  An iteration that recalibrates takes longer by, p = 20,000: n = 50,000, one chain of BayesA: 3.7 ms;
+// n = 50,000, 4 chains, half of the effects zero: 7.1 ms; n = 20,000, 16 chains: 8.9 ms (9.7, 32.2 and 41.0 ms; 3.9, 14.9
+// and 24.0 ms with one CTA a tile).
+constexpr int RECAL_CHUNK = 256;
+
 __device__ __forceinline__ void recal_partial_body(const Dev &D, const VB &vb, int force)
 {
+    __shared__ double s_x[RECAL_CHUNK][4];   // the values of codes 0, 1, 2 and the effect
+    __shared__ int s_k[RECAL_CHUNK], s_cnt[RECAL_CHUNK / 32];
     tc::pdl_trigger();
     tc::pdl_wait();
     const int rep = cur_rep(D);
     if (!force && (D.recal <= 0 || rep % D.recal != 0)) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles = (D.n + 255) / 256, total = tiles * RECAL_SPLIT * D.chains;
     const int per = (D.p + RECAL_SPLIT - 1) / RECAL_SPLIT;
     for (int t = vb.x; t < total; t += vb.nx) {
         const int c = t / (tiles * RECAL_SPLIT), split = (t / tiles) % RECAL_SPLIT;
-        const int i = (t % tiles) * 256 + threadIdx.x;
-        if (i >= D.n) continue;
+        const int i = (t % tiles) * 256 + tid;
         const int k0 = split * per, k1 = min(D.p, k0 + per);
         double acc = 0.0;
         const double *g = D.g + (size_t)c * D.p;
-        for (int k = k0; k < k1; ++k) {
-            const double gj = g[D.perm[k]];
-            if (gj == 0.0) continue;
-            acc = acc + D.xv[(size_t)k * 4 + D.G[(size_t)k * D.ldx + i]] * gj;
+        const int8_t *col = D.G + min(i, D.n - 1);
+        for (int c0 = k0; c0 < k1; c0 += RECAL_CHUNK) {
+            const int k = c0 + tid;
+            const double gj = k < k1 ? g[D.perm[k]] : 0.0;
+            const unsigned in = __ballot_sync(0xffffffffu, gj != 0.0);
+            if (lane == 0) s_cnt[warp] = __popc(in);
+            __syncthreads();   // also: every use of the previous chunk is done
+            int at = 0, m = 0;
+#pragma unroll
+            for (int w = 0; w < RECAL_CHUNK / 32; ++w) {
+                at += w < warp ? s_cnt[w] : 0;
+                m += s_cnt[w];
+            }
+            if (gj != 0.0) {
+                at += __popc(in & ((1u << lane) - 1u));
+                s_k[at] = k;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) s_x[at][q] = D.xv[(size_t)k * 4 + q];
+                s_x[at][3] = gj;
+            }
+            __syncthreads();
+#pragma unroll 8
+            for (int q = 0; q < m; ++q) acc = acc + s_x[q][col[(size_t)s_k[q] * D.ldx]] * s_x[q][3];
         }
-        D.recal_part[((size_t)c * RECAL_SPLIT + split) * D.ldr + i] = acc;
+        if (i < D.n) D.recal_part[((size_t)c * RECAL_SPLIT + split) * D.ldr + i] = acc;
     }
 }
 

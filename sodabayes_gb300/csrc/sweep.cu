@@ -209,7 +209,8 @@ __device__ __forceinline__ void draw_ahead(const Dev &D, const ChainScal *S, con
 }
 
 // The class (1-based) for the FP64 scores b_k + c_k r2 of up to DRAW_PRE classes: the first whose cumulative weight
-// exceeds u times their sum, weights exp(s_k - s_0), or relative to the largest score where that could overflow.  (The
+// exceeds u times their sum, weights exp(s_k - s_0), or relative to the largest score where that could overflow; there a
+// class more than 700 below the largest has none, as in the reference, which matters for u = 0.  (The
 // probabilities of models.f90:366-379 one by one take up to twelve exponentials and four divisions, 16 and 10 FP64
 // instructions of 64 cycles each, in every warp with a SNP outside the first class.)
 __device__ __forceinline__ int draw_class64(double r2, const double (&b)[DRAW_PRE], const double (&c)[DRAW_PRE],
@@ -230,7 +231,7 @@ __device__ __forceinline__ int draw_class64(double r2, const double (&b)[DRAW_PR
 #pragma unroll
     for (int k = 0; k < DRAW_PRE; ++k)
         if (k < nm) {
-            w[k] = k == 0 && !big ? 1.0 : exp(w[k] - ref);
+            w[k] = k == 0 && !big ? 1.0 : (big && ref - w[k] > 700.0 ? 0.0 : exp(w[k] - ref));
             sum = sum + w[k];
         }
     const double us = u * sum;
@@ -263,9 +264,9 @@ __device__ __forceinline__ double draw_snp(const Dev &D, const ChainScal *S, int
         int flag = 2;
         if (m == SODAGPU_BAYES_A || cl > 1) rhs = rhs + zz * gk;
         if (m == SODAGPU_BAYES_B && sizeof(T) == 8) {
-            // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2))
+            // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2)), which is 0 above 700 as in the reference
             const T d = a.b[0] - (a.b[1] + a.c * (rhs * rhs));
-            flag = a.u * ((T)1.0 + t_exp(d)) < (T)1.0 ? 2 : 1;
+            flag = d <= (T)700.0 && a.u * ((T)1.0 + t_exp(d)) < (T)1.0 ? 2 : 1;
         } else if (m == SODAGPU_BAYES_B) {
             const T s1 = q.logp[0];
             const T uhat = rhs / a.den;
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(64) k_skipped_pre(Dev D, int t0, int cnt)
 
 // The class of a SNP (1-based) from its uniform u and this lane's class score s (lanes 0 .. nm-1; all 32 enter): the
 // first class whose cumulative weight exceeds u times their sum, weights exp(s_k - s_0), or relative to the largest
-// score where that could overflow.
+// score where that could overflow (draw_class64).
 __device__ __forceinline__ int skipped_class(double s, double u, int nm)
 {
     const int lane = threadIdx.x & 31;
@@ -626,7 +627,7 @@ __device__ __forceinline__ int skipped_class(double s, double u, int nm)
         double top = lane < nm ? s : -1e308;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-        w = s - top;
+        w = top - s > 700.0 ? -1e308 : s - top;
     }
     w = lane < nm ? exp(w) : 0.0;
     for (int o = 1; o < nm; o <<= 1) {
@@ -670,9 +671,12 @@ __device__ __forceinline__ SkippedDraw skipped_draw(const Dev &D, const ChainSca
     x.flag = 2;
     if (m != SODAGPU_BAYES_A) {
         const double s = lane == 0 ? cb.y : fma(rhs * rhs, cb.x, cb.y);
-        if (m == SODAGPU_BAYES_B)   // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2))
-            x.flag = u * (1.0 + exp(__shfl_sync(0xffffffffu, s, 0) - __shfl_sync(0xffffffffu, s, 1))) < 1.0 ? 2 : 1;
-        else x.flag = skipped_class(s, u, nm);
+        if (m == SODAGPU_BAYES_B) {   // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2)), 0 above 700
+            const double d = __shfl_sync(0xffffffffu, s, 0) - __shfl_sync(0xffffffffu, s, 1);
+            x.flag = d <= 700.0 && u * (1.0 + exp(d)) < 1.0 ? 2 : 1;
+        } else {
+            x.flag = skipped_class(s, u, nm);
+        }
     }
     x.upd = x.gt = 0.0;
     if (m == SODAGPU_BAYES_A || m == SODAGPU_BAYES_B) {

@@ -563,8 +563,9 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
         return fail(SODAGPU_E_CUDA, "cuTensorMapEncodeTiled failed for the genotypes");
     int *d_err = nullptr, h_err = 0;
     TRY(c->alloc(&d_err, 1));
-    // subsets at a time: at most 64, and at most 4 GB of the factorisation's digits (the FP32 copies that start the
-    // Lanczos runs are a third of that)
+    // subsets at a time: at most 64, and at most 4 GB of the factorisation's digits, or one subset's (14 N^2 bytes).  The
+    // FP32 copies that start the Lanczos runs lie in the same memory: they are done with before the first digit is
+    // written.  All of it is given back before U is allocated, so that a build takes no more at its end than W and U.
     const size_t digits = zb_chol_digits(maxN);
     const int BATCH =
         (int)std::min<size_t>({(size_t)nb, (size_t)64, std::max<size_t>(1, ((size_t)4 << 30) / (digits * 2))});
@@ -591,7 +592,7 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     uint8_t *d_done = nullptr;
     TRY(c->alloc(&V, BATCH * vstride, false));
     TRY(c->alloc(&wpart, zb_lz_wpart(maxN, BATCH), false));
-    TRY(c->alloc(&W32, (size_t)BATCH * ld32 * maxN, false));
+    W32 = reinterpret_cast<float *>(dig);   // ld32 * maxN floats a subset: less than a third of its digits
     TRY(c->alloc(&V32, (size_t)BATCH * zb_lz_pre() * maxN, false));
     TRY(c->alloc(&ab32, (size_t)2 * BATCH * zb_lz_pre(), false));
     TRY(c->alloc(&alpha, (size_t)2 * BATCH * mmax));
@@ -666,6 +667,14 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
     CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CUDA_TRY(cudaStreamSynchronize(c->st));
     if (h_err) return fail(SODAGPU_E_TIMEOUT, "a bounded device wait of the Z build gave up");
+    c->release(V);
+    c->release(wpart);
+    c->release(V32);
+    c->release(ab32);
+    c->release(alpha);
+    c->release(d_done);
+    c->release(dig);
+    c->release(cwork);
     // pivoted fallback for the subsets whose factorisation failed (soda.f90:492-510)
     std::vector<int32_t> h_iskipped;
     int naless = p;
@@ -749,19 +758,10 @@ int sodagpu_build_z(sodagpu_ctx *c, const int32_t *permvec, int32_t *nskipped_ou
         CUDA_TRY(cudaStreamSynchronize(c->st));
     }
     c->release(W);
-    c->release(V);
-    c->release(wpart);
-    c->release(W32);
-    c->release(V32);
-    c->release(ab32);
-    c->release(alpha);
     c->release(d_batch);
     c->release(d_status);
-    c->release(d_done);
     c->release(d_wofs);
     c->release(d_err);
-    c->release(dig);
-    c->release(cwork);
     TRY(c->alloc(&c->iskipped, std::max(1, c->nskipped), false));
     TRY(c->alloc(&c->xpx, p));
     if (c->nskipped)

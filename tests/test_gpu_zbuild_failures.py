@@ -1,7 +1,8 @@
 """Subsets of the Z build that fail: a device wait that gives up in the pivoted
 fallback is reported, and a subset that is not positive definite leaves the
 others of its batch alone.  Both go through the C ABI with one call replaced
-(zbuild_hooks.cu).
+(zbuild_hooks.cu).  So does the memory that a build still holds at its end, which
+decides how large a subset can be.
 
 The factors of the other subsets do not depend on the failing one: they must be
 those of the build in which none fails, bit for bit, and satisfy U'U + X'X =
@@ -27,6 +28,9 @@ def hooks(gpu_lib, tmp_path_factory):
     lib.zbuild_hooks.restype = None
     lib.zbuild_hooks.argtypes = [C.c_int, C.c_int, C.c_double]
     plain, sg._lib = sg._lib, lib
+    lib.zbuild_free.restype = C.c_uint64
+    lib.zbuild_free.argtypes = [C.c_int]
+    lib.zbuild_hooks.free = lib.zbuild_free
     yield lib.zbuild_hooks
     sg._lib = plain
 
@@ -83,3 +87,15 @@ def test_one_subset_that_is_not_positive_definite(hooks, bs, late):
         m = xb.shape[1]
         u = xa[:m, k:k + m]
         assert np.max(np.abs(u.T @ u + xb.T @ xb - xxd[b] * np.eye(m))) <= eps * (4 * m * xxd[b] + 32 * n)
+
+
+def test_memory_held_when_the_factors_are_packed(hooks):
+    """W and U, 8 bytes an element each, besides the job's own arrays (here a few MB); 64 MB cover those and what the
+    runtime keeps."""
+    hooks(0, -1, 0.0)
+    p = 4000
+    codes = _codes(150, p, 2)
+    _build(codes, p)                  # the kernels are loaded
+    free = hooks.free(1)
+    _build(codes, p)
+    assert free - hooks.free(0) <= 2 * 8 * p * p + (64 << 20)

@@ -26,11 +26,12 @@ constexpr int GR_THREADS = 192;
 constexpr int GR_NMAX = 1 << 22;             // individuals: 4 n <= 2^24
 
 // res = (S - n pa pb) / sqrt(pa qa pb qb) for the SNP pair (a, b), a the later position, 0 where one is
-// monomorphic; p = 2 f, q = 1 - f.  The quotient by the product of the two standard deviations is formed from their
-// reciprocals with one correction by its exact remainder (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): a division an element would take longer than everything else.
+// monomorphic; p = 2 f, q = 1 - f.  A division an element would take longer than everything else, so each SNP has
+// 1 / sqrt(p q) in twice the working precision (Dekker, "A floating-point technique for extending the available
+// precision", Numer. Math. 18, 1971), and a quotient is a product: two roundings, of the numerator and of the result.
+// With rounded standard deviations the diagonal was off by their rounding twice, more than the rest of it.
 struct GramCol {
-    double p, np, sd, inv;
+    double p, np, inv, lo;
 };
 __device__ __forceinline__ GramCol gram_col(double f, int n)
 {
@@ -38,17 +39,20 @@ __device__ __forceinline__ GramCol gram_col(double f, int n)
     GramCol c;
     c.p = __dmul_rn(f, 2.0);
     c.np = __dmul_rn((double)n, c.p);
-    const bool mono = f <= ep || q <= ep;
-    c.sd = mono ? 0.0 : sqrt(__dmul_rn(c.p, q));
-    c.inv = mono ? 0.0 : 1.0 / c.sd;
+    c.inv = c.lo = 0.0;
+    if (f <= ep || q <= ep) return c;
+    const double ql = __dsub_rn(__dsub_rn(1.0, q), f);   // 1 - f = q + ql
+    const double v = __dmul_rn(c.p, q), vl = fma(c.p, ql, fma(c.p, q, -v));
+    c.inv = 1.0 / sqrt(v);
+    const double s = __dmul_rn(c.inv, c.inv), sl = fma(c.inv, c.inv, -s);
+    c.lo = 0.5 * c.inv * (fma(-v, s, 1.0) - fma(v, sl, vl * s));   // half of 1 - (v + vl) inv^2
     return c;
 }
-
-// num / (sda sdb) from inva = 1 / sda and invb = 1 / sdb, 0 where these are 0; off by at most a unit in the last place.
-__device__ __forceinline__ double gram_quot(double num, double sda, double sdb, double inva, double invb)
+// num (inva + loa) (invb + lob), rounded once.
+__device__ __forceinline__ double gram_scale(double num, double inva, double loa, double invb, double lob)
 {
-    const double r = inva * invb, den = sda * sdb, q = num * r;
-    return fma(fma(-q, den, num), r, q);
+    const double r = __dmul_rn(inva, invb);
+    return fma(num, r, num * fma(loa, invb, fma(inva, lob, fma(inva, invb, -r))));
 }
 
 __global__ void __launch_bounds__(GR_THREADS, 2)
@@ -60,7 +64,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
     __shared__ uint64_t s_full[GR_NS], s_free[GR_NS], s_done;
     __shared__ uint32_t s_tmem;
     __shared__ int s_err;
-    __shared__ double s_np[GR_T], s_sd[GR_T], s_inv[GR_T];
+    __shared__ double s_np[GR_T], s_inv[GR_T], s_lo[GR_T];
     const int b = batch_blocks[blockIdx.y];
     const int ls = blk_ls[b], N = blk_ls[b + 1] - ls, nt = (N + GR_T - 1) / GR_T;
     // the upper-triangular tile (ti, tj), ti <= tj
@@ -135,8 +139,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
             const int k = tj * GR_T + tid;
             const GramCol c = gram_col(k < N ? freq[perm[ls + k]] : 0.0, n);
             s_np[tid] = c.np;
-            s_sd[tid] = c.sd;
             s_inv[tid] = c.inv;
+            s_lo[tid] = c.lo;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (!tc::mbar_wait(&s_done, 0, tc::BUILD_WAIT_NS)) s_err = 1;   // every stage: up to 32,768
@@ -153,8 +157,8 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
             for (int e = 0; e < 8; ++e) {
                 const int k = k0 + e;
                 if (j >= N || k >= N || k < j) continue;
-                const double num = __dsub_rn((double)(v[e] * 262144.0f), __dmul_rn(s_np[8 * g + e], row.p));
-                const double res = gram_quot(num, row.sd, s_sd[8 * g + e], row.inv, s_inv[8 * g + e]);
+                const double num = fma(-s_np[8 * g + e], row.p, (double)(v[e] * 262144.0f));
+                const double res = gram_scale(num, row.inv, row.lo, s_inv[8 * g + e], s_lo[8 * g + e]);
                 Wb[(size_t)j + (size_t)k * N] = res;
                 Wb[(size_t)k + (size_t)j * N] = res;
                 if (Fb) {

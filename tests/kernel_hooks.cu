@@ -17,13 +17,12 @@ __global__ void k_quotients(int n, const double *a, const double *b, double *roo
     ref[2 * n + i] = a[i] / root[i];
 }
 
-__global__ void k_gram_quotients(int n, const double *num, const double *sd, double *quot, double *ref)
+__global__ void k_gram_scaled(int n, const double *num, const double *f, double *out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double a = sd[i], b = sd[n + i];
-    quot[i] = soda::gram_quot(num[i], a, b, 1.0 / a, 1.0 / b);
-    ref[i] = num[i] / (a * b);
+    const soda::GramCol a = soda::gram_col(f[i], 1), b = soda::gram_col(f[n + i], 1);
+    out[i] = soda::gram_scale(num[i], a.inv, a.lo, b.inv, b.lo);
 }
 
 }  // namespace
@@ -75,9 +74,9 @@ extern "C" int hook_quotients(int n, const double *a, const double *b, double *r
     return cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess ? 0 : 1;
 }
 
-// quot = num / (sd[0 .. n-1] sd[n .. 2n-1]) and CUDA's own quotient.
-extern "C" int hook_gram_quotients(int n, const double *num, const double *sd, double *quot, double *ref)
+// out = num / sqrt(pa qa pb qb) for the allele frequencies f[0 .. n-1] and f[n .. 2n-1].
+extern "C" int hook_gram_scaled(int n, const double *num, const double *f, double *out)
 {
-    k_gram_quotients<<<(n + 255) / 256, 256>>>(n, num, sd, quot, ref);
+    k_gram_scaled<<<(n + 255) / 256, 256>>>(n, num, f, out);
     return cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess ? 0 : 1;
 }

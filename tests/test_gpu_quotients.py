@@ -1,7 +1,8 @@
-"""The square root, its reciprocal and the quotients that the Z build forms by
-correction steps (chol_tc.cuh, gram_tc.cuh) against CUDA's own, which are
-correctly rounded: within a unit in the last place, 1 / sqrt within two (the
-reference is a rounded root's rounded reciprocal, off by one itself)."""
+"""The square root, its reciprocal and the quotients that the factorisation forms
+by correction steps (chol_tc.cuh) against CUDA's own, which are correctly
+rounded: within a unit in the last place, 1 / sqrt within two (the reference is
+a rounded root's rounded reciprocal, off by one itself); and the scaling of the
+Gram (gram_tc.cuh) against long double."""
 import ctypes as C
 
 import numpy as np
@@ -58,16 +59,26 @@ def test_root_reciprocal_and_quotient(lib, lo, hi):
     assert _ulps(quot, ref[2 * N:]) <= 1
 
 
-def test_gram_quotient(lib):
+def test_gram_scaling(lib):
+    """num / sqrt(pa qa pb qb) in long double: one rounding of a value that is known to a few 2^-100, so half a unit, and
+    0 for a monomorphic SNP.  Frequencies of counts in up to 200,000 chromosomes, rare ones and near 1 among them, and
+    pairs of the same SNP."""
     import torch
-    gen = torch.Generator(device="cuda").manual_seed(7)
-    f = torch.cat([torch.rand(N, dtype=torch.float64, device="cuda", generator=gen),
-                   10.0 ** (-6.0 * torch.rand(N, dtype=torch.float64, device="cuda", generator=gen))])
-    f = f.clamp(1e-7, 1 - 1e-7)
-    sd = torch.sqrt(2.0 * f * (1.0 - f))
-    num = _numbers(gen, N, -30, 24, edges=False) * (1 - 2 * (torch.rand(N, device="cuda", generator=gen) < 0.5).double())
-    num[:5] = 0.0
-    quot, ref = (torch.empty(N, dtype=torch.float64, device="cuda") for _ in range(2))
-    _call(lib.hook_gram_quotients, N, num, sd, quot, ref)
-    assert torch.all(quot[:5] == 0.0)
-    assert _ulps(quot[5:], ref[5:]) <= 1
+    n = 100000
+    rng = np.random.default_rng(7)
+    f = np.concatenate([rng.integers(1, 2000, 2 * n // 2) / 2000.0, rng.integers(1, 200000, n) / 200000.0])
+    f[1::7] = 1.0 - 10.0 ** (-5.5 * rng.random(f[1::7].size))
+    f[2::7] = 10.0 ** (-5.5 * rng.random(f[2::7].size))
+    f[n:n + n // 4] = f[:n // 4]
+    f[5], f[n + 6], f[7] = 0.0, 1.0, 1.0
+    num = rng.standard_normal(n) * 10.0 ** rng.uniform(-3, 7, n)
+    d = [torch.from_numpy(x).cuda() for x in (num, f, np.empty(n))]
+    _call(lib.hook_gram_scaled, n, *d)
+    got = d[2].cpu().numpy()
+    assert got[5] == got[6] == got[7] == 0.0
+    keep = np.ones(n, dtype=bool)
+    keep[5:8] = False
+    a, b = f[:n].astype(np.longdouble)[keep], f[n:].astype(np.longdouble)[keep]
+    want = num[keep] / (np.sqrt(2 * a * (1 - a)) * np.sqrt(2 * b * (1 - b)))
+    ulp = np.spacing(np.abs(got[keep]))
+    assert np.max(np.abs((got[keep] - want) / ulp)) <= 0.51

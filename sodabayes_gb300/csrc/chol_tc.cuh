@@ -10,7 +10,8 @@
 //     hold U to 2^-56 of the bound;
 //   * the product of digits s and t belongs to level s + t.  Products are at most 2^14, so the FP32 sums of a level
 //     (at most seven pairs) are exact over 128 rows of U.  Levels 2 .. 9 (34 pairs) are kept, in one tensor-memory
-//     accumulator each; what levels 10 and up hold is below 2^-59 of the bounds' product;
+//     accumulator each; what levels 10 and up hold is below 2^-61 of the bounds' product a row, of either sign: about
+//     sqrt(N) 2^-64 over N rows;
 //   * every 128 rows the levels are added into one 64-bit integer per element, in units of 2^-62 of the bounds'
 //     product (Cauchy-Schwarz keeps the whole sum within the bounds' product).
 // So C = M - sum_t U_ti U_tj is rounded once, where a chain of N FP64 multiply-adds rounds at every term.
@@ -22,7 +23,8 @@
 //
 // Measured, 10 subsets of 2000 SNPs: updates 3.2 ms, diagonal blocks 2.9, substitution 2.6 (the last two bound by the
 // FP64 pipe, which takes any warp's instruction 64 cycles), against 31.9 ms of FP64 kernels (rank-32 updates 25.6,
-// panels 6.3).  U'U + A - d I is 2.2e-17 d at N = 301 and 1.3e-17 d at N = 1000 (rms), as before.
+// panels 6.3).  U'U + A - d I, with A exact, is 1.5e-17 d at N = 300 and n = 700, 1.4e-17 d at 600 and 1,500, 1.3e-17 d
+// at 1000 and 2,000 (rms; 1.9e-17, 1.8e-17 and 1.9e-17 with the FP64 kernels and their Gram).
 #pragma once
 #include <cuda.h>
 #include "tc.cuh"
@@ -248,7 +250,9 @@ __device__ __forceinline__ double ch_div(double c, double root, double inv)
 
 // The panel's diagonal block, in steps of 8: a warp factors 8 x 8 with a column a lane, a thread a column solves the
 // rest of its rows, and the warps take the rank-8 update's rows.  Bound by the chain of FP64 instructions: about 17 a
-// pivot in the factoring warp, 52 a step in the solving ones; 92 us a panel (121 us in steps of 16).  inv: the pivots'
+// pivot in the factoring warp, 52 a step in the solving ones; 92 us a panel (121 us in steps of 16).  A step's eight
+// products are summed by themselves: taken out of the block's entries one at a time, each would be rounded at the size
+// of M, and the pivots were off by as much as 64 such roundings.  inv: the pivots'
 // reciprocals, for k_ch_trsm.
 constexpr int CH_D = 8;
 
@@ -317,10 +321,10 @@ __global__ void __launch_bounds__(256) k_ch_diag(double *W, const int64_t *wofs,
 #pragma unroll
             for (int q = 0; q < CH_D; ++q) m[q] = -T[kb + q][r];
             for (int cc = (r & ~31) + lane; cc < CH_P; cc += 32) {
-                double s = T[r][cc];
+                double s = m[0] * T[kb][cc];
 #pragma unroll
-                for (int q = 0; q < CH_D; ++q) s = fma(m[q], T[kb + q][cc], s);
-                if (cc >= r) T[r][cc] = s;
+                for (int q = 1; q < CH_D; ++q) s = fma(m[q], T[kb + q][cc], s);
+                if (cc >= r) T[r][cc] += s;
             }
         }
         __syncthreads();

@@ -208,6 +208,13 @@ __device__ __forceinline__ void draw_ahead(const Dev &D, const ChainScal *S, con
     }
 }
 
+// x <= 700, false for a NaN: by the words, an FP64 comparison takes the narrow pipe 64 cycles a warp.
+__device__ __forceinline__ bool at_most_700(double x)
+{
+    const int hi = __double2hiint(x), c = 0x4085E000;   // the upper word of 700
+    return hi < c || (hi == c && __double2loint(x) == 0);
+}
+
 // The class (1-based) for the FP64 scores b_k + c_k r2 of up to DRAW_PRE classes: the first whose cumulative weight
 // exceeds u times their sum, weights exp(s_k - s_0), or relative to the largest score where that could overflow; there a
 // class more than 700 below the largest has none, as in the reference, which matters for u = 0.  (The
@@ -226,12 +233,15 @@ __device__ __forceinline__ int draw_class64(double r2, const double (&b)[DRAW_PR
     if (big) {
 #pragma unroll
         for (int k = 1; k < DRAW_PRE; ++k) ref = fmax(ref, w[k]);
+#pragma unroll
+        for (int k = 0; k < DRAW_PRE; ++k)
+            if (ref - w[k] > 700.0) w[k] = -1e308;
     }
     double sum = 0.0;
 #pragma unroll
     for (int k = 0; k < DRAW_PRE; ++k)
         if (k < nm) {
-            w[k] = k == 0 && !big ? 1.0 : (big && ref - w[k] > 700.0 ? 0.0 : exp(w[k] - ref));
+            w[k] = k == 0 && !big ? 1.0 : exp(w[k] - ref);
             sum = sum + w[k];
         }
     const double us = u * sum;
@@ -266,7 +276,7 @@ __device__ __forceinline__ double draw_snp(const Dev &D, const ChainScal *S, int
         if (m == SODAGPU_BAYES_B && sizeof(T) == 8) {
             // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2)), which is 0 above 700 as in the reference
             const T d = a.b[0] - (a.b[1] + a.c * (rhs * rhs));
-            flag = d <= (T)700.0 && a.u * ((T)1.0 + t_exp(d)) < (T)1.0 ? 2 : 1;
+            flag = at_most_700(d) && a.u * ((T)1.0 + t_exp(d)) < (T)1.0 ? 2 : 1;
         } else if (m == SODAGPU_BAYES_B) {
             const T s1 = q.logp[0];
             const T uhat = rhs / a.den;
@@ -673,7 +683,7 @@ __device__ __forceinline__ SkippedDraw skipped_draw(const Dev &D, const ChainSca
         const double s = lane == 0 ? cb.y : fma(rhs * rhs, cb.x, cb.y);
         if (m == SODAGPU_BAYES_B) {   // the inclusion comes first: u < 1 / (1 + exp(s_1 - s_2)), 0 above 700
             const double d = __shfl_sync(0xffffffffu, s, 0) - __shfl_sync(0xffffffffu, s, 1);
-            x.flag = d <= 700.0 && u * (1.0 + exp(d)) < 1.0 ? 2 : 1;
+            x.flag = at_most_700(d) && u * (1.0 + exp(d)) < 1.0 ? 2 : 1;
         } else {
             x.flag = skipped_class(s, u, nm);
         }

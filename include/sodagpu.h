@@ -45,11 +45,16 @@ enum sodagpu_method {
     SODAGPU_BAYES_RC = 6
 };
 
-/* Arithmetic of the per-iteration sweep.  The Z build is FP64 in every mode.
+/* Arithmetic of the per-iteration sweep.  The Z build is the same in every
+ * mode, with results of FP64 precision: the Gram is exact integers, scaled in
+ * FP64; the Lanczos run for d is FP64, from a start vector found in FP32; the
+ * factor's products are exact products of 8-bit digits (56 bits of U relative
+ * to its column's bound) added in 64-bit integers, the rest of it FP64.
  *   FP64: genotypes as centred/scaled FP64 columns, U in FP64 — the parity mode.
  *   FP32: genotypes as centred/scaled FP32 values, U in FP32 — the plain path.
- *   FP8 : genotypes as exact 8-bit 0/1/2 codes with the centring applied as an
- *         FP32 rank-1 correction, U as BF16 hi+lo pairs.                      */
+ *   FP8 : genotypes as exact 0/1/2 codes with the centring applied as an FP32
+ *         rank-1 correction; U as BF16 hi+mid+lo terms on the tensor cores,
+ *         in FP32 on the CUDA cores.                                        */
 enum sodagpu_precision { SODAGPU_FP64 = 0, SODAGPU_FP32 = 1, SODAGPU_FP8 = 2 };
 
 /* Sweep kernels.  AUTO puts the genotype products of the FP8 mode with 4, 8
@@ -356,10 +361,11 @@ void sodagpu_batch_destroy(sodagpu_batch *batch);
  * zbuild_j = p[j] * (n[j] * N_j / gram_ops + N_j^2 / (3 * fp64_flops)) is the
  * Gram and Cholesky of its subsets (N_j = blocksize[j]).  model[] holds
  * {step_us, bw (bytes/s), e_x, e_u, gram_ops (int8 multiply-adds/s),
- * fp64_flops}; NULL takes values measured on GB300 for the FP8 mode
- * {30, 2.6e12, 1, 4, 5e13, 6e11} (the bandwidth as measured on a batch of
- * 32 BayesB analyses, n up to 20,000 and p up to 200,000: 90 GB per
- * iteration in 35.6 ms).  *steps receives S and *model_s the modelled
+ * fp64_flops}; NULL takes {30, 2.6e12, 1, 4, 5e13, 6e11}, measured on GB300
+ * for the FP8 mode (the bandwidth on a batch of 32 BayesB analyses, n up to
+ * 20,000 and p up to 200,000: 90 GB per iteration in 35.6 ms) with a dp4a Gram
+ * and an FP64 Cholesky.  The present ones are several times faster; the
+ * defaults are kept, so that the sizes chosen for a batch stay the same.  *steps receives S and *model_s the modelled
  * seconds of the choice. */
 int sodagpu_autotune_batch(int32_t njobs, const int32_t *n, const int32_t *p, int32_t iters,
                            int32_t max_blocksize, const double *model, int32_t *blocksize, int32_t *steps,

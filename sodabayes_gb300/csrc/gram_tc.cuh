@@ -6,8 +6,9 @@
 // products are integers times 2^-18, and their FP32 sums are exact while 4 n <= 2^24.
 //
 // One CTA per 128 x 128 tile of the upper triangle, two CTAs an SM: the FP64 scaling of a tile (about ten
-// instructions an element, 40 us on the SM's narrow FP64 pipe) runs while the other CTA's MMAs do.  It is what bounds
-// the kernel: 10 subsets of 2000 SNPs and 20,000 individuals take 0.62 ms, 7.1 ms with dp4a on the integer pipe.
+// instructions an element, 40 us on the SM's narrow FP64 pipe) runs while the other CTA's MMAs do.  It is the larger
+// part of the kernel (FP64 pipe 45% active, tensor pipe 26%, by ncu): 10 subsets of 2000 SNPs and 20,000 individuals
+// take 0.62 ms, 7.1 ms with dp4a on the integer pipe.
 //
 // Warps 0-3 scale and store, warp 4 loads 128 SNPs x 128 individuals of both sides by TMA (128-byte swizzle), warp 5
 // issues the MMAs.

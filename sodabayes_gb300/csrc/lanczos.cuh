@@ -9,8 +9,9 @@
 // chip) and the recurrence with its reorthogonalisation (k_lz_orth: a cluster of LZ_CTAS CTAs per subset, which
 // exchange their partial dot products through distributed shared memory; on one SM the dot products alone were 110 us
 // of its FP64 pipe).  Measured, 10 subsets of 2000 SNPs (n = 20,000, LD blocks): 128 FP32 steps of 32 +
-// 21 us and 40 FP64 steps of 84 + 27 us, 11.4 ms, against 46.7 ms for 112 FP64 steps of 279 + 139 us.  The eigenvalue
-// is off by 1.25e-16 (relative rms, 44 subsets of 96 to 1000 SNPs; 1.33e-16 from a random start).
+// 21 us and 40 FP64 steps of 84 + 27 us, 11.4 ms, against 46.7 ms for 112 FP64 steps of 279 + 139 us; with other data
+// of the same kind 24 FP64 steps did, 9.8 ms.  The eigenvalue is off by 1.25e-16 (relative rms, 44 subsets of 96 to
+// 1000 SNPs; 1.33e-16 from a random start).
 #pragma once
 #include <cooperative_groups.h>
 #include "rng.cuh"

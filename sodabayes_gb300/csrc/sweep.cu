@@ -957,18 +957,24 @@ static size_t skipped_smem(int n)
 // per-iteration statistics: class counts and sum g^2 per (group, class),
 // sum r^2 (models.f90:194, 321-325, 496-503, 515)
 // ---------------------------------------------------------------------------
-// CTAs 0..NSTAT-1 of a chain take the SNPs, the others MU_ROWS rows of r each.  With up to STAT_FAST (group,
-// class) cells one pass serves all of them: a warp adds the squares of its 32 SNPs cell by cell (sparse chains
-// have a few non-zero effects per warp) into its own row of shared sums, in a fixed order, and the counts go
-// through integer atomics; more cells take one pass over the SNPs each.  At p = 12,000, 12 cells and 16 chains
-// the one pass takes 13 us, twelve passes took 122 us.
-constexpr int STAT_FAST = 64;
+// CTAs 0..NSTAT-1 of a chain take the SNPs, the others MU_ROWS rows of r each.  One pass serves all (group, class)
+// cells; the counts go through integer atomics.  With up to STAT_FAST cells a warp adds the squares of its 32 SNPs cell
+// by cell (sparse chains have a few non-zero effects per warp) into its own row of shared sums, in a fixed order: seven
+// FP64 instructions, of 64 cycles each, for a cell with several.  From STAT_LARGE SNPs and up to STAT_OWN cells a
+// thread has sums of its own in shared memory, one FP64 instruction for a warp's 32 SNPs, and STAT_AHEAD loads in
+// flight.  The iteration's kernels beside the subsets', p = 500,000, 16 chains, a quarter of the effects not zero: 235 us
+// by warps, 105 us by threads; p = 200,000, one chain of BayesA: 44 and 34 us; p = 12,000, 12 cells, 16 chains: 48 and
+// 51 us, for the sums' clearing and reduction, so smaller jobs stay with the warps.  More than STAT_FAST cells take one
+// pass over the SNPs each (p = 12,000, 12 cells, 16 chains: 13 us in one pass, 122 us in twelve).
+constexpr int STAT_OWN = 16, STAT_FAST = 64, STAT_AHEAD = 4;
+constexpr int STAT_LARGE = STAT_AHEAD * NSTAT * 256;   // a full turn of every thread
 
 __device__ __forceinline__ void stats_body(const Dev &D, const VB &vb)
 {
     __shared__ double sh[33];
-    __shared__ double s_acc[8][STAT_FAST];
+    __shared__ double s_sum[STAT_OWN * 256];
     __shared__ int s_cnt[STAT_FAST];
+    static_assert(8 * STAT_FAST <= STAT_OWN * 256, "the warps' rows of sums fit");
     tc::pdl_trigger();
     tc::pdl_wait();
     const int c = vb.y;
@@ -987,8 +993,46 @@ __device__ __forceinline__ void stats_body(const Dev &D, const VB &vb)
     }
     const int ngm = D.ngroup * D.nmix;
     const size_t base = (size_t)c * D.p;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (ngm <= STAT_OWN && D.p >= STAT_LARGE) {
+        constexpr int STEP = NSTAT * 256;
+        double *own = s_sum + threadIdx.x;
+        for (int e = 0; e < ngm; ++e) own[256 * e] = 0.0;
+        if (threadIdx.x < ngm) s_cnt[threadIdx.x] = 0;
+        __syncthreads();
+        for (int j0 = vb.x * 256 + 32 * warp; j0 < D.p; j0 += STAT_AHEAD * STEP) {
+            int e[STAT_AHEAD];
+            double gj[STAT_AHEAD];
+#pragma unroll
+            for (int q = 0; q < STAT_AHEAD; ++q) {
+                const int64_t j = (int64_t)j0 + q * STEP + lane;
+                e[q] = j < D.p ? (D.grp[j] - 1) + (D.cls[base + j] - 1) * D.ngroup : -1;
+                gj[q] = j < D.p ? D.g[base + j] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < STAT_AHEAD; ++q) {
+                const unsigned same = __match_any_sync(0xffffffffu, e[q]);
+                if (e[q] >= 0 && lane == __ffs(same) - 1) atomicAdd(&s_cnt[e[q]], __popc(same));
+                // not zero, by its bits: an FP64 comparison would take the pipe as long as the addition
+                if (__double_as_longlong(gj[q]) << 1) own[256 * e[q]] = fma(gj[q], gj[q], own[256 * e[q]]);
+            }
+        }
+        __syncthreads();
+        for (int e = warp; e < ngm; e += 8) {
+            double t = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) t += s_sum[256 * e + 32 * w + lane];
+            t = warp_sum(t);
+            if (lane == 0) {
+                const size_t o = ((size_t)c * NSTAT + vb.x) * ngm + e;
+                D.statpart[o] = t;
+                D.cntpart[o] = s_cnt[e];
+            }
+        }
+        return;
+    }
     if (ngm <= STAT_FAST) {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double (*s_acc)[STAT_FAST] = reinterpret_cast<double (*)[STAT_FAST]>(s_sum);
         for (int e = threadIdx.x; e < 8 * ngm; e += 256) s_acc[e / ngm][e % ngm] = 0.0;
         if (threadIdx.x < ngm) s_cnt[threadIdx.x] = 0;
         __syncthreads();
